@@ -82,12 +82,43 @@ bool invert(std::vector<double> &M, int n)  // Gauss-Jordan with partial pivotin
     return true;
 }
 
-bool chunking(int nz, int lmax, int &nch, int &L)
+bool chunking(int nz, int lmax, int &nch, int &L, int max_nch = 20)
 {
     nch = (nz + lmax - 1) / lmax;
     L = (nz + nch - 1) / nch;
-    if (nch > 20) return false;  // block geometry of sparc_col.cu (ColCfg MAXNCH)
+    if (nch > max_nch) return false;  // block geometry of sparc_col.cu (max_nch)
     return nz - (nch - 1) * L >= 2 && L >= 2;
+}
+
+// Chunk length (8 to 16 rows) and block width (8, 4 or 2 columns) of an FP64 column pass over ncols
+// columns.  The pass is bound by the double-precision pipe, where a warp occupies its SM quadrant for
+// 64 cycles per instruction however few of its lanes work and however few warps there are.  The
+// length depends on nz alone, so that a solve has the same bits in any batch: the least of warps of a
+// 4-column block, in fours for the four quadrants, times instructions of a warp, the latter about 100
+// per row and 200 for the four solves' couplings (300 rows: 30 chunks of 10, 120 threads).  The width minimises that over the
+// fullest SM, the wider where equal (memory sectors): one solve of 256 columns takes 64 blocks of 4,
+// or 32 of 152 SMs with blocks of 8.
+bool column_geometry(int nz, long long ncols, int nx, int &cw, int &nch, int &L)
+{
+    int best = 0;
+    for (int lmax = 16; lmax >= 8; lmax--) {
+        int n, l;
+        if (!chunking(nz, lmax, n, l, 40)) continue;
+        const int cost = ((4 * n + 31) / 32 + 3) / 4 * (l + 2);
+        if (best && cost >= best) continue;
+        best = cost;
+        nch = n;
+        L = l;
+    }
+    if (!best) return false;
+    long long least = -1;
+    for (int w = 8; w >= 2; w /= 2) {
+        const long long cost = ((ncols / w + 151) / 152 * ((w * nch + 31) / 32) + 3) / 4;
+        if (nx % w || (least >= 0 && cost >= least)) continue;
+        least = cost;
+        cw = w;
+    }
+    return true;
 }
 
 bool build_ztab(int nz, int ibc, int nch, int L, HostZTab &t)
@@ -173,6 +204,34 @@ bool build_ztab(int nz, int ibc, int nch, int L, HostZTab &t)
     if (!invert(M, n2)) return false;
     t.G = M;
     return true;
+}
+
+// The rows of the reduced inverse that the chunks' couplings use (x[first row - 1] and x[last row
+// + 1]; zero where there is none), cut to the smallest window of 2 h + 2 boundary values around
+// each chunk, the same h for all, outside of which every entry is below tol times its row's largest.
+// GB: [nch][2][gw], chunk j starting at boundary value min(max(2 j - h, 0), 2 nch - gw).
+int coupling_window(const HostZTab &t, double tol, std::vector<double> &GB)
+{
+    const int nch = t.nch, n2 = 2 * nch;
+    int h = 0;
+    auto row = [&](int j, int side) { return side == 0 ? (j > 0 ? 2 * j - 1 : -1) : (j < nch - 1 ? 2 * j + 2 : -1); };
+    for (int j = 0; j < nch; j++)
+        for (int side = 0; side < 2; side++) {
+            const int r = row(j, side);
+            if (r < 0) continue;
+            double big = 0.0;
+            for (int q = 0; q < n2; q++) big = std::max(big, std::fabs(t.G[(size_t)r * n2 + q]));
+            for (int q = 0; q < n2; q++)
+                if (std::fabs(t.G[(size_t)r * n2 + q]) > tol * big) h = std::max(h, std::max(2 * j - q, q - (2 * j + 1)));
+        }
+    const int gw = std::min(2 * h + 2, n2);
+    GB.assign((size_t)nch * 2 * gw, 0.0);
+    for (int j = 0; j < nch; j++)
+        for (int side = 0; side < 2; side++) {
+            const int r = row(j, side), q0 = std::min(std::max(2 * j + 1 - gw / 2, 0), n2 - gw);
+            for (int q = 0; r >= 0 && q < gw; q++) GB[((size_t)j * 2 + side) * gw + q] = t.G[(size_t)r * n2 + q0 + q];
+        }
+    return gw;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -327,7 +386,8 @@ void zband_host(const HostZTab &t, const HostBand &h, const double *b, double *x
 void zsolve_host(const HostZTab &t, const double *b, double *x, const double *preset_v, int n1)
 {
     const int nz = t.nz, nch = t.nch, L = t.L, n2 = 2 * nch;
-    std::vector<double> col(nz), y(nz), ub(n2);
+    std::vector<double> col(nz), y(nz), ub(n2), GB;
+    const int gw = coupling_window(t, 1e-20, GB);
     for (int i = 0; i < n1; i++) {
         for (int k = 0; k < nz; k++) col[k] = b[(size_t)k * n1 + i];
         auto rhs = [&](int k) {
@@ -348,8 +408,11 @@ void zsolve_host(const HostZTab &t, const double *b, double *x, const double *pr
         for (int c = 0; c < nch; c++) {
             const int s = c * L, e = std::min(nz, (c + 1) * L) - 1;
             double xl = 0, xr = 0;
-            if (c > 0) for (int q = 0; q < n2; q++) xl += t.G[(size_t)(2 * c - 1) * n2 + q] * ub[q];
-            if (c < nch - 1) for (int q = 0; q < n2; q++) xr += t.G[(size_t)(2 * c + 2) * n2 + q] * ub[q];
+            const int q0 = std::min(std::max(2 * c + 1 - gw / 2, 0), n2 - gw);
+            for (int q = 0; q < gw; q++) {
+                xl += GB[((size_t)c * 2) * gw + q] * ub[q0 + q];
+                xr += GB[((size_t)c * 2 + 1) * gw + q] * ub[q0 + q];
+            }
             for (int k = s; k <= e; k++) x[(size_t)k * n1 + i] = y[k] - t.WL[k] * xl - t.VU[k] * xr;
         }
     }
@@ -404,12 +467,14 @@ struct DevZ {
 template <typename T>
 cudaError_t upload_ztab(const HostZTab &h, DevZ<T> &d, std::vector<void *> &allocs)
 {
-    const int nz = h.nz, n2 = 2 * h.nch;
-    const size_t n = (size_t)nz * 5 + (size_t)nz * 5 + (size_t)n2 * n2;
+    const int nz = h.nz;
+    std::vector<double> GB;
+    const int gw = coupling_window(h, sizeof(T) == 8 ? 1e-20 : 1e-11, GB);
+    const size_t n = (size_t)nz * 5 + (size_t)nz * 5 + GB.size();
     std::vector<T> host(n);
     size_t o = 0;
     auto put = [&](const std::vector<double> &v) { for (double x : v) host[o++] = (T)x; };
-    put(h.w5); put(h.ib); put(h.lwib); put(h.gm); put(h.WL); put(h.VU); put(h.G);
+    put(h.w5); put(h.ib); put(h.lwib); put(h.gm); put(h.WL); put(h.VU); put(GB);
     cudaError_t e = cudaMalloc(&d.buf, n * sizeof(T));
     if (e != cudaSuccess) return e;
     allocs.push_back(d.buf);
@@ -423,6 +488,7 @@ cudaError_t upload_ztab(const HostZTab &h, DevZ<T> &d, std::vector<void *> &allo
     d.tab.WL = p; p += nz;
     d.tab.VU = p; p += nz;
     d.tab.G = p;
+    d.tab.gw = gw;
     d.tab.c1 = (T)h.c1;
     d.tab.c2 = (T)h.c2;
     d.tab.preset_row = h.preset_row;
@@ -504,6 +570,7 @@ struct Solver {
 struct sparc_plan {
     sparc_config_t cfg{};
     int nch = 0, L = 0, nch64 = 0, L64 = 0;
+    int cw64 = 0;  // block width of the FP64 column pass where column_geometry chose it and nch, L (0: not chosen)
     std::vector<void *> allocs;
     HostZTab hz[4], hz64[4];
     DevZ<double> z64[4];
@@ -601,12 +668,12 @@ int alloc_solver(sparc_plan *p)
     a.d_time = p->d_time;
     a.src_until = c.src_until; a.k_inj = c.k_inj; a.k_obs = c.k_obs; a.steps_out = c.steps_out;
     a.filt_k0 = c.filter_k0; a.filt_xall = c.filter_all_x;
-    // partitioned-solve block width: 32, 8 or 4 columns on request; otherwise 32 when those blocks
-    // (nx / 32 per solve) fill the 152 SMs, else 8.  One FP64 solve of 256 columns (the plain
-    // configuration): column pass 0.66 ms per step at 32 columns (8 blocks), 0.33 at 8 (32
-    // blocks), 0.35 at 4 (64 blocks, 76 threads each) on a GB300
+    // partitioned-solve block width: 32, 8 or 4 columns on request; for FP64 what column_geometry chose;
+    // otherwise 32 when those blocks (nx / 32 per solve) fill the 152 SMs, else 8
     if ((c.column_block == 32 || c.column_block == 8 || c.column_block == 4) && nx % c.column_block == 0) {
         a.colw = c.column_block;
+    } else if (p->cw64) {
+        a.colw = p->cw64;
     } else {
         a.colw = (nx % 32 == 0 && (long long)(nx / 32) * nb >= 152) ? 32 : 8;
     }
@@ -1037,6 +1104,9 @@ int sparc_plan_create(const sparc_config_t *cfg, sparc_plan_t **out)
         delete p;
         return fail(SPARC_ERR_SIZE, "sparc_plan_create: nz too large for the column chunking");
     }
+    // FP64, no width or variant asked for
+    if (cfg->precision == 64 && cfg->column_impl != 1 && cfg->column_block == 0)
+        column_geometry(cfg->nz, (long long)cfg->nx * cfg->nbatch, cfg->nx, p->cw64, p->nch, p->L);
     for (int ibc = 0; ibc < 4; ibc++) {
         if (!build_ztab(cfg->nz, ibc, p->nch, p->L, p->hz[ibc]) ||
             !build_ztab(cfg->nz, ibc, p->nch64, p->L64, p->hz64[ibc])) {

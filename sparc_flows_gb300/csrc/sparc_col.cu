@@ -16,24 +16,22 @@
 
 namespace sparc {
 
-// Column-block geometry: CW columns per block, at most MAXNCH chunks of at most LMAX rows.
-template <typename T>
-struct ColCfg;
-// Narrow blocks (8 columns = one 32-byte sector per row for FP32) so that several blocks are
-// resident per SM and their barrier-separated phases overlap each other's memory latency.
-template <>
-struct ColCfg<float> {
-    static constexpr int LMAX = 16, MAXNCH = 20;
-};
-template <>
-struct ColCfg<double> {
-    static constexpr int LMAX = 16, MAXNCH = 20;
-};
+// Column-block geometry: CW columns per block, chunks of at most LMAX rows.  FP32 blocks are 32
+// columns wide or narrow (8 columns = one 32-byte sector per row) so that several are resident per
+// SM and their barrier-separated phases overlap each other's memory latency.  FP64 is bound by the
+// double-precision pipe: a warp-wide instruction holds its SM quadrant for 64 cycles, so the width
+// (8, 4 or 2 columns) and the rows per thread are chosen to spread the warps over all 608 quadrants
+// (column_geometry in sparc_capi.cu).  FP64 column pass on a GB300, CUDA events: one solve of 256 x 300
+// without flow 50 us a launch (64 blocks of 4 columns, 10-row chunks) against 67 with 32 blocks of 8
+// columns and 16-row chunks; four solves with flow 80 us against 106.
+constexpr int COL_LMAX = 16;
 template <typename T, int CW>
-constexpr int min_blocks() { return CW <= 8 ? (sizeof(T) == 4 ? 4 : 2) : 1; }
+constexpr int max_nch() { return sizeof(T) == 8 && CW <= 8 ? 40 : 20; }
+template <typename T, int CW>
+constexpr int min_blocks() { return CW <= 8 ? (sizeof(T) == 4 ? 4 : CW <= 4 ? 2 : 1) : 1; }
 
 template <typename T, int CW, int LMAX>
-__global__ void __launch_bounds__(CW *ColCfg<T>::MAXNCH, (min_blocks<T, CW>())) col_stage_kernel(StepArgs<T> a)
+__global__ void __launch_bounds__(CW *max_nch<T, CW>(), (min_blocks<T, CW>())) col_stage_kernel(StepArgs<T> a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *B0 = reinterpret_cast<T *>(smem_raw);
@@ -315,7 +313,7 @@ __device__ void end_step_compensated(const StepArgs<float> &a, float *B0, float 
 }
 
 template <typename T, int CW, int LMAX>
-__global__ void __launch_bounds__(CW *ColCfg<T>::MAXNCH, (min_blocks<T, CW>())) end_step_kernel(StepArgs<T> a)
+__global__ void __launch_bounds__(CW *max_nch<T, CW>(), (min_blocks<T, CW>())) end_step_kernel(StepArgs<T> a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *B0 = reinterpret_cast<T *>(smem_raw);
@@ -395,7 +393,7 @@ aux:
 // Generic compact derivative of n1 columns: dvar = stretch .* dbyd2(var), optional
 // FILTER_VAR_Z (kernels.f90:891-928) afterwards.
 template <typename T, int CW, int LMAX>
-__global__ void __launch_bounds__(CW *ColCfg<T>::MAXNCH, (min_blocks<T, CW>())) ddz_kernel(ZTab<T> tb, int nch, int L, const T *__restrict__ var,
+__global__ void __launch_bounds__(CW *max_nch<T, CW>(), (min_blocks<T, CW>())) ddz_kernel(ZTab<T> tb, int nch, int L, const T *__restrict__ var,
                                                          T *__restrict__ dvar, int n1, int nz,
                                                          const T *__restrict__ preset,
                                                          const T *__restrict__ stretch, int filter)
@@ -489,7 +487,7 @@ __device__ __forceinline__ void kacc_dz(const KAccArgs<T> &a, const T *src, T *B
 }
 
 template <typename T, int CW, int LMAX>
-__global__ void __launch_bounds__(CW *ColCfg<T>::MAXNCH, (min_blocks<T, CW>())) kacc_col_kernel(KAccArgs<T> a)
+__global__ void __launch_bounds__(CW *max_nch<T, CW>(), (min_blocks<T, CW>())) kacc_col_kernel(KAccArgs<T> a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *B0 = reinterpret_cast<T *>(smem_raw);
@@ -541,7 +539,7 @@ cudaError_t launch_kacc_row(const KAccArgs<T> &a, cudaStream_t st);
 template <typename T, int CW>
 static cudaError_t launch_kacc_cw(const KAccArgs<T> &a, cudaStream_t st)
 {
-    constexpr int LMAX = ColCfg<T>::LMAX;
+    constexpr int LMAX = COL_LMAX;
     const size_t smem = ((size_t)2 * a.nz * CW + (size_t)2 * a.nch * CW) * sizeof(T);
     auto k = kacc_col_kernel<T, CW, LMAX>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -554,7 +552,7 @@ template <typename T>
 cudaError_t launch_kacc(const KAccArgs<T> &a, cudaStream_t st)
 {
     const int cw = a.colw == 32 ? 32 : 8;
-    if (a.nx % cw || a.L > ColCfg<T>::LMAX || a.nch > ColCfg<T>::MAXNCH) return cudaErrorInvalidValue;
+    if (a.nx % cw || a.L > COL_LMAX || a.nch > (cw == 32 ? max_nch<T, 32>() : max_nch<T, 8>())) return cudaErrorInvalidValue;
     cudaError_t e = launch_kacc_row<T>(a, st);
     if (e != cudaSuccess) return e;
     return cw == 32 ? launch_kacc_cw<T, 32>(a, st) : launch_kacc_cw<T, 8>(a, st);
@@ -565,7 +563,7 @@ template cudaError_t launch_kacc<double>(const KAccArgs<double> &, cudaStream_t)
 template <typename T, int CW>
 static cudaError_t launch_col_stage_cw(const StepArgs<T> &a, cudaStream_t st)
 {
-    constexpr int LMAX = ColCfg<T>::LMAX;
+    constexpr int LMAX = COL_LMAX;
     const size_t smem = ((size_t)2 * a.nz * CW + (size_t)8 * a.nch * CW) * sizeof(T);
     auto k = col_stage_kernel<T, CW, LMAX>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -577,11 +575,14 @@ static cudaError_t launch_col_stage_cw(const StepArgs<T> &a, cudaStream_t st)
 template <typename T>
 cudaError_t launch_col_stage(const StepArgs<T> &a, cudaStream_t st)
 {
-    if (a.nx % a.colw || a.L > ColCfg<T>::LMAX || a.nch > ColCfg<T>::MAXNCH) return cudaErrorInvalidValue;
+    if (a.nx % a.colw || a.L > COL_LMAX || a.nch > (a.colw == 32 ? max_nch<T, 32>() : max_nch<T, 8>())) return cudaErrorInvalidValue;
     switch (a.colw) {
         case 32: return launch_col_stage_cw<T, 32>(a, st);
         case 8: return launch_col_stage_cw<T, 8>(a, st);
         case 4: return launch_col_stage_cw<T, 4>(a, st);
+        case 2:
+            if constexpr (sizeof(T) == 8) return launch_col_stage_cw<T, 2>(a, st);
+            return cudaErrorInvalidValue;
         default: return cudaErrorInvalidValue;
     }
 }
@@ -589,7 +590,7 @@ cudaError_t launch_col_stage(const StepArgs<T> &a, cudaStream_t st)
 template <typename T, int CW>
 static cudaError_t launch_end_step_cw(const StepArgs<T> &a, cudaStream_t st)
 {
-    constexpr int LMAX = ColCfg<T>::LMAX;
+    constexpr int LMAX = COL_LMAX;
     const size_t smem = (size_t)a.nz * CW * sizeof(T) * (a.ALO ? 2 : 1);
     auto k = end_step_kernel<T, CW, LMAX>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -602,7 +603,7 @@ template <typename T>
 cudaError_t launch_end_step(const StepArgs<T> &a, cudaStream_t st)
 {
     const int cw = a.colw == 32 ? 32 : 8;
-    if (a.nx % cw || a.L > ColCfg<T>::LMAX || a.nch > ColCfg<T>::MAXNCH) return cudaErrorInvalidValue;
+    if (a.nx % cw || a.L > COL_LMAX || a.nch > (cw == 32 ? max_nch<T, 32>() : max_nch<T, 8>())) return cudaErrorInvalidValue;
     return cw == 32 ? launch_end_step_cw<T, 32>(a, st) : launch_end_step_cw<T, 8>(a, st);
 }
 
@@ -610,7 +611,7 @@ template <typename T, int CW>
 static cudaError_t launch_ddz_cw(const ZTab<T> &tb, int nch, int L, const T *var, T *dvar, int n1, int nz,
                                  const T *preset, const T *stretch, int filter, cudaStream_t st)
 {
-    constexpr int LMAX = ColCfg<T>::LMAX;
+    constexpr int LMAX = COL_LMAX;
     const size_t smem = ((size_t)nz * CW + (size_t)2 * nch * CW) * sizeof(T);
     auto k = ddz_kernel<T, CW, LMAX>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -623,10 +624,10 @@ template <typename T>
 cudaError_t launch_ddz(const ZTab<T> &tb, int nch, int L, const T *var, T *dvar, int n1, int nz, const T *preset,
                        const T *stretch, int filter, cudaStream_t st)
 {
-    if (L > ColCfg<T>::LMAX || nch > ColCfg<T>::MAXNCH || n1 <= 0) return cudaErrorInvalidValue;
+    if (L > COL_LMAX || nch > max_nch<T, 8>() || n1 <= 0) return cudaErrorInvalidValue;
     // many columns (a 3-D field: nb * ny * nx): 32 columns per block, four 32-byte sectors per
     // row access; few (a 2-D row of nx): 8, so that enough blocks exist
-    if (n1 % 32 == 0 && n1 >= 32 * 152 * 8)
+    if (n1 % 32 == 0 && n1 >= 32 * 152 * 8 && nch <= max_nch<T, 32>())
         return launch_ddz_cw<T, 32>(tb, nch, L, var, dvar, n1, nz, preset, stretch, filter, st);
     return launch_ddz_cw<T, 8>(tb, nch, L, var, dvar, n1, nz, preset, stretch, filter, st);
 }

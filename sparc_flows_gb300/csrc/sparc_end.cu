@@ -2,10 +2,11 @@
 // records driver.f90:386-417), streamed through 32-column tiles.
 //
 // A block owns one (solve, component) pair -- (xi_x, v_x) or (xi_z, v_z), which are coupled
-// because the RHS of xi is v -- over 32 adjacent x-columns and the full depth.  Its 16 warps take
-// rows w, w + 16, ...; lane = column, so every global access of a warp is one 128-byte row
-// segment.  Step 1: u_xi = xi + dt (v + bs rhs_v(s-1)) (zero on the RHS boundary rows/columns),
-// u_v = v + dt rhs_v(s), into shared memory [nz][32] (no bank conflicts), together with the
+// because the RHS of xi is v -- over CW adjacent x-columns and the full depth.  Its 512 threads take
+// rows w, w + 512 / CW, ...; consecutive threads are consecutive columns, so with CW = 32 every
+// global access of a warp is one 128-byte row segment.  CW is 32 where those blocks fill the SMs and
+// as narrow as one 32-byte sector where they would not (end_width below).  Step 1: u_xi = xi + dt (v + bs rhs_v(s-1)) (zero on the RHS boundary rows/columns),
+// u_v = v + dt rhs_v(s), into shared memory [nz][CW] (no bank conflicts), together with the
 // vertical-PML update of one psi component and the acceleration record.  Step 2, after one
 // barrier: FILTER_VARS_2D of both fields from shared memory, the state written in place, the
 // partial-state and seismogram records.  Rows are independent within a step, so each thread
@@ -14,30 +15,30 @@
 
 namespace sparc {
 
-constexpr int END_CW = 32, END_WARPS = 16;
+constexpr int END_CW = 32, END_THREADS = 512;
 
 // The 11-point filter, operation order of FILTER_VARS_2D (physics2d.f90:517-522, the neighbour
 // weights already halved).
-template <typename T>
+template <typename T, int W>
 __device__ __forceinline__ T end_filt11(const T *B, int k, int c)
 {
     const T c0 = T(0.75390625), h1 = T(0.5 * 0.41015625), h2 = T(0.5 * -0.234375), h3 = T(0.5 * 0.087890625),
             h4 = T(0.5 * -0.01953125), h5 = T(0.5 * 0.001953125);
-    constexpr int W = END_CW;
     return c0 * B[k * W + c] + h1 * (B[(k - 1) * W + c] + B[(k + 1) * W + c]) +
            h2 * (B[(k - 2) * W + c] + B[(k + 2) * W + c]) + h3 * (B[(k - 3) * W + c] + B[(k + 3) * W + c]) +
            h4 * (B[(k - 4) * W + c] + B[(k + 4) * W + c]) + h5 * (B[(k - 5) * W + c] + B[(k + 5) * W + c]);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(END_CW *END_WARPS) end_step_stream_kernel(StepArgs<T> a)
+template <typename T, int CW>
+__global__ void __launch_bounds__(END_THREADS) end_step_stream_kernel(StepArgs<T> a)
 {
+    constexpr int ROWS = END_THREADS / CW;  // rows in flight per pass over the depth
     extern __shared__ __align__(16) unsigned char smem_e[];
     T *Uxi = reinterpret_cast<T *>(smem_e);
     const int nz = a.nz, nx = a.nx;
-    T *Uv = Uxi + (size_t)nz * END_CW;
-    const int c = threadIdx.x % END_CW, w = threadIdx.x / END_CW;
-    const int x = blockIdx.x * END_CW + c;
+    T *Uv = Uxi + (size_t)nz * CW;
+    const int c = threadIdx.x % CW, w = threadIdx.x / CW;
+    const int x = blockIdx.x * CW + c;
     const int p = blockIdx.y & 1, b = blockIdx.y >> 1;  // component (0: x, 1: z), solve
     const size_t F = (size_t)nz * nx;
     const int time = *a.d_time;
@@ -54,13 +55,13 @@ __global__ void __launch_bounds__(END_CW *END_WARPS) end_step_stream_kernel(Step
     {
         constexpr int MP = 4;  // PML rows per batch and thread (the PML arrays hold both layers)
         const size_t ring = (size_t)a.slot_s * a.nb * 2 * a.nzpml * nx;
-        for (int base = w; base < a.nzpml; base += MP * END_WARPS) {
+        for (int base = w; base < a.nzpml; base += MP * ROWS) {
             T pv[MP];
             size_t qv[MP];
             int np = 0;
 #pragma unroll
             for (int i = 0; i < MP; i++) {
-                const int pi = base + i * END_WARPS;
+                const int pi = base + i * ROWS;
                 if (pi < a.nzpml) {
                     const size_t qz = (((size_t)b * 2 + p) * a.nzpml + pi) * nx + x;
                     qv[i] = qz;
@@ -75,12 +76,12 @@ __global__ void __launch_bounds__(END_CW *END_WARPS) end_step_stream_kernel(Step
     }
     // ---- 1: updated fields into shared memory; acc record
 #pragma unroll 4
-    for (int k = w; k < nz; k += END_WARPS) {
+    for (int k = w; k < nz; k += ROWS) {
         const size_t g = (size_t)k * nx + x;
         const T xi = __ldg(Axi + g), v = __ldg(Av + g), r4 = __ldg(R4 + g), r5 = __ldg(R5 + g);
         const T sxi = (k == 0 || xbc) ? T(0) : v + bs * r4;  // scr xi = v of stage 5, RHS zeros
-        Uxi[k * END_CW + c] = xi + dt * sxi;
-        Uv[k * END_CW + c] = v + dt * r5;
+        Uxi[k * CW + c] = xi + dt * sxi;
+        Uv[k * CW + c] = v + dt * r5;
         if (snap) snap[(size_t)(4 + p) * F + g] = r5;
     }
     __syncthreads();
@@ -88,16 +89,16 @@ __global__ void __launch_bounds__(END_CW *END_WARPS) end_step_stream_kernel(Step
     const bool xf = a.filt_xall || ((x >= a.nh - 1) && (x <= nx - a.nh));
     T *Gxi = a.A + ((size_t)b * 4 + p) * F, *Gv = a.A + ((size_t)b * 4 + 2 + p) * F;
 #pragma unroll 2
-    for (int k = w; k < nz; k += END_WARPS) {
+    for (int k = w; k < nz; k += ROWS) {
         const size_t g = (size_t)k * nx + x;
-        T oxi = Uxi[k * END_CW + c], ov = Uv[k * END_CW + c];
+        T oxi = Uxi[k * CW + c], ov = Uv[k * CW + c];
         if (xf && k >= a.filt_k0 && k <= nz - 2) {
             if (k >= 5 && k <= nz - 6) {
-                oxi = end_filt11(Uxi, k, c);
-                ov = end_filt11(Uv, k, c);
+                oxi = end_filt11<T, CW>(Uxi, k, c);
+                ov = end_filt11<T, CW>(Uv, k, c);
             } else {
-                oxi = T(0.5) * (Uxi[(k + 1) * END_CW + c] + Uxi[(k - 1) * END_CW + c]);
-                ov = T(0.5) * (Uv[(k + 1) * END_CW + c] + Uv[(k - 1) * END_CW + c]);
+                oxi = T(0.5) * (Uxi[(k + 1) * CW + c] + Uxi[(k - 1) * CW + c]);
+                ov = T(0.5) * (Uv[(k + 1) * CW + c] + Uv[(k - 1) * CW + c]);
             }
         }
         Gxi[g] = oxi;
@@ -255,17 +256,40 @@ size_t end_stream_smem_bytes(int nz)
     return (size_t)2 * nz * END_CW * sizeof(T);
 }
 
+// Tile width: the widest whose blocks (two per solve and tile) number two per SM, else one 32-byte
+// sector.  One FP64 solve of 256 x 300: 16 blocks of 32 columns 75 us, 128 of 4 columns 16 us;
+// one FP32 solve of 512 x 300: 32 blocks of 32 columns 17 us, 128 of 8 10 us (GB300).
+template <typename T>
+static int end_width(const StepArgs<T> &a)
+{
+    int w = END_CW;
+    while (w > 32 / (int)sizeof(T) && (long long)(a.nx / w) * 2 * a.nb < 2 * 152) w /= 2;
+    return w;
+}
+
+template <typename T, int CW>
+static cudaError_t end_stream_cw(const StepArgs<T> &a, cudaStream_t st)
+{
+    const size_t smem = (size_t)2 * a.nz * CW * sizeof(T);
+    auto k = end_step_stream_kernel<T, CW>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<dim3(a.nx / CW, 2 * a.nb), END_THREADS, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
 template <typename T>
 cudaError_t launch_end_step_stream(const StepArgs<T> &a, cudaStream_t st)
 {
     if (a.nx % END_CW || a.ALO) return cudaErrorInvalidValue;
-    const size_t smem = end_stream_smem_bytes<T>(a.nz);
-    cudaError_t e = cudaFuncSetAttribute(end_step_stream_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return e;
-    dim3 grid(a.nx / END_CW, 2 * a.nb);
-    end_step_stream_kernel<T><<<grid, END_CW * END_WARPS, smem, st>>>(a);
-    return cudaGetLastError();
+    switch (end_width(a)) {
+        case 32: return end_stream_cw<T, 32>(a, st);
+        case 16: return end_stream_cw<T, 16>(a, st);
+        case 8: return end_stream_cw<T, 8>(a, st);
+        default: break;
+    }
+    if constexpr (sizeof(T) == 8) return end_stream_cw<T, 4>(a, st);
+    return cudaErrorInvalidValue;
 }
 
 template size_t end_stream_smem_bytes<float>(int);
