@@ -18,66 +18,75 @@
 //                     top and bottom rows zero                          (displacement.f90:419-474)
 // End of step: s3_end_kernel (a += dt scr with FILTER_VARS_3D_HORIZ_PML when due, one thread
 // per column with an 11-value window in registers, in place), the PML auxiliaries, the record.
-#include "sparc_common.cuh"
+#include "sparc_wfft.cuh"
 
 namespace sparc {
 
 constexpr int S3_THREADS = 256;
 
 // ---------------------------------------------------------------------------------------------
-// y-derivative: a block takes 16 consecutive x-columns of one (level, solve) plane; each warp
-// transforms two of them (packed as real and imaginary parts of one complex row of length NY,
-// the shared-memory Stockham FFT of the x pass), derivative by i k * stretchy, inverse.  Loads
-// and stores go through shared memory so that each global access covers 16 consecutive x
-// (64 bytes in FP32) of one y-row.
-constexpr int DDY_COLS = 16;
-constexpr int DDY_WARPS = DDY_COLS / 2;
-// Per-warp region of the shared-memory transform: xr, xi, yr, yi of NY values each, every array
-// offset by one more word and the regions DDY_SPAN(NY) words apart (not a multiple of 32), so
-// that the 16 columns a warp scatters on load (and gathers on store) fall in different banks.
-template <int NY>
-constexpr int ddy_span() { return 4 * NY + 5; }
+// y-derivative: neighbouring threads are neighbouring x-columns, so every load and store of a plane is
+// contiguous and goes straight between global memory and the registers of the transform.  A block takes
+// 2 XL columns of one (level, solve) plane, columns x0 + c and x0 + XL + c sharing a transform as real and
+// imaginary part; thread (c, t) holds y = t + L m of both (sparc_wfft.cuh), and the exchanges between the
+// stages go through shared memory [NY][XL], free of bank conflicts.
+template <typename T, int NY>
+struct DdyCfg {
+    static constexpr int V = NY == 512 ? 16 : WFft<T, NY>::V, L = NY / V;
+    // columns of a 128-byte row segment; half of that where the threads of a block would be 1024
+    static constexpr int XL = sizeof(T) == 4 && L < 32 ? 32 : 16;
+    static constexpr int THREADS = L * XL;
+    // resident blocks that the registers are limited for: FP32 is bound by memory and wants two
+    static constexpr int BLOCKS = sizeof(T) == 4 && V == 8 ? 2 : 1;
+    static constexpr size_t SMEM = (size_t)2 * ColExchange<T, NY, XL>::SPAN * sizeof(T);
+};
 
 template <typename T, int NY>
-__global__ void __launch_bounds__(DDY_WARPS *WARP) ddy_kernel(const T *__restrict__ var, T *__restrict__ dvar,
-                                                             int nx, T stretchy, const T *twr, const T *twi,
-                                                             const T *kap)
+__global__ void __launch_bounds__((DdyCfg<T, NY>::THREADS), (DdyCfg<T, NY>::BLOCKS)) ddy_kernel(const T *__restrict__ var, T *__restrict__ dvar,
+                                                                      int nx, T stretchy, const T *twr, const T *twi,
+                                                                      const T *kap)
 {
+    using C = DdyCfg<T, NY>;
+    constexpr int XL = C::XL, V = C::V, L = C::L;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *sm = reinterpret_cast<T *>(smem_raw);
-    constexpr int S = ddy_span<NY>();
-    __shared__ T s_inv[DDY_COLS];
-    __shared__ int s_off[DDY_WARPS][2];  // offsets of the result arrays in each warp's region
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const size_t plane = (size_t)blockIdx.y * NY * nx;
-    const int x0 = blockIdx.x * DDY_COLS;
-    for (int idx = threadIdx.x; idx < NY * DDY_COLS; idx += DDY_WARPS * WARP) {
-        const int y = idx / DDY_COLS, c = idx % DDY_COLS;
-        sm[(c >> 1) * S + (c & 1) * (NY + 1) + y] = var[plane + (size_t)y * nx + x0 + c];
+    __shared__ RowMax<T> red[2][L][XL];
+    const int c = threadIdx.x % XL, t = threadIdx.x / XL;
+    // a last block that would pass the plane's end starts earlier and repeats columns (same values)
+    const int x0 = min((int)blockIdx.x * 2 * XL, nx - 2 * XL);
+    const T *src = var + (size_t)blockIdx.y * NY * nx + x0 + c;
+    T *dst = dvar + (size_t)blockIdx.y * NY * nx + x0 + c;
+    T re[V], im[V];
+    RowMax<T> mr, mi;
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        re[m] = src[(size_t)(t + L * m) * nx];
+        im[m] = src[(size_t)(t + L * m) * nx + XL];
     }
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        mr.add(re[m]);
+        mi.add(im[m]);
+    }
+    red[0][t][c] = mr;
+    red[1][t][c] = mi;
     __syncthreads();
-    T *base = sm + warp * S;
-    T *xr = base, *xi = base + (NY + 1), *yr = base + 2 * (NY + 1), *yi = base + 3 * (NY + 1);
-    T mr = T(0), mi = T(0);
-    for (int y = lane; y < NY; y += WARP) {
-        mr = fmax(mr, fabs(xr[y]));
-        mi = fmax(mi, fabs(xi[y]));
+#pragma unroll
+    for (int j = 0; j < L; j++) {
+        mr.merge(red[0][j][c]);
+        mi.merge(red[1][j][c]);
     }
-    T sr, si, isr, isi;
-    warp_row_scale(mr, sr, isr);
-    warp_row_scale(mi, si, isi);
-    T *orr, *oi;
-    fft_deriv<T, NY>(xr, xi, yr, yi, twr, twi, kap, stretchy, lane, orr, oi, sr, si);
-    if (lane == 0) {
-        s_inv[2 * warp] = isr;
-        s_inv[2 * warp + 1] = isi;
-        s_off[warp][0] = (int)(orr - base);
-        s_off[warp][1] = (int)(oi - base);
+    const RowScale<T> sr = row_scale<T>(mr), si = row_scale<T>(mi);
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        re[m] = scale_in(re[m], sr);
+        im[m] = scale_in(im[m], si);
     }
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < NY * DDY_COLS; idx += DDY_WARPS * WARP) {
-        const int y = idx / DDY_COLS, c = idx % DDY_COLS, w = c >> 1;
-        dvar[plane + (size_t)y * nx + x0 + c] = sm[w * S + s_off[w][c & 1] + y] * s_inv[c];
+    const ColExchange<T, NY, XL> ex{reinterpret_cast<T *>(smem_raw), c};
+    wfft_deriv<T, NY, V, WFft<T, NY>::RADIX4>(re, im, ex, twr, twi, kap, stretchy, t);
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        dst[(size_t)(t + L * m) * nx] = scale_out(re[m], sr);
+        dst[(size_t)(t + L * m) * nx + XL] = scale_out(im[m], si);
     }
 }
 
@@ -85,12 +94,12 @@ template <typename T, int NY>
 static cudaError_t ddy_n(const T *var, T *dvar, int nplanes, int nx, T stretchy, const T *twr, const T *twi,
                          const T *kap, cudaStream_t st)
 {
-    const size_t smem = (size_t)DDY_WARPS * ddy_span<NY>() * sizeof(T);
+    using C = DdyCfg<T, NY>;
     auto k = ddy_kernel<T, NY>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
     if (e != cudaSuccess) return e;
-    dim3 grid(nx / DDY_COLS, nplanes);
-    k<<<grid, DDY_WARPS * WARP, smem, st>>>(var, dvar, nx, stretchy, twr, twi, kap);
+    dim3 grid((nx + 2 * C::XL - 1) / (2 * C::XL), nplanes);
+    k<<<grid, C::THREADS, C::SMEM, st>>>(var, dvar, nx, stretchy, twr, twi, kap);
     return cudaGetLastError();
 }
 
@@ -99,10 +108,11 @@ cudaError_t launch_ddy(const T *var, T *dvar, int nplanes, int nx, int ny, T str
                        const T *kap, cudaStream_t st)
 {
     if (nplanes <= 0) return cudaSuccess;
-    if (nx % DDY_COLS) return cudaErrorInvalidValue;
+    if (nx < 64 || nx % 16) return cudaErrorInvalidValue;
     if (nplanes > 65535) return cudaErrorInvalidValue;
 #define CASE(n_) if (ny == n_) return ddy_n<T, n_>(var, dvar, nplanes, nx, stretchy, twr, twi, kap, st);
-    CASE(64) CASE(128) CASE(192) CASE(256) CASE(384) CASE(512)
+    CASE(64) CASE(128) CASE(192) CASE(256) CASE(384)
+    if constexpr (sizeof(T) == 4) { CASE(512) }
 #undef CASE
     return cudaErrorInvalidValue;
 }

@@ -92,26 +92,33 @@ bool chunking(int nz, int lmax, int &nch, int &L, int max_nch = 20)
 
 // Chunk length (8 to 16 rows) and block width (8, 4 or 2 columns) of an FP64 column pass over ncols
 // columns.  The pass is bound by the double-precision pipe, where a warp occupies its SM quadrant for
-// 64 cycles per instruction however few of its lanes work and however few warps there are.  The
-// length depends on nz alone, so that a solve has the same bits in any batch: the least of warps of a
-// 4-column block, in fours for the four quadrants, times instructions of a warp, the latter about 100
-// per row and 200 for the four solves' couplings (300 rows: 30 chunks of 10, 120 threads).  The width minimises that over the
-// fullest SM, the wider where equal (memory sectors): one solve of 256 columns takes 64 blocks of 4,
-// or 32 of 152 SMs with blocks of 8.
+// 64 cycles per instruction however few of its lanes work and however few warps there are.  A warp
+// issues about 100 instructions per row of its chunk and 8 per boundary value that the four solves
+// couple it to (the window reaches 48 rows each way).  The length depends on nz alone, so that a solve
+// has the same bits in any batch: the shortest, so that one solve spreads furthest, whose instructions
+// for 8 columns are no more than those of 16-row chunks coupled to every boundary value (300 rows: 30
+// chunks of 10, 9400 instructions against 9500).  The width minimises the warps of the
+// fullest SM, the wider where equal (memory sectors); from 152 blocks of 8 on, two of which an SM holds, it
+// is 8.  One solve of 256 columns takes 64 blocks of 4 (68 us a launch against 78 with 8, with flow), 2048
+// columns 256 blocks of 8 (122 us against 181 with 4), 6144 columns 768 of 8 (395 against 428).
 bool column_geometry(int nz, long long ncols, int nx, int &cw, int &nch, int &L)
 {
-    int best = 0;
-    for (int lmax = 16; lmax >= 8; lmax--) {
+    if (!chunking(nz, 16, nch, L, 32)) return false;
+    const int budget = (8 * nch + 31) / 32 * (100 * L + 16 * nch);
+    for (int lmax = 8; lmax < 16; lmax++) {
         int n, l;
-        if (!chunking(nz, lmax, n, l, 40)) continue;
-        const int cost = ((4 * n + 31) / 32 + 3) / 4 * (l + 2);
-        if (best && cost >= best) continue;
-        best = cost;
+        if (!chunking(nz, lmax, n, l, 32)) continue;
+        const int window = std::min(4 * ((48 + l - 1) / l) + 2, 2 * n);
+        if ((8 * n + 31) / 32 * (100 * l + 8 * window) > budget) continue;
         nch = n;
         L = l;
+        break;
     }
-    if (!best) return false;
     long long least = -1;
+    if (nx % 8 == 0 && ncols / 8 >= 152) {
+        cw = 8;
+        return true;
+    }
     for (int w = 8; w >= 2; w /= 2) {
         const long long cost = ((ncols / w + 151) / 152 * ((w * nch + 31) / 32) + 3) / 4;
         if (nx % w || (least >= 0 && cost >= least)) continue;
@@ -1173,7 +1180,7 @@ int sparc_ddx(sparc_plan_t *p, const double *var, double *dvar, int nrows, doubl
 {
     if (!p || !var || !dvar || nrows < 0) return fail(SPARC_ERR_ARG, "sparc_ddx: bad argument");
     CK(launch_ddx<double>(var, dvar, nrows, p->cfg.nx, stretchx, p->fft64.twr, p->fft64.twi, p->fft64.kap,
-                          (cudaStream_t)stream));
+                          (cudaStream_t)stream, p->cfg.precision == 32));
     return SPARC_OK;
 }
 

@@ -26,9 +26,9 @@ namespace sparc {
 // columns and 16-row chunks; four solves with flow 80 us against 106.
 constexpr int COL_LMAX = 16;
 template <typename T, int CW>
-constexpr int max_nch() { return sizeof(T) == 8 && CW <= 8 ? 40 : 20; }
+constexpr int max_nch() { return sizeof(T) == 8 && CW <= 8 ? 32 : 20; }
 template <typename T, int CW>
-constexpr int min_blocks() { return CW <= 8 ? (sizeof(T) == 4 ? 4 : CW <= 4 ? 2 : 1) : 1; }
+constexpr int min_blocks() { return CW <= 8 ? (sizeof(T) == 4 ? 4 : 2) : 1; }
 
 template <typename T, int CW, int LMAX>
 __global__ void __launch_bounds__(CW *max_nch<T, CW>(), (min_blocks<T, CW>())) col_stage_kernel(StepArgs<T> a)
@@ -560,10 +560,9 @@ cudaError_t launch_kacc(const KAccArgs<T> &a, cudaStream_t st)
 template cudaError_t launch_kacc<float>(const KAccArgs<float> &, cudaStream_t);
 template cudaError_t launch_kacc<double>(const KAccArgs<double> &, cudaStream_t);
 
-template <typename T, int CW>
+template <typename T, int CW, int LMAX = COL_LMAX>
 static cudaError_t launch_col_stage_cw(const StepArgs<T> &a, cudaStream_t st)
 {
-    constexpr int LMAX = COL_LMAX;
     const size_t smem = ((size_t)2 * a.nz * CW + (size_t)8 * a.nch * CW) * sizeof(T);
     auto k = col_stage_kernel<T, CW, LMAX>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -578,10 +577,19 @@ cudaError_t launch_col_stage(const StepArgs<T> &a, cudaStream_t st)
     if (a.nx % a.colw || a.L > COL_LMAX || a.nch > (a.colw == 32 ? max_nch<T, 32>() : max_nch<T, 8>())) return cudaErrorInvalidValue;
     switch (a.colw) {
         case 32: return launch_col_stage_cw<T, 32>(a, st);
-        case 8: return launch_col_stage_cw<T, 8>(a, st);
-        case 4: return launch_col_stage_cw<T, 4>(a, st);
+        // FP64 chunks of up to 12 rows: register arrays of that length, so that two 8-column blocks
+        // are resident
+        case 8:
+            if constexpr (sizeof(T) == 8)
+                if (a.L <= 12) return launch_col_stage_cw<T, 8, 12>(a, st);
+            return launch_col_stage_cw<T, 8>(a, st);
+        case 4:
+            if constexpr (sizeof(T) == 8)
+                if (a.L <= 12) return launch_col_stage_cw<T, 4, 12>(a, st);
+            return launch_col_stage_cw<T, 4>(a, st);
         case 2:
-            if constexpr (sizeof(T) == 8) return launch_col_stage_cw<T, 2>(a, st);
+            if constexpr (sizeof(T) == 8)
+                return a.L <= 12 ? launch_col_stage_cw<T, 2, 12>(a, st) : launch_col_stage_cw<T, 2>(a, st);
             return cudaErrorInvalidValue;
         default: return cudaErrorInvalidValue;
     }

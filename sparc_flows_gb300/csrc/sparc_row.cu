@@ -9,6 +9,7 @@
 //                                 the column pass needs for its ibc=3 boundary);
 //   d/dx of v_x, v_z at stage s -> advection terms -2 v0x d/dx (physics2d.f90:1065-1079).
 #include "sparc_fft512.cuh"
+#include "sparc_wfft.cuh"
 
 namespace sparc {
 
@@ -64,136 +65,24 @@ __device__ __forceinline__ void row_load(const StepArgs<T> &a, const RowCtx<T> &
 }
 
 // From gpx = dp/dx and dxx = dxi_x/dx at column x: x-PML, RHS v_x of stage s-1, dxi_x/dx for the
-// column pass; the inputs (v_x, v_z at stage s) of the second FFT (MODE != 2).
+// column pass, and the inputs (v_x, v_z at stage s) of the second FFT (MODE != 2).  Loads and arithmetic
+// only: what is to be stored is returned (svx: RHS v_x of stage s-1, dxo: dxi_x/dx) or, for the x-PML
+// columns, left in the row's scratch P ([3][nhx]: psi_vx RHS or, closing pass, the new psi_vx;
+// psi_gradp_x RHS; closing pass, the new psi_gradp_x).  The stores follow in row_mid_store.
 template <typename T, int MODE>
-__device__ __forceinline__ void row_mid(const StepArgs<T> &a, const RowCtx<T> &r, int x, T gpx, T dxx, T &vxs, T &vzs)
+__device__ __forceinline__ void row_mid_load(const StepArgs<T> &a, const RowCtx<T> &r, int x, T gpx, T dxx, T *P,
+                                             T &svx, T &dxo, T &vxs, T &vzs)
 {
     const int b = r.b, k = r.k, nx = r.nx, nh = r.nh, nhx = r.nhx;
     const size_t F = r.F, ro = r.ro;
     const bool pml = (x < nh) || (x >= nx - nh);
     const int ai = (x < nh) ? x : x - (nx - nh) + nh;
-    if (MODE != 2 && k == a.nz - 1) a.TOPDX[(size_t)b * nx + x] = dxx;
     if (pml) {
         const T axv = __ldg(r.axk + ai), bxv = __ldg(r.bxk + ai);
+        T ngp = T(0);
         if (MODE != 0) {  // psi_gradp_x of stage s-1
             const size_t q = ((size_t)1 * a.nz + k) * nhx + ai;
             T ps = r.PXb[q];
-            if (a.stage >= 3) ps += r.bsm1 * a.SPX[((size_t)a.slot_sm2 * a.nb + b) * 2 * a.nz * nhx + q];
-            gpx += ps;
-            a.SPX[((size_t)a.slot_sm1 * a.nb + b) * 2 * a.nz * nhx + q] = axv * gpx + bxv * ps;
-        }
-        if (MODE != 2) {  // psi_vx of stage s
-            const size_t q = ((size_t)0 * a.nz + k) * nhx + ai;
-            T ps = r.PXb[q];
-            if (MODE == 1) ps += r.bs * a.SPX[((size_t)a.slot_sm1 * a.nb + b) * 2 * a.nz * nhx + q];
-            dxx += ps;
-            a.SPX[((size_t)a.slot_s * a.nb + b) * 2 * a.nz * nhx + q] = axv * dxx + bxv * ps;
-        }
-    }
-    T svx = T(0);
-    if (MODE != 0) {
-        svx = __ldg(a.RVXP + (size_t)b * F + ro + x) - r.rhoinv_k * gpx;
-        if (k == 0 || x == 0 || x == nx - 1) svx = T(0);
-        svp(a, a.slot_sm1, b, 0)[ro + x] = svx;
-    }
-    vxs = T(0);
-    vzs = T(0);
-    if (MODE != 2) {
-        a.DX[(size_t)b * F + ro + x] = dxx;
-        vxs = __ldg(r.Ab + F_VX * F + ro + x);
-        vzs = __ldg(r.Ab + F_VZ * F + ro + x);
-        if (MODE == 1) {
-            vxs += r.bs * svx;
-            vzs += r.bs * __ldg(svp(a, a.slot_sm1, b, 1) + ro + x);
-        }
-    } else if (pml) {
-        // closing pass: pmlvarsx += deltat * scrpmlx (step.f90:112-115)
-        for (int c = 0; c < 2; c++) {
-            const size_t q = ((size_t)c * a.nz + k) * nhx + ai;
-            r.PXb[q] += a.dt * a.SPX[((size_t)a.slot_sm1 * a.nb + b) * 2 * a.nz * nhx + q];
-        }
-    }
-}
-
-// x-advection terms -2 v0x d/dx of v_x, v_z at column x.
-template <typename T>
-__device__ __forceinline__ void row_out(const StepArgs<T> &a, const RowCtx<T> &r, int x, T dvx, T dvz)
-{
-    const T w = T(-2) * a.fsign * __ldg(a.v0x + (size_t)r.b * a.bg2 + r.ro + x);
-    a.FXX[(size_t)r.b * r.F + r.ro + x] = w * dvx;
-    a.FXZ[(size_t)r.b * r.F + r.ro + x] = w * dvz;
-}
-
-template <typename T, int N, int MODE>
-__global__ void __launch_bounds__(ROW_WPB *WARP) row_stage_kernel(StepArgs<T> a)
-{
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *sm = reinterpret_cast<T *>(smem_raw);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (MODE == 0 && blockIdx.x == 0 && threadIdx.x == 0) *a.d_time += 1;  // new step begins
-    const int row = blockIdx.x * ROW_WPB + warp;
-    if (row >= a.nb * a.nz) return;
-    T *xr = sm + warp * 4 * N, *xi = xr + N, *yr = xi + N, *yi = yr + N;
-    const RowCtx<T> r(a, row, N);
-
-    T mr = T(0), mi = T(0);
-    for (int x = lane; x < N; x += WARP) {
-        T p, xis;
-        row_load<T, MODE>(a, r, x, p, xis);
-        xr[x] = p;
-        xi[x] = xis;
-        mr = fmax(mr, fabs(p));
-        mi = fmax(mi, fabs(xis));
-    }
-    T sr, si, isr, isi;
-    warp_row_scale(mr, sr, isr);
-    warp_row_scale(mi, si, isi);
-    __syncwarp();
-    T *o1r, *o1i;
-    fft_deriv<T, N>(xr, xi, yr, yi, a.twr, a.twi, a.kap, a.stretchx, lane, o1r, o1i, sr, si);
-    __syncwarp();
-
-    T mr2 = T(0), mi2 = T(0);
-    for (int x = lane; x < N; x += WARP) {
-        T vxs, vzs;
-        row_mid<T, MODE>(a, r, x, o1r[x] * isr, o1i[x] * isi, vxs, vzs);
-        if (MODE != 2) {
-            o1r[x] = vxs;
-            o1i[x] = vzs;
-            mr2 = fmax(mr2, fabs(vxs));
-            mi2 = fmax(mi2, fabs(vzs));
-        }
-    }
-    if (MODE == 2 || !a.flows) return;
-    T sr2, si2, isr2, isi2;
-    warp_row_scale(mr2, sr2, isr2);
-    warp_row_scale(mi2, si2, isi2);
-    __syncwarp();
-    T *gr = (o1r == xr) ? yr : xr, *gi = (o1r == xr) ? yi : xi;
-    T *o2r, *o2i;
-    fft_deriv<T, N>(o1r, o1i, gr, gi, a.twr, a.twi, a.kap, a.stretchx, lane, o2r, o2i, sr2, si2);
-    __syncwarp();
-    for (int x = lane; x < N; x += WARP) row_out(a, r, x, o2r[x] * isr2, o2i[x] * isi2);
-}
-
-// row_mid without global stores, for the register-FFT pass: the loads and arithmetic of column x;
-// what row_mid stores is returned (svx: RHS v_x of stage s-1, dxo: dxi_x/dx) or, for the x-PML
-// columns, left in the warp scratch P ([3][nhx]: psi_vx RHS or, closing pass, the new psi_vx;
-// psi_gradp_x RHS; closing pass, the new psi_gradp_x).  The stores follow in row_mid_store.
-template <int MODE>
-__device__ __forceinline__ void row_mid_load(const StepArgs<float> &a, const RowCtx<float> &r, int x, float gpx,
-                                             float dxx, float *P, float &svx, float &dxo, float &vxs, float &vzs)
-{
-    const int b = r.b, k = r.k, nx = r.nx, nh = r.nh, nhx = r.nhx;
-    const size_t F = r.F, ro = r.ro;
-    const bool pml = (x < nh) || (x >= nx - nh);
-    const int ai = (x < nh) ? x : x - (nx - nh) + nh;
-    if (pml) {
-        const float axv = __ldg(r.axk + ai), bxv = __ldg(r.bxk + ai);
-        float ngp = 0.f;
-        if (MODE != 0) {  // psi_gradp_x of stage s-1
-            const size_t q = ((size_t)1 * a.nz + k) * nhx + ai;
-            float ps = r.PXb[q];
             if (a.stage >= 3) ps += r.bsm1 * a.SPX[((size_t)a.slot_sm2 * a.nb + b) * 2 * a.nz * nhx + q];
             gpx += ps;
             ngp = axv * gpx + bxv * ps;
@@ -201,7 +90,7 @@ __device__ __forceinline__ void row_mid_load(const StepArgs<float> &a, const Row
         }
         if (MODE != 2) {  // psi_vx of stage s
             const size_t q = ((size_t)0 * a.nz + k) * nhx + ai;
-            float ps = r.PXb[q];
+            T ps = r.PXb[q];
             if (MODE == 1) ps += r.bs * a.SPX[((size_t)a.slot_sm1 * a.nb + b) * 2 * a.nz * nhx + q];
             dxx += ps;
             P[ai] = axv * dxx + bxv * ps;
@@ -211,14 +100,14 @@ __device__ __forceinline__ void row_mid_load(const StepArgs<float> &a, const Row
             P[2 * nhx + ai] = r.PXb[q1] + a.dt * ngp;
         }
     }
-    svx = 0.f;
+    svx = T(0);
     if (MODE != 0) {
         svx = __ldg(a.RVXP + (size_t)b * F + ro + x) - r.rhoinv_k * gpx;
-        if (k == 0 || x == 0 || x == nx - 1) svx = 0.f;
+        if (k == 0 || x == 0 || x == nx - 1) svx = T(0);
     }
     dxo = dxx;
-    vxs = 0.f;
-    vzs = 0.f;
+    vxs = T(0);
+    vzs = T(0);
     if (MODE != 2) {
         vxs = __ldg(r.Ab + F_VX * F + ro + x);
         vzs = __ldg(r.Ab + F_VZ * F + ro + x);
@@ -229,13 +118,12 @@ __device__ __forceinline__ void row_mid_load(const StepArgs<float> &a, const Row
     }
 }
 
-// The x-PML stores of row_mid_load from the warp scratch P (lanes over the PML columns).
-template <int MODE>
-__device__ __forceinline__ void row_mid_store_pml(const StepArgs<float> &a, const RowCtx<float> &r, const float *P,
-                                                  int lane)
+// The x-PML stores of row_mid_load from the scratch P (the row's lanes over the PML columns).
+template <typename T, int MODE, int LANES>
+__device__ __forceinline__ void row_mid_store_pml(const StepArgs<T> &a, const RowCtx<T> &r, const T *P, int lane)
 {
     const int b = r.b, k = r.k, nhx = r.nhx;
-    for (int ai = lane; ai < nhx; ai += WARP) {
+    for (int ai = lane; ai < nhx; ai += LANES) {
         const size_t q0 = ((size_t)0 * a.nz + k) * nhx + ai, q1 = ((size_t)1 * a.nz + k) * nhx + ai;
         if (MODE != 0) a.SPX[((size_t)a.slot_sm1 * a.nb + b) * 2 * a.nz * nhx + q1] = P[nhx + ai];
         if (MODE != 2) {
@@ -244,6 +132,97 @@ __device__ __forceinline__ void row_mid_store_pml(const StepArgs<float> &a, cons
             r.PXb[q0] = P[ai];
             r.PXb[q1] = P[2 * nhx + ai];
         }
+    }
+}
+
+// The row pass with the register transforms of sparc_wfft.cuh: WFft<T, N>::ROWS rows per warp, thread t of a
+// row holding columns t + L m.
+template <typename T, int N, int MODE>
+__global__ void __launch_bounds__(ROW_WPB *WARP) row_stage_kernel(StepArgs<T> a, int region)
+{
+    using W = WFft<T, N>;
+    constexpr int V = W::V, L = W::L;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int t = (threadIdx.x & 31) % L, slot = threadIdx.x / L;  // row of the block
+    if (MODE == 0 && blockIdx.x == 0 && threadIdx.x == 0) *a.d_time += 1;  // new step begins
+    const int rows = a.nb * a.nz, first = blockIdx.x * (blockDim.x / L) + slot;
+    const bool valid = first < rows;
+    const int row = valid ? first : rows - 1;  // the warp's other rows need every lane
+    T *S = reinterpret_cast<T *>(smem_raw) + (size_t)slot * region;
+    const RowExchange<T, N> ex{S};
+    const RowCtx<T> r(a, row, N);
+
+    T re[V], im[V];
+    RowMax<T> mr, mi;
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        row_load<T, MODE>(a, r, t + L * m, re[m], im[m]);
+        mr.add(re[m]);
+        mi.add(im[m]);
+    }
+    mr.template reduce<L>();
+    mi.template reduce<L>();
+    RowScale<T> sr = row_scale<T>(mr), si = row_scale<T>(mi);
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        re[m] = scale_in(re[m], sr);
+        im[m] = scale_in(im[m], si);
+    }
+    wfft_deriv<T, N, V, W::RADIX4>(re, im, ex, a.twr, a.twi, a.kap, a.stretchx, t);
+
+    RowMax<T> mr2, mi2;
+    // FP32: every load of the row before its first store, where the registers hold what is to be stored
+    constexpr bool DEFER = sizeof(T) == 4 && V < 32;
+    constexpr int VD = DEFER ? V : 1;
+    T svx[VD], dxo[VD];
+    __syncwarp();  // the transform's last reads of S are done before S holds the x-PML values
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        const int x = t + L * m, md = DEFER ? m : 0;
+        T vxs, vzs;
+        const T dxx = scale_out(im[m], si);
+        if (MODE != 2 && r.k == a.nz - 1 && valid) a.TOPDX[(size_t)r.b * N + x] = dxx;  // without the x-PML term
+        row_mid_load<T, MODE>(a, r, x, scale_out(re[m], sr), dxx, S, svx[md], dxo[md], vxs, vzs);
+        if (!DEFER && valid) {
+            if (MODE != 0) svp(a, a.slot_sm1, r.b, 0)[r.ro + x] = svx[md];
+            if (MODE != 2) a.DX[(size_t)r.b * r.F + r.ro + x] = dxo[md];
+        }
+        re[m] = vxs;
+        im[m] = vzs;
+        mr2.add(vxs);
+        mi2.add(vzs);
+    }
+    __syncwarp();
+    if (valid) row_mid_store_pml<T, MODE, L>(a, r, S, t);
+    if (DEFER && valid) {
+#pragma unroll
+        for (int m = 0; m < V; m++) {
+            const int x = t + L * m, md = DEFER ? m : 0;
+            if (MODE != 0) svp(a, a.slot_sm1, r.b, 0)[r.ro + x] = svx[md];
+            if (MODE != 2) a.DX[(size_t)r.b * r.F + r.ro + x] = dxo[md];
+        }
+    }
+    if (MODE == 2 || !a.flows) return;
+    __syncwarp();  // the x-PML values are read before the next transform reuses S
+    mr2.template reduce<L>();
+    mi2.template reduce<L>();
+    sr = row_scale<T>(mr2);
+    si = row_scale<T>(mi2);
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        re[m] = scale_in(re[m], sr);
+        im[m] = scale_in(im[m], si);
+    }
+    wfft_deriv<T, N, V, W::RADIX4>(re, im, ex, a.twr, a.twi, a.kap, a.stretchx, t);
+    if (!valid) return;
+    T wv[V];  // -2 v0x of the row, loaded before the advection terms are stored
+#pragma unroll
+    for (int m = 0; m < V; m++) wv[m] = T(-2) * a.fsign * __ldg(a.v0x + (size_t)r.b * a.bg2 + r.ro + t + L * m);
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        const size_t q = (size_t)r.b * r.F + r.ro + t + L * m;
+        a.FXX[q] = wv[m] * scale_out(re[m], sr);
+        a.FXZ[q] = wv[m] * scale_out(im[m], si);
     }
 }
 
@@ -314,14 +293,14 @@ __global__ void __launch_bounds__(ROW_WPB *WARP, 4) row_stage_reg512_kernel(Step
 #pragma unroll
     for (int n2 = 0; n2 < 16; n2++) {
         float vxs, vzs;
-        row_mid_load<MODE>(a, r, lane + 32 * n2, re[n2] * isr, im[n2] * isi, S, svx[n2], dxo[n2], vxs, vzs);
+        row_mid_load<float, MODE>(a, r, lane + 32 * n2, re[n2] * isr, im[n2] * isi, S, svx[n2], dxo[n2], vxs, vzs);
         re[n2] = vxs;
         im[n2] = vzs;
         mr2 = fmaxf(mr2, fabsf(vxs));
         mi2 = fmaxf(mi2, fabsf(vzs));
     }
     __syncwarp();
-    row_mid_store_pml<MODE>(a, r, S, lane);
+    row_mid_store_pml<float, MODE, WARP>(a, r, S, lane);
     {
         const size_t F = r.F, ro = r.ro;
 #pragma unroll
@@ -351,36 +330,46 @@ __global__ void __launch_bounds__(ROW_WPB *WARP, 4) row_stage_reg512_kernel(Step
     }
 }
 
-// Generic spectral x-derivative of nrows rows (two rows per warp).
-template <typename T, int N>
+// Generic spectral x-derivative of nrows rows, two to a transform.
+template <typename T, int N, bool FOUR>
 __global__ void __launch_bounds__(ROW_WPB *WARP) ddx_kernel(const T *__restrict__ var, T *__restrict__ dvar,
                                                               int nrows, T stretchx, const T *twr, const T *twi,
                                                               const T *kap)
 {
+    using W = WFft<T, N, FOUR>;
+    constexpr int V = W::V, L = W::L;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *sm = reinterpret_cast<T *>(smem_raw);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int r0 = 2 * (blockIdx.x * ROW_WPB + warp);
-    if (r0 >= nrows) return;
-    const bool two = r0 + 1 < nrows;
-    T *xr = sm + warp * 4 * N, *xi = xr + N, *yr = xi + N, *yi = yr + N;
-    T mr = T(0), mi = T(0);
-    for (int x = lane; x < N; x += WARP) {
-        xr[x] = var[(size_t)r0 * N + x];
-        xi[x] = two ? var[(size_t)(r0 + 1) * N + x] : T(0);
-        mr = fmax(mr, fabs(xr[x]));
-        mi = fmax(mi, fabs(xi[x]));
+    const int t = (threadIdx.x & 31) % L, slot = threadIdx.x / L;
+    const int r0 = 2 * (blockIdx.x * (blockDim.x / L) + slot);
+    const bool one = r0 < nrows, two = r0 + 1 < nrows;
+    const RowExchange<T, N> ex{reinterpret_cast<T *>(smem_raw) + (size_t)slot * W::REGION};
+    const T *src = var + (size_t)r0 * N + t;
+    T re[V], im[V];
+    RowMax<T> mr, mi;
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        re[m] = one ? src[L * m] : T(0);
+        im[m] = two ? src[N + L * m] : T(0);
     }
-    T sr, si, isr, isi;
-    warp_row_scale(mr, sr, isr);
-    warp_row_scale(mi, si, isi);
-    __syncwarp();
-    T *orr, *oi;
-    fft_deriv<T, N>(xr, xi, yr, yi, twr, twi, kap, stretchx, lane, orr, oi, sr, si);
-    __syncwarp();
-    for (int x = lane; x < N; x += WARP) {
-        dvar[(size_t)r0 * N + x] = orr[x] * isr;
-        if (two) dvar[(size_t)(r0 + 1) * N + x] = oi[x] * isi;
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        mr.add(re[m]);
+        mi.add(im[m]);
+    }
+    mr.template reduce<L>();
+    mi.template reduce<L>();
+    const RowScale<T> sr = row_scale<T>(mr), si = row_scale<T>(mi);
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        re[m] = scale_in(re[m], sr);
+        im[m] = scale_in(im[m], si);
+    }
+    wfft_deriv<T, N, V, W::RADIX4>(re, im, ex, twr, twi, kap, stretchx, t);
+    T *dst = dvar + (size_t)r0 * N + t;
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        if (one) dst[L * m] = scale_out(re[m], sr);
+        if (two) dst[N + L * m] = scale_out(im[m], si);
     }
 }
 
@@ -425,22 +414,15 @@ static cudaError_t row_stage_n(const StepArgs<T> &a, cudaStream_t st)
         else row_reg512_launch<2>(a, grid, st);
         return cudaGetLastError();
     }
-    const int rows = a.nb * a.nz;
-    const int grid = (rows + ROW_WPB - 1) / ROW_WPB;
-    const size_t smem = (size_t)ROW_WPB * 4 * N * sizeof(T);
-    if (a.stage == 1) {
-        auto k = row_stage_kernel<T, N, 0>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k<<<grid, ROW_WPB * WARP, smem, st>>>(a);
-    } else if (a.stage <= 5) {
-        auto k = row_stage_kernel<T, N, 1>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k<<<grid, ROW_WPB * WARP, smem, st>>>(a);
-    } else {
-        auto k = row_stage_kernel<T, N, 2>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k<<<grid, ROW_WPB * WARP, smem, st>>>(a);
-    }
+    // four warps a block; two, so that the blocks reach every SM, where the rows are few
+    const int rows = a.nb * a.nz, wpb = rows <= 152 * ROW_WPB * WFft<T, N>::ROWS ? 2 : ROW_WPB;
+    const int slots = wpb * WFft<T, N>::ROWS, grid = (rows + slots - 1) / slots;
+    const int region = max(WFft<T, N>::REGION, 3 * a.nhx);  // exchange arrays, or the row's x-PML values
+    const size_t smem = (size_t)slots * region * sizeof(T);
+    auto k = a.stage == 1 ? row_stage_kernel<T, N, 0> : a.stage <= 5 ? row_stage_kernel<T, N, 1> : row_stage_kernel<T, N, 2>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<grid, wpb * WARP, smem, st>>>(a, region);
     return cudaGetLastError();
 }
 
@@ -453,25 +435,29 @@ cudaError_t launch_row_stage(const StepArgs<T> &a, cudaStream_t st)
     return cudaErrorInvalidValue;
 }
 
-template <typename T, int N>
+template <typename T, int N, bool FOUR>
 static cudaError_t ddx_n(const T *var, T *dvar, int nrows, T stretchx, const T *twr, const T *twi, const T *kap,
                          cudaStream_t st)
 {
-    const int pairs = (nrows + 1) / 2;
-    const int grid = (pairs + ROW_WPB - 1) / ROW_WPB;
-    const size_t smem = (size_t)ROW_WPB * 4 * N * sizeof(T);
-    auto k = ddx_kernel<T, N>;
+    const int pairs = (nrows + 1) / 2, wpb = pairs <= 152 * ROW_WPB * WFft<T, N, FOUR>::ROWS ? 1 : ROW_WPB;
+    const int slots = wpb * WFft<T, N, FOUR>::ROWS, grid = (pairs + slots - 1) / slots;
+    const size_t smem = (size_t)slots * WFft<T, N, FOUR>::REGION * sizeof(T);
+    auto k = ddx_kernel<T, N, FOUR>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k<<<grid, ROW_WPB * WARP, smem, st>>>(var, dvar, nrows, stretchx, twr, twi, kap);
+    k<<<grid, wpb * WARP, smem, st>>>(var, dvar, nrows, stretchx, twr, twi, kap);
     return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_ddx(const T *var, T *dvar, int nrows, int nx, T stretchx, const T *twr, const T *twi,
-                       const T *kap, cudaStream_t st)
+                       const T *kap, cudaStream_t st, bool setup)
 {
     if (nrows <= 0) return cudaSuccess;
-#define CASE(n_) if (nx == n_) return ddx_n<T, n_>(var, dvar, nrows, stretchx, twr, twi, kap, st);
+#define CASE(n_)                                                                                                     \
+    if (nx == n_)                                                                                                    \
+        return radix_four<T, n_>() && !setup                                                                         \
+                   ? ddx_n<T, n_, radix_four<T, n_>()>(var, dvar, nrows, stretchx, twr, twi, kap, st)                 \
+                   : ddx_n<T, n_, false>(var, dvar, nrows, stretchx, twr, twi, kap, st);
     SPARC_FFT_SIZES(CASE)
 #undef CASE
     return cudaErrorInvalidValue;
@@ -482,65 +468,60 @@ cudaError_t launch_ddx(const T *var, T *dvar, int nrows, int nx, T stretchx, con
 template <typename T, int N>
 __global__ void __launch_bounds__(ROW_WPB *WARP) kacc_row_kernel(KAccArgs<T> a)
 {
+    using W = WFft<T, N>;
+    constexpr int V = W::V, L = W::L;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T *sm = reinterpret_cast<T *>(smem_raw);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = blockIdx.x * ROW_WPB + warp;
-    if (row >= a.nb * a.nz) return;
-    T *xr = sm + warp * 4 * N, *xi = xr + N, *yr = xi + N, *yi = yr + N;
+    const int t = (threadIdx.x & 31) % L, slot = threadIdx.x / L;
+    const int rows = a.nb * a.nz, first = blockIdx.x * (blockDim.x / L) + slot;
+    const bool valid = first < rows;
+    const int row = valid ? first : rows - 1;
+    const RowExchange<T, N> ex{reinterpret_cast<T *>(smem_raw) + (size_t)slot * W::REGION};
     const int b = row / a.nz, k = row - b * a.nz;
-    const size_t F = (size_t)a.nz * N, ro = (size_t)k * N;
-    const T *f = a.fsn + a.fbase + (size_t)b * a.fstride;
-    const T *av = a.adj + (size_t)b * a.astride;
-    T *w = a.work + (size_t)b * 4 * F;
+    const size_t F = (size_t)a.nz * N, q = (size_t)k * N + t;
+    const T *f = a.fsn + a.fbase + (size_t)b * a.fstride + q;
+    const T *av = a.adj + (size_t)b * a.astride + q;
+    T *w = a.work + (size_t)b * 4 * F + q;
     // forward xi_x with adjoint v_x, then forward v_x with v_z: the forward and adjoint fields
     // carry unrelated normalisations, so each row is scaled before it shares an FFT
-    T mr = T(0), mi = T(0);
-    for (int x = lane; x < N; x += WARP) {
-        xr[x] = f[0 * F + ro + x];
-        xi[x] = av[ro + x];
-        mr = fmax(mr, fabs(xr[x]));
-        mi = fmax(mi, fabs(xi[x]));
-    }
-    T sr, si, isr, isi;
-    warp_row_scale(mr, sr, isr);
-    warp_row_scale(mi, si, isi);
-    __syncwarp();
-    T *o1r, *o1i;
-    fft_deriv<T, N>(xr, xi, yr, yi, a.twr, a.twi, a.kap, a.stretchx, lane, o1r, o1i, sr, si);
-    __syncwarp();
-    T mr2 = T(0), mi2 = T(0);
-    for (int x = lane; x < N; x += WARP) {
-        w[0 * F + ro + x] = o1r[x] * isr;
-        w[1 * F + ro + x] = o1i[x] * isi;
-        o1r[x] = f[2 * F + ro + x];
-        o1i[x] = f[3 * F + ro + x];
-        mr2 = fmax(mr2, fabs(o1r[x]));
-        mi2 = fmax(mi2, fabs(o1i[x]));
-    }
-    T sr2, si2, isr2, isi2;
-    warp_row_scale(mr2, sr2, isr2);
-    warp_row_scale(mi2, si2, isi2);
-    __syncwarp();
-    T *gr = (o1r == xr) ? yr : xr, *gi = (o1r == xr) ? yi : xi;
-    T *o2r, *o2i;
-    fft_deriv<T, N>(o1r, o1i, gr, gi, a.twr, a.twi, a.kap, a.stretchx, lane, o2r, o2i, sr2, si2);
-    __syncwarp();
-    for (int x = lane; x < N; x += WARP) {
-        w[2 * F + ro + x] = o2r[x] * isr2;
-        w[3 * F + ro + x] = o2i[x] * isi2;
+#pragma unroll
+    for (int pair = 0; pair < 2; pair++) {
+        const T *p0 = pair == 0 ? f : f + 2 * F, *p1 = pair == 0 ? av : f + 3 * F;
+        T re[V], im[V];
+        RowMax<T> mr, mi;
+#pragma unroll
+        for (int m = 0; m < V; m++) {
+            re[m] = __ldg(p0 + L * m);
+            im[m] = __ldg(p1 + L * m);
+            mr.add(re[m]);
+            mi.add(im[m]);
+        }
+        mr.template reduce<L>();
+        mi.template reduce<L>();
+        const RowScale<T> sr = row_scale<T>(mr), si = row_scale<T>(mi);
+#pragma unroll
+        for (int m = 0; m < V; m++) {
+            re[m] = scale_in(re[m], sr);
+            im[m] = scale_in(im[m], si);
+        }
+        wfft_deriv<T, N, V, W::RADIX4>(re, im, ex, a.twr, a.twi, a.kap, a.stretchx, t);
+#pragma unroll
+        for (int m = 0; m < V; m++) {
+            if (!valid) continue;
+            w[(size_t)(2 * pair) * F + L * m] = scale_out(re[m], sr);
+            w[(size_t)(2 * pair + 1) * F + L * m] = scale_out(im[m], si);
+        }
     }
 }
 
 template <typename T, int N>
 static cudaError_t kacc_row_n(const KAccArgs<T> &a, cudaStream_t st)
 {
-    const int rows = a.nb * a.nz;
-    const int grid = (rows + ROW_WPB - 1) / ROW_WPB;
-    const size_t smem = (size_t)ROW_WPB * 4 * N * sizeof(T);
+    const int rows = a.nb * a.nz, slots = ROW_WPB * WFft<T, N>::ROWS;
+    const size_t smem = (size_t)slots * WFft<T, N>::REGION * sizeof(T);
     auto k = kacc_row_kernel<T, N>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k<<<grid, ROW_WPB * WARP, smem, st>>>(a);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<(rows + slots - 1) / slots, ROW_WPB * WARP, smem, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -558,8 +539,8 @@ template cudaError_t launch_kacc_row<double>(const KAccArgs<double> &, cudaStrea
 template cudaError_t launch_row_stage<float>(const StepArgs<float> &, cudaStream_t);
 template cudaError_t launch_row_stage<double>(const StepArgs<double> &, cudaStream_t);
 template cudaError_t launch_ddx<float>(const float *, float *, int, int, float, const float *, const float *,
-                                       const float *, cudaStream_t);
+                                       const float *, cudaStream_t, bool);
 template cudaError_t launch_ddx<double>(const double *, double *, int, int, double, const double *,
-                                        const double *, const double *, cudaStream_t);
+                                        const double *, const double *, cudaStream_t, bool);
 
 }  // namespace sparc
