@@ -1555,9 +1555,10 @@ namespace {
 template <typename T>
 struct Plan3 {
     std::vector<void *> allocs;
-    T *A = nullptr, *SCR = nullptr, *X = nullptr, *PV = nullptr, *SPV = nullptr, *PSI = nullptr;
-    T *D1 = nullptr, *D2 = nullptr, *D3 = nullptr, *PP = nullptr, *RHO = nullptr, *GX = nullptr, *GY = nullptr,
-      *GZ = nullptr;
+    T *A = nullptr, *PV = nullptr, *SPV = nullptr;
+    T *XV = nullptr;  // stage velocities, two slots of [3][F]
+    T *ADV = nullptr; // advection sums [3][F] (with flow)
+    T *D1 = nullptr, *PP = nullptr, *RHO = nullptr;
     T *prof = nullptr, *v0 = nullptr, *pat = nullptr;
     T *ADJ = nullptr;  // adjoint forcing of the current step at the observation level [nb][ny][nx]
     DevZ<T> z[2];  // ibc 0, 1
@@ -1605,10 +1606,9 @@ int alloc_plan3(sparc3d_plan *p)
     const long long F = p->F, P = p->P, nz = c.nz, npml = c.npmlbot + c.npmltop;
     struct Req { T **ptr; size_t n; };
     std::vector<Req> reqs = {
-        {&S.A, (size_t)6 * F}, {&S.SCR, (size_t)6 * F}, {&S.X, (size_t)6 * F},
-        {&S.PV, (size_t)2 * P}, {&S.SPV, (size_t)2 * P}, {&S.PSI, (size_t)2 * P},
-        {&S.D1, (size_t)F}, {&S.D2, (size_t)F}, {&S.D3, (size_t)F}, {&S.PP, (size_t)F}, {&S.RHO, (size_t)F},
-        {&S.GX, (size_t)F}, {&S.GY, (size_t)F}, {&S.GZ, (size_t)F},
+        {&S.A, (size_t)6 * F}, {&S.XV, (size_t)6 * F}, {&S.ADV, c.flows ? (size_t)3 * F : 1},
+        {&S.PV, (size_t)2 * P}, {&S.SPV, (size_t)2 * P},
+        {&S.D1, (size_t)F}, {&S.PP, (size_t)F}, {&S.RHO, (size_t)F},
         {&S.prof, (size_t)(8 * nz + 2 * npml)}, {&S.v0, c.flows ? (size_t)3 * nz * p->nxy : 1},
         {&S.pat, (size_t)c.nbatch * p->nxy}, {&S.ADJ, (size_t)c.nbatch * p->nxy},
     };
@@ -1673,35 +1673,44 @@ cudaError_t d3z(sparc3d_plan *p, const T *v, T *dv, int ibc, cudaStream_t st, in
                          S.stretch, filter, st);
 }
 
-// MP_FLOWS_PML_3D_DISPL (displacement.f90:377-477) on X (psi: PSI), into SCR and SPV.
+// The five stages of MP_FLOWS_PML_3D_DISPL (displacement.f90:377-477) and the end of the step; acc: where the
+// last stage's RHS of v is kept for a kernel-stage record, or null.
 template <typename T>
-cudaError_t rhs3(sparc3d_plan *p, const T *X, const T *PSI, T amp, cudaStream_t st)
+cudaError_t stages3(sparc3d_plan *p, T amp, T *acc, cudaStream_t st)
 {
     Plan3<T> &S = plan3<T>(p);
     const sparc3d_config_t &c = p->cfg;
-    const long long F = p->F, P = p->P;
-    const S3Args a{c.nx, c.ny, c.nz, c.nbatch, c.npmlbot, c.npmltop, c.k_src, c.flows, p->nxy};
+    const long long F = p->F;
+    S3Step<T> a{};
+    a.nx = c.nx; a.ny = c.ny; a.nz = c.nz; a.nb = c.nbatch;
+    a.npmlbot = c.npmlbot; a.npmltop = c.npmltop; a.e_rad = c.k_src; a.k_obs = c.k_obs; a.flows = c.flows;
+    a.nxy = p->nxy; a.lvl = p->nxy * c.nbatch; a.F = F; a.npv = p->P; a.v0n = (long long)c.nz * p->nxy;
+    a.bg = S.bg;
+    a.stretch = S.stretch;
+    a.dt = (T)c.deltat;
+    a.amp = amp;
+    a.A = S.A; a.S = S.ADV; a.D = S.D1; a.P = S.PP; a.RHO = S.RHO; a.PV = S.PV; a.SPV = S.SPV;
+    a.v0 = S.v0; a.PAT = S.pat; a.ADJ = p->adj ? S.ADJ : nullptr;
+    const S3Fft<T> fx{S.fx.twr, S.fx.twi, S.fx.kap, (T)c.stretchx}, fy{S.fy.twr, S.fy.twi, S.fy.kap, (T)c.stretchy};
     cudaError_t e;
 #define R3(call) do { e = (call); if (e != cudaSuccess) return e; } while (0)
-    R3(d3x<T>(p, X, S.D1, st));
-    R3(d3y<T>(p, X + F, S.D2, st));
-    R3(d3z<T>(p, X + 2 * F, S.D3, 1, st));
-    R3(launch_s3_div<T>(a, S.bg, S.D1, S.D2, S.D3, X + 2 * F, PSI, S.SPV, S.PP, S.RHO, st));
-    R3(d3x<T>(p, S.PP, S.GX, st));
-    R3(d3y<T>(p, S.PP, S.GY, st));
-    R3(d3z<T>(p, S.PP, S.GZ, 0, st));
-    if (c.flows) {
-        const long long q = (long long)c.nz * p->nxy;
-        for (int comp = 0; comp < 3; comp++) {
-            const T *v = X + (3 + comp) * F;
-            R3(d3x<T>(p, v, S.D1, st));
-            R3(d3y<T>(p, v, S.D2, st));
-            R3(d3z<T>(p, v, S.D3, 1, st));
-            R3(launch_s3_adv<T>(a, S.D1, S.D2, S.D3, S.v0, S.v0 + q, S.v0 + 2 * q, S.SCR + (3 + comp) * F, st));
-        }
+    for (int s = 0; s < 5; s++) {
+        a.b = (T)c.betas[s];
+        a.Xv = s == 0 ? S.A + 3 * F : S.XV + (s % 2) * 3 * F;
+        a.Xp = s == 0 ? nullptr : s == 1 ? S.A + 3 * F : S.XV + ((s - 1) % 2) * 3 * F;
+        R3(launch_s3x<T>(a, fx, s == 0 ? 0 : 1, st));
+        R3(launch_s3y<T>(a, fy, false, st));
+        R3(launch_s3z<T>(a, S.z[0].tab, S.z[1].tab, p->nch, p->L, false, st));
+        // the next stage's velocities, in the slot that this stage's passes have finished with; after the last
+        // stage the new v, in the state
+        a.bn = s < 4 ? (T)c.betas[s + 1] : a.dt;
+        a.Xn = s < 4 ? S.XV + ((s + 1) % 2) * 3 * F : S.A + 3 * F;
+        a.acc = s < 4 ? nullptr : acc;
+        R3(launch_s3z<T>(a, S.z[0].tab, S.z[1].tab, p->nch, p->L, true, st));
+        R3(launch_s3y<T>(a, fy, true, st));
     }
-    R3(launch_s3_rhs<T>(a, S.bg, X, S.SCR, S.GX, S.GY, S.GZ, PSI + P, S.SPV + P, S.RHO, S.pat, amp,
-                        p->adj ? S.ADJ : nullptr, c.k_obs, st));
+    R3(launch_s3x<T>(a, fx, 2, st));
+    R3(launch_s3_end<T>(a, c.filter_every == 2 && (p->time + 1) % 2 == 0, st));
 #undef R3
     return cudaSuccess;
 }
@@ -1715,9 +1724,9 @@ cudaError_t record3(sparc3d_plan *p, T *snap, cudaStream_t st)
     const long long F = p->F;
     cudaError_t e;
     if ((e = d3x<T>(p, S.A, S.D1, st)) != cudaSuccess) return e;
-    if ((e = d3y<T>(p, S.A + F, S.D2, st)) != cudaSuccess) return e;
-    if ((e = d3z<T>(p, S.A + 2 * F, S.D3, 1, st, 1)) != cudaSuccess) return e;
-    return launch_s3_record<T>(F, S.D1, S.D2, S.D3, S.A, S.SCR, snap, st);
+    if ((e = d3y<T>(p, S.A + F, S.PP, st)) != cudaSuccess) return e;
+    if ((e = d3z<T>(p, S.A + 2 * F, S.RHO, 1, st, 1)) != cudaSuccess) return e;
+    return launch_s3_record<T>(F, S.D1, S.PP, S.RHO, S.A, S.XV + 3 * F, snap, st);
 }
 
 template <typename T>
@@ -1726,8 +1735,7 @@ cudaError_t step3(sparc3d_plan *p, T *seis, int cap, int &nrec, cudaStream_t st,
 {
     Plan3<T> &S = plan3<T>(p);
     const sparc3d_config_t &c = p->cfg;
-    const long long F = p->F, P = p->P;
-    const S3Args a{c.nx, c.ny, c.nz, c.nbatch, c.npmlbot, c.npmltop, c.k_src, c.flows, p->nxy};
+    const long long F = p->F;
     const T amp = (T)(p->time >= 0 && p->time < (int)p->amp.size() ? p->amp[p->time] : 0.0);
     cudaError_t e;
     if (p->adj) {  // this step's adjoint forcing (the same in all five stages)
@@ -1742,19 +1750,9 @@ cudaError_t step3(sparc3d_plan *p, T *seis, int cap, int &nrec, cudaStream_t st,
         }
         if (e != cudaSuccess) return e;
     }
-    for (int s = 0; s < 5; s++) {
-        const T *X = S.A, *PSI = S.PV;
-        if (s > 0) {
-            e = launch_s3_stage_in<T>(6 * F, S.A, S.SCR, S.X, (T)c.betas[s], 2 * P, S.PV, S.SPV, S.PSI, st);
-            if (e != cudaSuccess) return e;
-            X = S.X;
-            PSI = S.PSI;
-        }
-        e = rhs3<T>(p, X, PSI, amp, st);
-        if (e != cudaSuccess) return e;
-    }
-    const int filter = (c.filter_every == 2 && (p->time + 1) % 2 == 0) ? 1 : 0;
-    e = launch_s3_end<T>(a, S.A, S.SCR, (T)c.deltat, filter, S.PV, S.SPV, st);
+    const int jrec = c.steps_out > 0 && p->time % c.steps_out == 0 ? p->time / c.steps_out - rec0 : -1;
+    const bool keep = snaps && jrec >= 0 && jrec < snap_cap;  // kernel-stage record jrec of the window
+    e = stages3<T>(p, amp, keep ? S.XV + 3 * F : nullptr, st);
     if (e != cudaSuccess) return e;
     if (c.steps_out > 0 && p->time % c.steps_out == 0) {
         if (seis && nrec < cap) {
@@ -1764,9 +1762,8 @@ cudaError_t step3(sparc3d_plan *p, T *seis, int cap, int &nrec, cudaStream_t st,
             if (e != cudaSuccess) return e;
         }
         nrec++;
-        const int j = p->time / c.steps_out - rec0;  // kernel-stage record j of the window
-        if (snaps && j >= 0 && j < snap_cap) {
-            e = record3<T>(p, snaps + (size_t)j * 5 * F, st);
+        if (keep) {
+            e = record3<T>(p, snaps + (size_t)jrec * 5 * F, st);
             if (e != cudaSuccess) return e;
         }
     }
@@ -1783,15 +1780,15 @@ cudaError_t kacc3(sparc3d_plan *p, const T *snap, double *out, cudaStream_t st)
     cudaError_t e;
 #define K3(call) do { e = (call); if (e != cudaSuccess) return e; } while (0)
     K3(d3x<T>(p, S.A + 3 * F, S.D1, st));
-    K3(d3y<T>(p, S.A + 4 * F, S.D2, st));
-    K3(d3z<T>(p, S.A + 5 * F, S.D3, 1, st, 1));
-    K3(launch_s3_kacc_div<T>(F, S.D1, S.D2, S.D3, snap, out, st));
+    K3(d3y<T>(p, S.A + 4 * F, S.PP, st));
+    K3(d3z<T>(p, S.A + 5 * F, S.RHO, 1, st, 1));
+    K3(launch_s3_kacc_div<T>(F, S.D1, S.PP, S.RHO, snap, out, st));
     for (int j = 0; j < 3; j++) {
         const T *vf = snap + (size_t)(1 + j) * F;
         K3(d3x<T>(p, vf, S.D1, st));
-        K3(d3y<T>(p, vf, S.D2, st));
-        K3(d3z<T>(p, vf, S.D3, 1, st, 1));
-        K3(launch_s3_kacc_v<T>(F, S.D1, S.D2, S.D3, S.A + (size_t)(3 + j) * F, out, st));
+        K3(d3y<T>(p, vf, S.PP, st));
+        K3(d3z<T>(p, vf, S.RHO, 1, st, 1));
+        K3(launch_s3_kacc_v<T>(F, S.D1, S.PP, S.RHO, S.A + (size_t)(3 + j) * F, out, st));
     }
 #undef K3
     return cudaSuccess;
@@ -1910,11 +1907,9 @@ int sparc3d_reset_state(sparc3d_plan_t *p, int time0, void *stream)
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const size_t es = p->cfg.precision == 32 ? sizeof(float) : sizeof(double);
     void *A = p->cfg.precision == 32 ? (void *)p->s32.A : (void *)p->s64.A;
-    void *SCR = p->cfg.precision == 32 ? (void *)p->s32.SCR : (void *)p->s64.SCR;
     void *PV = p->cfg.precision == 32 ? (void *)p->s32.PV : (void *)p->s64.PV;
     void *SPV = p->cfg.precision == 32 ? (void *)p->s32.SPV : (void *)p->s64.SPV;
     CK(cudaMemsetAsync(A, 0, 6 * p->F * es, st));
-    CK(cudaMemsetAsync(SCR, 0, 6 * p->F * es, st));
     CK(cudaMemsetAsync(PV, 0, 2 * p->P * es, st));
     CK(cudaMemsetAsync(SPV, 0, 2 * p->P * es, st));
     p->time = time0;

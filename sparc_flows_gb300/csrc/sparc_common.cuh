@@ -435,13 +435,31 @@ bool fft_size_supported(int n);
 
 // ------------------------------------------------------------------------------------------
 // 3-D displacement step (sparc_3d.cu).  Fields [nz][nb][ny][nx]; nxy = nx * ny.
-struct S3Args {
-    int nx, ny, nz, nb, npmlbot, npmltop, e_rad, flows;
-    long long nxy;
-};
 template <typename T>
 struct S3Bg {  // profiles in z ([nz]) and PML coefficients ([npmlbot + npmltop])
     const T *rhoinv, *rho0, *c2rho0, *gradp0_z, *gradrho0_z, *g, *source_dep, *az, *bz;
+};
+template <typename T>
+struct S3Fft {
+    const T *twr, *twi, *kap;
+    T stretch;
+};
+template <typename T>
+struct S3Step {  // one pass of stage s
+    int nx, ny, nz, nb, npmlbot, npmltop, e_rad, k_obs, flows;
+    long long nxy, lvl, F, npv, v0n;  // lvl = nb nxy, F = nz lvl, npv: one PML auxiliary, v0n: one flow component
+    S3Bg<T> bg;
+    const T *stretch;
+    T b, bn, dt, amp;  // beta of this stage and of the next (after the last: deltat), deltat
+    T *A;              // state [6][F]
+    T *Xv, *Xn;        // Xv [3][F] of this stage, of the next (the state's v after the last)
+    const T *Xp;       // of the stage before (null in the first)
+    T *S;              // advection sums [3][F] (with flow)
+    T *D, *P, *RHO;    // d xi_x/dx + d xi_y/dy, p, rho'
+    T *PV, *SPV;       // PML auxiliaries [2][npv]: psi_vz, psi_p, and their RHS
+    const T *v0;       // flow [3][v0n]
+    const T *PAT, *ADJ;  // source pattern, adjoint forcing of the step (null: none), [lvl]
+    T *acc;            // RHS of v [3][F] where the last stage's is recorded, or null
 };
 bool ddy_size_supported(int ny);
 template <typename T>
@@ -450,24 +468,23 @@ cudaError_t launch_ddy(const T *var, T *dvar, int nplanes, int nx, int ny, T str
 template <typename T>
 cudaError_t launch_s3_stage_in(long long n6, const T *A, const T *SCR, T *X, T beta, long long np, const T *PV,
                                const T *SPV, T *PSI, cudaStream_t st);
-template <typename T>
-cudaError_t launch_s3_div(const S3Args &a, const S3Bg<T> &bg, const T *D1, const T *D2, T *D3, const T *XIZ,
-                          const T *PSIVZ, T *SPSIVZ, T *PP, T *RHO, cudaStream_t st);
-template <typename T>
-cudaError_t launch_s3_adv(const S3Args &a, const T *D1, const T *D2, const T *D3, const T *V0X, const T *V0Y,
-                          const T *V0Z, T *OUT, cudaStream_t st);
 struct S3Lagr {  // the 7 LAGRANGE_INTERP weights of one step
     double w[7];
 };
+// mode 0: first stage, 1: later stages, 2: after the last
 template <typename T>
-cudaError_t launch_s3_rhs(const S3Args &a, const S3Bg<T> &bg, const T *X, T *SCR, const T *GX, const T *GY,
-                          const T *GZ, const T *PSIP, T *SPSIP, const T *RHO, const T *PAT, T amp, const T *ADJ,
-                          int k_obs, cudaStream_t st);
+cudaError_t launch_s3x(const S3Step<T> &a, const S3Fft<T> &f, int mode, cudaStream_t st);
+template <typename T>
+cudaError_t launch_s3y(const S3Step<T> &a, const S3Fft<T> &f, bool pressure, cudaStream_t st);
+template <typename T>
+cudaError_t launch_s3z(const S3Step<T> &a, const ZTab<T> &z0, const ZTab<T> &z1, int nch, int L, bool rhs, cudaStream_t st);
+template <typename T>
+cudaError_t launch_s3_end(const S3Step<T> &a, bool filter, cudaStream_t st);
 template <typename T>
 cudaError_t launch_s3_adjsrc(long long lvl, long long nxy, const double *rows, int nrows, int i0, const S3Lagr &w,
                              double scale, T *ADJ, cudaStream_t st);
 template <typename T>
-cudaError_t launch_s3_record(long long F, const T *D1, const T *D2, const T *D3, const T *A, const T *SCR, T *snap,
+cudaError_t launch_s3_record(long long F, const T *D1, const T *D2, const T *D3, const T *A, const T *ACC, T *snap,
                              cudaStream_t st);
 template <typename T>
 cudaError_t launch_s3_kacc_div(long long F, const T *D1, const T *D2, const T *D3, const T *snap, double *out,
@@ -475,10 +492,6 @@ cudaError_t launch_s3_kacc_div(long long F, const T *D1, const T *D2, const T *D
 template <typename T>
 cudaError_t launch_s3_kacc_v(long long F, const T *D1, const T *D2, const T *D3, const T *va, double *out,
                              cudaStream_t st);
-template <typename T>
-cudaError_t launch_s3_end(const S3Args &a, T *A, const T *SCR, T dt, int filter, T *PV, const T *SPV,
-                          cudaStream_t st);
-
 // 2-D sponge step (option 5, sparc_sponge.cu).  Fields [nz][nb][nx].
 struct S5Args {
     int nx, nz, nb, e_rad, i0, i1;  // filter columns [i0, i1]

@@ -45,15 +45,18 @@ struct WFft {
 // writes of every stage on distinct banks.
 template <typename T, int N>
 struct RowExchange {
+    static constexpr bool TWO = false;  // a warp's barrier costs less than a second buffer
     static constexpr int SPAN = N + N / 8;
     T *s;
     __device__ __forceinline__ void sync() const { __syncwarp(); }
+    template <int BUF>
     __device__ __forceinline__ void put(int i, T re, T im) const
     {
         const int q = i + (i >> 3);
         s[q] = re;
         s[SPAN + q] = im;
     }
+    template <int BUF>
     __device__ __forceinline__ void get(int i, T &re, T &im) const
     {
         const int q = i + (i >> 3);
@@ -65,27 +68,34 @@ struct RowExchange {
 // Column: a block transforms XL adjacent columns (neighbouring threads are neighbouring columns, so
 // global and shared accesses are contiguous), rows of XL values.  Where a row is half of the 32 banks
 // (16 columns of FP32), a row of padding per 8 keeps the two rows that a warp writes on different halves.
+// Two buffers in turn: a thread that writes one has passed the barrier behind every read of it, so an
+// exchange takes one block barrier instead of two.
 template <typename T, int N, int XL>
 struct ColExchange {
+    static constexpr bool TWO = true;
     static constexpr bool PAD = XL * sizeof(T) < 128;
     static constexpr int SPAN = (PAD ? N + N / 8 : N) * XL;
     T *s;
     int x;
     __device__ __forceinline__ void sync() const { __syncthreads(); }
     __device__ __forceinline__ int at(int i) const { return (PAD ? i + (i >> 3) : i) * XL + x; }
+    static constexpr size_t BYTES = (size_t)4 * SPAN * sizeof(T);  // both buffers
+    template <int BUF>
     __device__ __forceinline__ void put(int i, T re, T im) const
     {
-        s[at(i)] = re;
-        s[SPAN + at(i)] = im;
+        s[2 * BUF * SPAN + at(i)] = re;
+        s[(2 * BUF + 1) * SPAN + at(i)] = im;
     }
+    template <int BUF>
     __device__ __forceinline__ void get(int i, T &re, T &im) const
     {
-        re = s[at(i)];
-        im = s[SPAN + at(i)];
+        re = s[2 * BUF * SPAN + at(i)];
+        im = s[(2 * BUF + 1) * SPAN + at(i)];
     }
 };
 
-template <typename T, int N, int V, bool FOUR, int I, int NS, bool INV, class EX>
+// BUF: buffer of the stage's exchange.
+template <typename T, int N, int V, bool FOUR, int I, int NS, bool INV, int BUF, class EX>
 __device__ __forceinline__ void wfft_stages(T (&re)[V], T (&im)[V], const EX &ex, const T *__restrict__ twr,
                                             const T *__restrict__ twi, int t)
 {
@@ -118,18 +128,18 @@ __device__ __forceinline__ void wfft_stages(T (&re)[V], T (&im)[V], const EX &ex
             }
         }
         if constexpr (I + 1 < RX::count()) {
-            ex.sync();  // the buffer's last readers are done
+            if constexpr (!EX::TWO) ex.sync();  // the buffer's last readers are done
 #pragma unroll
             for (int q = 0; q < Q; q++) {
                 const int j = t + q * L, base = (j / NS) * NS * R + j % NS;
 #pragma unroll
-                for (int r = 0; r < R; r++) ex.put(base + r * NS, re[q + r * Q], im[q + r * Q]);
+                for (int r = 0; r < R; r++) ex.template put<BUF>(base + r * NS, re[q + r * Q], im[q + r * Q]);
             }
             ex.sync();
 #pragma unroll
-            for (int m = 0; m < V; m++) ex.get(t + L * m, re[m], im[m]);
+            for (int m = 0; m < V; m++) ex.template get<BUF>(t + L * m, re[m], im[m]);
         }
-        wfft_stages<T, N, V, FOUR, I + 1, NS * R, INV>(re, im, ex, twr, twi, t);
+        wfft_stages<T, N, V, FOUR, I + 1, NS * R, INV, 1 - BUF>(re, im, ex, twr, twi, t);
     }
 }
 
@@ -142,7 +152,7 @@ template <typename T, int N, int V, bool FOUR, class EX>
 __device__ __forceinline__ void wfft_deriv(T (&re)[V], T (&im)[V], const EX &ex, const T *__restrict__ twr,
                                            const T *__restrict__ twi, const T *__restrict__ kap, T scale, int t)
 {
-    wfft_stages<T, N, V, FOUR, 0, 1, false>(re, im, ex, twr, twi, t);
+    wfft_stages<T, N, V, FOUR, 0, 1, false, 0>(re, im, ex, twr, twi, t);
 #pragma unroll
     for (int m = 0; m < V; m++) {
         const T kk = mul_rn(__ldg(kap + t + (N / V) * m), scale);
@@ -150,7 +160,8 @@ __device__ __forceinline__ void wfft_deriv(T (&re)[V], T (&im)[V], const EX &ex,
         re[m] = mul_rn(-kk, b);  // rounded here, not contracted into the next stage's additions
         im[m] = mul_rn(kk, a);
     }
-    wfft_stages<T, N, V, FOUR, 0, 1, true>(re, im, ex, twr, twi, t);
+    // the forward transform's exchanges took the buffers 0, 1, ... in turn
+    wfft_stages<T, N, V, FOUR, 0, 1, true, (WRadices<T, N, FOUR>::count() - 1) % 2>(re, im, ex, twr, twi, t);
 }
 
 // ---- power-of-two row scales (pow2_scale_of): only the exponent of a row's largest |v| and whether
