@@ -234,6 +234,20 @@ int sparc_zband_host(int nz, int ibc, const double *b, double *x, const double *
 int sparc_colmat_apply(const double *W, int nz, const double *in, double *out, int nb, int nx, int i0, int i1,
                        int accumulate, void *stream);
 
+/* One reverse step of the discrete adjoint of STEP (step.f90:43-119) with MP_QUIET_PML_2D_DISPL and
+ * FILTER_VARS_2D, for an FP64 plan with flow and one shared background (no reference counterpart).
+ * sparc_adjoint_prepare builds the plan's transposed column tables (once; before a stream capture);
+ * sparc_adjoint_step recomputes the stages of the step from a0 [nb][4][nz][nx], Pz [nb][2][nzpml][nx], Px
+ * [nb][2][nz][2 npmlhor] with forcing [nb][nx] added to RHS v_z at the injection row (the plan's state is left as
+ * it is, its stage buffers are used), then takes la, lZ, lW, the adjoints of the step's outputs, to those of its
+ * inputs in place and adds the gradients with respect to v0x, v0z and c2rho0 of each solve to gx, gz, gc
+ * [nb][nz][nx].  work: sparc_adjoint_step_bytes device bytes.  Device pointers; no allocation, no synchronisation. */
+size_t sparc_adjoint_step_bytes(const sparc_plan_t *p);
+int sparc_adjoint_prepare(sparc_plan_t *p);
+int sparc_adjoint_step(sparc_plan_t *p, const double *a0, const double *Pz, const double *Px, const double *forcing,
+                       double *la, double *lZ, double *lW, double *gx, double *gz, double *gc, void *work, void *stream);
+
+
 /* Host-only FP64 evaluation of the partitioned compact-derivative algebra that the device
  * code applies (no GPU needed): x[nz][n1] = dbyd2(b, ibc) without the stretch factor, with
  * the same chunking as a plan whose chunks hold at most lmax rows.  For validating the

@@ -128,46 +128,10 @@ bool column_geometry(int nz, long long ncols, int nx, int &cw, int &nch, int &L)
     return true;
 }
 
-bool build_ztab(int nz, int ibc, int nch, int L, HostZTab &t)
+// Chunk-local factors, spikes and reduced inverse of the tridiagonal system (lowr, 1, uppr) of t.
+bool factor_ztab(HostZTab &t)
 {
-    if (nz < 8) return false;
-    t.nz = nz; t.ibc = ibc; t.nch = nch; t.L = L;
-    const float d2i = (float)(nz - 1);
-    const float C1 = d2i * 7.0f / 9.0f, C2 = d2i / 36.0f;  // dbyd2.f:82-83
-    t.c1 = C1; t.c2 = C2;
-    const float b1 = -(43.0f / 96.0f * d2i), b2 = -(5.0f / 6.0f * d2i), b3 = 9.0f / 8.0f * d2i,
-                b4 = 1.0f / 6.0f * d2i, b5 = -(1.0f / 96.0f * d2i);        // dbyd2.f:101-105
-    const float f1 = -(10.0f / 3.0f * d2i), f2 = -(3.0f * d2i), f3 = 6.0f * d2i, f4 = 1.0f / 3.0f * d2i;  // :119-122
-    const float alpha = 1.0f / 3.0f, alpha2 = 3.0f / 4.0f, gamma2 = 1.0f / 8.0f, alpha1 = 6.0f, beta1 = 3.0f;
-    const float cnst = 1.0f / (alpha2 - beta1 * gamma2);
-    const float up1 = (alpha1 * alpha2 - beta1) * cnst;
-    t.w5.assign((size_t)nz * 5, 0.0);
-    const double r1[5] = {b1, b2, b3, b4, b5};                 // row 1 on b[0..4]
-    const double rm2[5] = {-(double)b5, -(double)b4, -(double)b3, -(double)b2, -(double)b1};  // row nz-2 on b[nz-5..]
-    for (int j = 0; j < 5; j++) { t.w5[1 * 5 + j] = r1[j]; t.w5[(size_t)(nz - 2) * 5 + j] = rm2[j]; }
-    t.preset_row = -1;
-    if (ibc == 1 || ibc == 3) {  // row 0: 4-point closure, then preconditioned with row 1 (dbyd2.f:178-182)
-        const double r0[5] = {f1, f2, f3, f4, 0.0};
-        for (int j = 0; j < 5; j++) t.w5[j] = ((double)alpha2 * r0[j] - (double)beta1 * r1[j]) * (double)cnst;
-    }
-    if (ibc == 1 || ibc == 2) {  // row nz-1 on b[nz-5..nz-1] (dbyd2.f:139-142, 183-187)
-        const double rl[5] = {0.0, -(double)f4, -(double)f3, -(double)f2, -(double)f1};
-        for (int j = 0; j < 5; j++)
-            t.w5[(size_t)(nz - 1) * 5 + j] = ((double)alpha2 * rl[j] - (double)beta1 * rm2[j]) * (double)cnst;
-    }
-    if (ibc == 2) t.preset_row = 0;
-    if (ibc == 3) t.preset_row = nz - 1;
-    // matrix (dbyd2.f:151-196)
-    t.uppr.assign(nz, 0.0);
-    t.lowr.assign(nz, 0.0);
-    for (int k = 2; k <= nz - 3; k++) t.uppr[k] = alpha;
-    t.uppr[0] = (ibc % 2 == 0) ? 0.0 : (double)up1;
-    t.uppr[1] = alpha2;
-    t.uppr[nz - 2] = gamma2;
-    for (int k = 0; k < nz; k++) t.lowr[k] = t.uppr[nz - 1 - k];
-    t.lowr[nz - 1] = (ibc != 1 && ibc != 2) ? 0.0 : (double)up1;
-    t.uppr[nz - 1] = 0.0;
-    t.lowr[0] = 0.0;
+    const int nz = t.nz, nch = t.nch, L = t.L;
     // chunk-local factors and spikes
     t.ib.assign(nz, 0.0); t.lwib.assign(nz, 0.0); t.gm.assign(nz, 0.0);
     t.WL.assign(nz, 0.0); t.VU.assign(nz, 0.0);
@@ -211,6 +175,60 @@ bool build_ztab(int nz, int ibc, int nch, int L, HostZTab &t)
     if (!invert(M, n2)) return false;
     t.G = M;
     return true;
+}
+
+bool build_ztab(int nz, int ibc, int nch, int L, HostZTab &t)
+{
+    if (nz < 8) return false;
+    t.nz = nz; t.ibc = ibc; t.nch = nch; t.L = L;
+    const float d2i = (float)(nz - 1);
+    const float C1 = d2i * 7.0f / 9.0f, C2 = d2i / 36.0f;  // dbyd2.f:82-83
+    t.c1 = C1; t.c2 = C2;
+    const float b1 = -(43.0f / 96.0f * d2i), b2 = -(5.0f / 6.0f * d2i), b3 = 9.0f / 8.0f * d2i,
+                b4 = 1.0f / 6.0f * d2i, b5 = -(1.0f / 96.0f * d2i);        // dbyd2.f:101-105
+    const float f1 = -(10.0f / 3.0f * d2i), f2 = -(3.0f * d2i), f3 = 6.0f * d2i, f4 = 1.0f / 3.0f * d2i;  // :119-122
+    const float alpha = 1.0f / 3.0f, alpha2 = 3.0f / 4.0f, gamma2 = 1.0f / 8.0f, alpha1 = 6.0f, beta1 = 3.0f;
+    const float cnst = 1.0f / (alpha2 - beta1 * gamma2);
+    const float up1 = (alpha1 * alpha2 - beta1) * cnst;
+    t.w5.assign((size_t)nz * 5, 0.0);
+    const double r1[5] = {b1, b2, b3, b4, b5};                 // row 1 on b[0..4]
+    const double rm2[5] = {-(double)b5, -(double)b4, -(double)b3, -(double)b2, -(double)b1};  // row nz-2 on b[nz-5..]
+    for (int j = 0; j < 5; j++) { t.w5[1 * 5 + j] = r1[j]; t.w5[(size_t)(nz - 2) * 5 + j] = rm2[j]; }
+    t.preset_row = -1;
+    if (ibc == 1 || ibc == 3) {  // row 0: 4-point closure, then preconditioned with row 1 (dbyd2.f:178-182)
+        const double r0[5] = {f1, f2, f3, f4, 0.0};
+        for (int j = 0; j < 5; j++) t.w5[j] = ((double)alpha2 * r0[j] - (double)beta1 * r1[j]) * (double)cnst;
+    }
+    if (ibc == 1 || ibc == 2) {  // row nz-1 on b[nz-5..nz-1] (dbyd2.f:139-142, 183-187)
+        const double rl[5] = {0.0, -(double)f4, -(double)f3, -(double)f2, -(double)f1};
+        for (int j = 0; j < 5; j++)
+            t.w5[(size_t)(nz - 1) * 5 + j] = ((double)alpha2 * rl[j] - (double)beta1 * rm2[j]) * (double)cnst;
+    }
+    if (ibc == 2) t.preset_row = 0;
+    if (ibc == 3) t.preset_row = nz - 1;
+    // matrix (dbyd2.f:151-196)
+    t.uppr.assign(nz, 0.0);
+    t.lowr.assign(nz, 0.0);
+    for (int k = 2; k <= nz - 3; k++) t.uppr[k] = alpha;
+    t.uppr[0] = (ibc % 2 == 0) ? 0.0 : (double)up1;
+    t.uppr[1] = alpha2;
+    t.uppr[nz - 2] = gamma2;
+    for (int k = 0; k < nz; k++) t.lowr[k] = t.uppr[nz - 1 - k];
+    t.lowr[nz - 1] = (ibc != 1 && ibc != 2) ? 0.0 : (double)up1;
+    t.uppr[nz - 1] = 0.0;
+    t.lowr[0] = 0.0;
+    return factor_ztab(t);
+}
+
+// The table of the transposed system T^T x = rhs of t, same chunks (the stencil weights stay t's).
+bool transpose_ztab(const HostZTab &t, HostZTab &tt)
+{
+    tt = t;
+    for (int k = 0; k < t.nz; k++) {
+        tt.lowr[k] = k > 0 ? t.uppr[k - 1] : 0.0;
+        tt.uppr[k] = k < t.nz - 1 ? t.lowr[k + 1] : 0.0;
+    }
+    return factor_ztab(tt);
 }
 
 // The rows of the reduced inverse that the chunks' couplings use (x[first row - 1] and x[last row
@@ -596,6 +614,8 @@ struct sparc_plan {
     cudaStream_t g_stream = nullptr;
     double *d_srcw = nullptr;
     int *d_srcidx = nullptr;
+    DevZ<double> zT[4];  // transposed systems of ibc 1, 2, 3 (sparc_adjoint_prepare)
+    bool have_zT = false;
 };
 
 namespace {
@@ -1498,6 +1518,106 @@ int sparc_adjoint(sparc_plan_t *p, const void *fsn, int nfwd, int nsteps, double
                  : run_forward<double>(p, nsteps - done, -1.0, nullptr, nullptr, 0, 0, 1, st);
         if (rc != SPARC_OK) return rc;
     }
+    return SPARC_OK;
+}
+
+// Work of a reverse step, in doubles: the stage caches [5 stages][5][nb F], lX [4 nb F], x-derivatives [3 nb F],
+// ldxx [nb F], the auxiliaries' adjoints, and the tables of the recomputed stages.
+static size_t adjoint_work(const sparc_plan *p, size_t (&at)[8])
+{
+    const sparc_config_t &c = p->cfg;
+    const size_t nb = c.nbatch, NF = nb * c.nx * c.nz, nZ = nb * 2 * (c.npmlbot + c.npmltop) * c.nx,
+                 nW = nb * 2 * c.nz * 2 * c.npmlhor;
+    const size_t len[8] = {25 * NF, 4 * NF, 3 * NF, NF, nZ, nW, nb * c.nx, 16};
+    size_t o = 0;
+    for (int i = 0; i < 8; i++) {
+        at[i] = o;
+        o += len[i];
+    }
+    return o;
+}
+
+size_t sparc_adjoint_step_bytes(const sparc_plan_t *p)
+{
+    size_t at[8];
+    return p ? adjoint_work(p, at) * sizeof(double) : 0;
+}
+
+int sparc_adjoint_prepare(sparc_plan_t *p)
+{
+    if (!p) return fail(SPARC_ERR_ARG, "sparc_adjoint_prepare: null plan");
+    if (p->cfg.precision != 64 || !p->cfg.flows || p->cfg.bg_per_solve)
+        return fail(SPARC_ERR_STATE, "sparc_adjoint_prepare: needs an FP64 plan with flow and one shared background");
+    if (p->have_zT) return SPARC_OK;
+    for (int ibc = 1; ibc < 4; ibc++) {
+        HostZTab t;
+        if (!transpose_ztab(p->hz[ibc], t)) return fail(SPARC_ERR_SIZE, "sparc_adjoint_prepare: singular reduced system");
+        const cudaError_t e = upload_ztab<double>(t, p->zT[ibc], p->allocs);
+        if (e != cudaSuccess) return fail(SPARC_ERR_CUDA, std::string("sparc_adjoint_prepare: ") + cudaGetErrorString(e));
+    }
+    p->have_zT = true;
+    return SPARC_OK;
+}
+
+int sparc_adjoint_step(sparc_plan_t *p, const double *a0, const double *Pz, const double *Px, const double *forcing,
+                       double *la, double *lZ, double *lW, double *gx, double *gz, double *gc, void *work, void *stream)
+{
+    if (!p || !a0 || !Pz || !Px || !forcing || !la || !lZ || !lW || !gx || !gz || !gc || !work)
+        return fail(SPARC_ERR_ARG, "sparc_adjoint_step: null argument");
+    if (!p->have_zT || !p->have_bg) return fail(SPARC_ERR_STATE, "sparc_adjoint_step: sparc_adjoint_prepare and the background come first");
+    const cudaStream_t st = (cudaStream_t)stream;
+    const sparc_config_t &c = p->cfg;
+    size_t at[8];
+    adjoint_work(p, at);
+    double *w = (double *)work;
+    const size_t NF = (size_t)c.nbatch * c.nx * c.nz;
+    AdjArgs g{};
+    StepArgs<double> &a = g.a;
+    a = p->s64.a;
+    double *inj = w + at[6], *tab = w + at[7];
+    int *time = (int *)(tab + 8), *idx = (int *)(tab + 9);
+    CK(launch_adj_tables(time, idx, tab, inj, c.nbatch * c.nx, st));
+    // the five stages of the step from (a0, Pz, Px), keeping what the transposed stages need
+    a.A = const_cast<double *>(a0);
+    a.PZ = const_cast<double *>(Pz);
+    a.PX = const_cast<double *>(Px);
+    a.fsign = 1.0;
+    a.unstretch_top = p->unstretch_top;
+    a.seis = a.snaps = nullptr;
+    a.nrec_cap = 0;
+    a.d_time = time;
+    a.src_until = 0;
+    a.ntab = 1;
+    a.src_w = tab;
+    a.src_idx = idx;
+    a.src_rows = forcing;
+    a.nrows = 1;
+    a.inj_scale = inj;
+    for (int s = 1; s <= 5; s++) {
+        a.stage = s;
+        a.bs = c.betas[s - 1];
+        a.bsm1 = s >= 2 ? c.betas[s - 2] : 0.0;
+        a.slot_s = s % 3; a.slot_sm1 = (s - 1) % 3; a.slot_sm2 = (s + 1) % 3;
+        a.cache = w + at[0] + (size_t)(s - 1) * 5 * NF;
+        CK(launch_row_stage<double>(a, st));
+        CK(launch_col_stage<double>(a, st));
+    }
+    a.cache = nullptr;
+    g.la = la; g.lZ = lZ; g.lW = lW;
+    g.gx = gx; g.gz = gz; g.gc = gc;
+    g.lX = w + at[1]; g.D = w + at[2]; g.ldxx = w + at[3]; g.lZw = w + at[4]; g.lWw = w + at[5];
+    g.t1 = p->zT[1].tab; g.t2 = p->zT[2].tab; g.t3 = p->zT[3].tab;
+    g.unstretch_top = p->unstretch_top;
+    CK(launch_adj_filter(g, st));
+    CK(cudaMemcpyAsync(g.lZw, lZ, (at[5] - at[4]) * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    CK(cudaMemcpyAsync(g.lWw, lW, (at[6] - at[5]) * sizeof(double), cudaMemcpyDeviceToDevice, st));
+    for (int s = 4; s >= 0; s--) {
+        g.cf = s == 4 ? c.deltat : c.betas[s + 1];
+        g.cache = w + at[0] + (size_t)s * 5 * NF;
+        CK(launch_adj_row(g, s == 4 ? 0 : 1, st));
+        CK(launch_adj_col(g, st));
+    }
+    CK(launch_adj_row(g, 2, st));
     return SPARC_OK;
 }
 

@@ -98,6 +98,7 @@ __global__ void __launch_bounds__(CW *max_nch<T, CW>(), (min_blocks<T, CW>())) c
                     fd = __ldg(a.fdz + qb);
                 }
                 const T div = __ldg(a.DX + (size_t)b * F + q) + dzz;
+                if (sizeof(T) == 8 && a.cache) a.cache[(4 * (size_t)a.nb + b) * F + q] = div;
                 const T c2r = a.c2d ? __ldg(a.c2rho0 + (size_t)b * a.bg2 + q) : __ldg(a.c2rho0 + k);
                 const T gp = __ldg(a.gp0 + k) * fd, gr = __ldg(a.gr0 + k) * fd;
                 const T p = -c2r * div - gp * xz[m];
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(CW *max_nch<T, CW>(), (min_blocks<T, CW>())) c
                 T rv = T(0);
                 if (a.flows) {
                     const T dvxdz = zcorrect(a.z1, y2[m], k, xl2, xr2) * __ldg(a.stretch + k);
+                    if (sizeof(T) == 8 && a.cache) a.cache[((size_t)a.nb + b) * F + q] = dvxdz;
                     rv = __ldg(a.FXX + (size_t)b * F + q) - T(2) * a.fsign * __ldg(a.v0z + (size_t)b * a.bg2 + q) * dvxdz;
                 }
                 a.RVXP[(size_t)b * F + q] = rv;
@@ -191,6 +193,7 @@ __global__ void __launch_bounds__(CW *max_nch<T, CW>(), (min_blocks<T, CW>())) c
             if (k == a.k_inj) r += forcing;
             if (a.flows) {
                 const T dvzdz = zcorrect(a.z1, y2[m], k, xl2, xr2) * __ldg(a.stretch + k);
+                if (sizeof(T) == 8 && a.cache) a.cache[(3 * (size_t)a.nb + b) * F + q] = dvzdz;
                 r += __ldg(a.FXZ + (size_t)b * F + q) - T(2) * a.fsign * __ldg(a.v0z + (size_t)b * a.bg2 + q) * dvzdz;
             }
             if (k == 0 || x == 0 || x == nx - 1) r = T(0);

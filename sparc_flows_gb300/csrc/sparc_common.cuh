@@ -84,6 +84,22 @@ struct StepArgs {
     T *seis, *snaps;
     int nrec_cap;
     int rec0;  // records rec0 .. rec0 + nrec_cap - 1 are written, to slots 0 .. nrec_cap - 1
+    T *cache;  // FP64: d_x v_x, d_z v_x, d_x v_z, d_z v_z and div xi of this stage, [5][nb][nz][nx]; null: not kept
+};
+
+// One transposed stage of the discrete adjoint (sparc_adjoint.cu), FP64 with flow and a shared background.  The
+// adjoint of the stage's RHS is cf times that of the stage input of the stage after it (lX, lZw, lWw).
+struct AdjArgs {
+    StepArgs<double> a;
+    double cf;
+    double *la, *lZ, *lW;        // adjoints of the state [nb][4][nz][nx] and PML auxiliaries, accumulated over the stages
+    double *lX, *lZw, *lWw;      // of the stage input, in and out
+    double *D;                   // x-derivatives [3][nb][nz][nx]: of v0x lRvx, v0x lRvz, lgpx
+    double *ldxx;                // adjoint of d xi_x/dx [nb][nz][nx]
+    const double *cache;         // the stage's [5][nb][nz][nx] (StepArgs::cache)
+    double *gx, *gz, *gc;        // gradients with respect to v0x, v0z, c2rho0, per solve
+    ZTab<double> t1, t2, t3;     // transposed tridiagonal systems of ibc 1, 2, 3
+    double unstretch_top;
 };
 
 template <typename T>
@@ -432,6 +448,13 @@ template <typename T>
 cudaError_t launch_kacc(const KAccArgs<T> &k, cudaStream_t st);
 
 bool fft_size_supported(int n);
+
+// mode 0: first transposed stage (no ldxx yet), 1: later, 2: after the last (ldxx alone)
+cudaError_t launch_adj_row(const AdjArgs &g, int mode, cudaStream_t st);
+cudaError_t launch_adj_col(const AdjArgs &g, cudaStream_t st);
+// mu = (filter)^T la, into la and lX; and the small tables of the recomputed stages
+cudaError_t launch_adj_filter(const AdjArgs &g, cudaStream_t st);
+cudaError_t launch_adj_tables(int *time, int *idx, double *w, double *inj, int n, cudaStream_t st);
 
 // ------------------------------------------------------------------------------------------
 // 3-D displacement step (sparc_3d.cu).  Fields [nz][nb][ny][nx]; nxy = nx * ny.

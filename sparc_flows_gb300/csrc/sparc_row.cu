@@ -221,8 +221,13 @@ __global__ void __launch_bounds__(ROW_WPB *WARP) row_stage_kernel(StepArgs<T> a,
 #pragma unroll
     for (int m = 0; m < V; m++) {
         const size_t q = (size_t)r.b * r.F + r.ro + t + L * m;
-        a.FXX[q] = wv[m] * scale_out(re[m], sr);
-        a.FXZ[q] = wv[m] * scale_out(im[m], si);
+        const T dvx = scale_out(re[m], sr), dvz = scale_out(im[m], si);
+        a.FXX[q] = wv[m] * dvx;
+        a.FXZ[q] = wv[m] * dvz;
+        if (sizeof(T) == 8 && a.cache) {
+            a.cache[q] = dvx;
+            a.cache[2 * a.nb * r.F + q] = dvz;
+        }
     }
 }
 

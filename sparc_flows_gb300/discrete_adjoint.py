@@ -7,8 +7,8 @@ The reference has no discrete adjoint: its adjoint run is a time-reversed forwar
 flow negated (driver.f90:144-147) whose kernels match finite differences only to discretisation
 accuracy.  Here the forward solve is the device step of the plan (fused kernels, sparc_forward);
 the backward pass replays it segment by segment from HBM checkpoints (sparc_checkpoint_save /
-load), recomputes the five stage inputs of each step with the same operators applied one at a
-time, and applies the transposed stages in reverse order:
+load), recomputes the five stage inputs of each step and applies the transposed stages in reverse
+order:
 
   x-derivative  D_x (spectral, Nyquist bin dropped) is real antisymmetric: D_x^T = -D_x, applied
                 with the device ddx;
@@ -28,8 +28,10 @@ derivative with respect to v0 is accumulated from the recomputed stage inputs, a
 curl(rho0 c psi) / rho0 (driver.f90:94-115) is linear in psi, so its transpose gives dL/dpsi.
 The sound speed enters through p = -c^2 rho0 div - ...: dL/d(c^2 rho0) = -sum lambda_p div over
 stages and steps (the exact counterpart of kernel_c, with the PML profiles held fixed).
-Pointwise algebra runs as device tensor arithmetic; every derivative, transposed derivative and
-transposed filter is one of the plan's kernels.
+StepOperators applies every operator one at a time (pointwise algebra as device tensor arithmetic,
+each derivative, transposed derivative and transposed filter one kernel): the form the tests take
+apart.  ExactGradient runs the fused reverse step (sparc_adjoint_step): the plan's own row and column
+passes recompute the stages, one x and one z pass per stage transpose them.
 """
 from __future__ import annotations
 
@@ -322,29 +324,26 @@ class ExactGradient:
 
     def _static(self):
         """Static device buffers of one reverse step: the state before the step, the adjoints,
-        the gradient accumulators, the forcing row and the flow."""
+        the gradient accumulators of each solve, the forcing row and the work of sparc_adjoint_step."""
         if getattr(self, "_s", None) is None:
             ops, dev = self.ops, self.ws.dev
             sa, sz, sw = ((ops.nb, 4, ops.nz, ops.nx), (ops.nb, 2, ops.nzpml, ops.nx), (ops.nb, 2, ops.nz, ops.nhx))
+            sg = (ops.nb, ops.nz, ops.nx)
             z = lambda sh: torch.zeros(sh, dtype=F64, device=dev)  # noqa: E731
-            self._s = dict(a=z(sa), Pz=z(sz), Px=z(sw), la=z(sa), lZ=z(sz), lW=z(sw), gx=z((ops.nz, ops.nx)),
-                           gz=z((ops.nz, ops.nx)), gc=z((ops.nz, ops.nx)), f=z((ops.nb, ops.nx)),
-                           v0x=z((ops.nz, ops.nx)),
-                           v0z=z((ops.nz, ops.nx)))
+            self._s = dict(a=z(sa), Pz=z(sz), Px=z(sw), la=z(sa), lZ=z(sz), lW=z(sw), gx=z(sg),
+                           gz=z(sg), gc=z(sg), f=z((ops.nb, ops.nx)))
+            self._work = torch.empty(int(self.ws.L.sparc_adjoint_step_bytes(self.ws.plan)), dtype=torch.uint8,
+                                     device=dev)
+            capi.check(self.ws.L.sparc_adjoint_prepare(self.ws.plan), "sparc_adjoint_prepare")
         return self._s
 
     def _reverse_step(self):
         """Recompute the stages of one step from the static state and apply the transposed step
-        to the static adjoints in place, accumulating the flow gradient."""
-        S, ops = self._s, self.ops
-        _, _, _, caches = ops.step(S["a"], S["Pz"], S["Px"], S["v0x"], S["v0z"], S["f"])
-        la, lZ, lW, g1, g2, g3 = ops.step_T(S["la"], S["lZ"], S["lW"], S["v0x"], S["v0z"], caches)
-        S["la"].copy_(la)
-        S["lZ"].copy_(lZ)
-        S["lW"].copy_(lW)
-        S["gx"].add_(g1)
-        S["gz"].add_(g2)
-        S["gc"].add_(g3)
+        to the static adjoints in place, accumulating the gradients (sparc_adjoint_step: the fused
+        counterpart of StepOperators.step and step_T)."""
+        S = self._s
+        args = [_ptr(S[k]) for k in ("a", "Pz", "Px", "f", "la", "lZ", "lW", "gx", "gz", "gc")]
+        capi.check(self.ws.L.sparc_adjoint_step(self.ws.plan, *args, _ptr(self._work), _stream()), "sparc_adjoint_step")
 
     def _run_reverse_step(self):
         """One reverse step, replayed from a CUDA graph when capture works (the same launches
@@ -380,8 +379,6 @@ class ExactGradient:
         S = self._static()
         for k in ("la", "lZ", "lW", "gx", "gz", "gc"):
             S[k].zero_()
-        S["v0x"].copy_(ws.bg["v0x"][0])
-        S["v0z"].copy_(ws.bg["v0z"][0])
         grad_rec = grad_rec.to(device=ws.dev, dtype=F64)
         for m in range(self.nseg - 1, -1, -1):
             n0, n1 = m * self.seg, min((m + 1) * self.seg, n)
@@ -400,7 +397,7 @@ class ExactGradient:
                 else:
                     S["f"].copy_(fc)
                 self._run_reverse_step()
-        self.last = {"v0x": S["gx"].clone(), "v0z": S["gz"].clone(), "c2rho0": S["gc"].clone()}
+        self.last = {"v0x": S["gx"].sum(0), "v0z": S["gz"].sum(0), "c2rho0": S["gc"].sum(0)}
         return self.psi_gradient(self.last["v0x"], self.last["v0z"])
 
     def set_c2rho0(self, c2rho0: torch.Tensor):
