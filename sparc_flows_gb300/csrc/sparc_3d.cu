@@ -129,19 +129,6 @@ bool ddy_size_supported(int ny)
 }
 
 // ---------------------------------------------------------------------------------------------
-template <typename T>
-__global__ void __launch_bounds__(S3_THREADS) s3_stage_in(long long n6, const T *__restrict__ A,
-                                                          const T *__restrict__ SCR, T *__restrict__ X, T beta,
-                                                          long long np, const T *__restrict__ PV,
-                                                          const T *__restrict__ SPV, T *__restrict__ PSI)
-{
-    const long long stride = (long long)gridDim.x * S3_THREADS;
-    for (long long i = (long long)blockIdx.x * S3_THREADS + threadIdx.x; i < n6 + np; i += stride) {
-        if (i < n6) X[i] = A[i] + beta * SCR[i];
-        else PSI[i - n6] = PV[i - n6] + beta * SPV[i - n6];
-    }
-}
-
 // PML level of row k (-1 outside the vertical PML).
 template <typename T>
 __device__ __forceinline__ int s3_pml(const S3Step<T> &a, int k)
@@ -688,14 +675,6 @@ static unsigned s3_grid(long long n)
     return (unsigned)(g < 152LL * 16 ? g : 152LL * 16);
 }
 
-template <typename T>
-cudaError_t launch_s3_stage_in(long long n6, const T *A, const T *SCR, T *X, T beta, long long np, const T *PV,
-                               const T *SPV, T *PSI, cudaStream_t st)
-{
-    s3_stage_in<T><<<s3_grid(n6 + np), S3_THREADS, 0, st>>>(n6, A, SCR, X, beta, np, PV, SPV, PSI);
-    return cudaGetLastError();
-}
-
 template <typename T, int N>
 static cudaError_t s3x_n(const S3Step<T> &a, const S3Fft<T> &f, int mode, cudaStream_t st)
 {
@@ -816,8 +795,6 @@ cudaError_t launch_s3_kacc_v(long long F, const T *D1, const T *D2, const T *D3,
 #define S3_INST(T)                                                                                                    \
     template cudaError_t launch_ddy<T>(const T *, T *, int, int, int, T, const T *, const T *, const T *,            \
                                        cudaStream_t);                                                                \
-    template cudaError_t launch_s3_stage_in<T>(long long, const T *, const T *, T *, T, long long, const T *,        \
-                                               const T *, T *, cudaStream_t);                                        \
     template cudaError_t launch_s3x<T>(const S3Step<T> &, const S3Fft<T> &, int, cudaStream_t);                      \
     template cudaError_t launch_s3y<T>(const S3Step<T> &, const S3Fft<T> &, bool, cudaStream_t);                     \
     template cudaError_t launch_s3z<T>(const S3Step<T> &, const ZTab<T> &, const ZTab<T> &, int, int, bool,          \

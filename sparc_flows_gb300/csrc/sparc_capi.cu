@@ -2157,10 +2157,10 @@ namespace {
 template <typename T>
 struct Plan5 {
     std::vector<void *> allocs;
-    T *A = nullptr, *SCR = nullptr, *X = nullptr, *DVX = nullptr, *DVZ = nullptr, *GX = nullptr, *GZ = nullptr;
+    T *A = nullptr, *SCR = nullptr;
+    T *DX = nullptr;  // x-derivatives [2][F] of v_x, p; option 12: [4][F], of the flux and b_z too
     T *prof = nullptr, *pat = nullptr;
-    T *PV = nullptr, *SPV = nullptr, *PSI = nullptr;  // PML auxiliaries [npa][npml][nb][nx] (options 6, 12)
-    T *FLUX = nullptr, *DZBX = nullptr, *DZF = nullptr, *DXF = nullptr, *DXBZ = nullptr;  // option 12 work
+    T *PV = nullptr, *SPV = nullptr;  // PML auxiliaries [npa][npml][nb][nx] (options 6, 12)
     T *MAG = nullptr;                                  // option 12: box, boz, curlboy [3][nz][nx]
     DevZ<T> z1;
     DevFFT<T> fx;
@@ -2172,7 +2172,7 @@ struct Plan5 {
 
 struct sparc5_plan {
     sparc5_config_t cfg{};
-    int nch = 0, L = 0;
+    int nch = 0, L = 0, cw = 8;  // chunks of the z pass and its block width
     HostZTab hz1;
     Plan5<float> s32;
     Plan5<double> s64;
@@ -2203,12 +2203,11 @@ int alloc_plan5(sparc5_plan *p)
     const sparc5_config_t &c = p->cfg;
     const size_t F = (size_t)p->F, nz = c.nz, npml = npml5(c), nf = nf5(c);
     const size_t P2 = (size_t)npa5(c) * npml * c.nbatch * c.nx;
-    const size_t FM = c.option == 12 ? F : 0, NM = c.option == 12 ? 3 * nz * (size_t)c.nx : 0;
+    const size_t NM = c.option == 12 ? 3 * nz * (size_t)c.nx : 0;
     struct Req { T **ptr; size_t n; };
-    std::vector<Req> reqs = {{&S.A, nf * F}, {&S.SCR, nf * F}, {&S.X, nf * F}, {&S.DVX, F}, {&S.DVZ, F}, {&S.GX, F},
-                             {&S.GZ, F}, {&S.prof, 9 * nz + 2 * npml}, {&S.pat, (size_t)c.nbatch * c.nx},
-                             {&S.PV, P2}, {&S.SPV, P2}, {&S.PSI, P2}, {&S.FLUX, FM}, {&S.DZBX, FM}, {&S.DZF, FM},
-                             {&S.DXF, FM}, {&S.DXBZ, FM}, {&S.MAG, NM}};
+    std::vector<Req> reqs = {{&S.A, nf * F}, {&S.SCR, nf * F}, {&S.DX, (c.option == 12 ? 4 : 2) * F},
+                             {&S.prof, 9 * nz + 2 * npml}, {&S.pat, (size_t)c.nbatch * c.nx},
+                             {&S.PV, P2}, {&S.SPV, P2}, {&S.MAG, NM}};
     for (auto &r : reqs) {
         void *ptr = nullptr;
         const size_t bytes = std::max<size_t>(r.n, 1) * sizeof(T);
@@ -2249,42 +2248,29 @@ cudaError_t step5(sparc5_plan *p, T *seis, int cap, int &nrec, cudaStream_t st)
     Plan5<T> &S = plan5<T>(p);
     const sparc5_config_t &c = p->cfg;
     const long long F = p->F, lvl = (long long)c.nbatch * c.nx;
-    const bool pml = c.option == 6 || c.option == 12, mhd = c.option == 12;
-    const int nf = nf5(c);
-    const S5Args a{c.nx, c.nz, c.nbatch, c.k_src, c.filter_all_x ? 0 : c.npmlhor - 1,
-                   c.filter_all_x ? c.nx - 1 : c.nx - c.npmlhor, pml ? c.npmlbot : 0, pml ? c.npmltop : 0,
-                   nf, npa5(c)};
-    const long long P2 = (long long)npa5(c) * npml5(c) * lvl;
-    const T amp = (T)(p->time >= 0 && p->time < (int)p->amp.size() ? p->amp[p->time] : 0.0);
+    const bool pml = c.option == 6 || c.option == 12;
+    S5Step<T> a{};
+    a.nx = c.nx; a.nz = c.nz; a.nb = c.nbatch; a.option = c.option; a.e_rad = c.k_src;
+    a.i0 = c.filter_all_x ? 0 : c.npmlhor - 1;
+    a.i1 = c.filter_all_x ? c.nx - 1 : c.nx - c.npmlhor;
+    a.npmlbot = pml ? c.npmlbot : 0;
+    a.npmltop = pml ? c.npmltop : 0;
+    a.lvl = lvl; a.F = F;
+    a.bg = S.bg;
+    a.stretch = S.stretch;
+    a.dt = (T)c.deltat;
+    a.amp = (T)(p->time >= 0 && p->time < (int)p->amp.size() ? p->amp[p->time] : 0.0);
+    a.A = S.A; a.SCR = S.SCR; a.DX = S.DX; a.PV = S.PV; a.SPV = S.SPV; a.PAT = S.pat;
+    const S3Fft<T> fx{S.fx.twr, S.fx.twi, S.fx.kap, (T)c.stretchx};
     cudaError_t e;
     for (int s = 0; s < 5; s++) {
-        const T *X = S.A, *PSI = S.PV;
-        if (s > 0) {
-            e = launch_s3_stage_in<T>(nf * F, S.A, S.SCR, S.X, (T)c.betas[s], P2, S.PV, S.SPV, S.PSI, st);
-            if (e != cudaSuccess) return e;
-            X = S.X;
-            PSI = S.PSI;
-        }
-        const int nrows = c.nz * c.nbatch;
-        e = launch_ddx<T>(X + F, S.DVX, nrows, c.nx, (T)c.stretchx, S.fx.twr, S.fx.twi, S.fx.kap, st);
-        if (e == cudaSuccess) e = launch_ddx<T>(X + 4 * F, S.GX, nrows, c.nx, (T)c.stretchx, S.fx.twr, S.fx.twi, S.fx.kap, st);
-        if (e == cudaSuccess) e = launch_ddz<T>(S.z1.tab, p->nch, p->L, X + 3 * F, S.DVZ, (int)lvl, c.nz, nullptr, S.stretch, 0, st);
-        if (e == cudaSuccess) e = launch_ddz<T>(S.z1.tab, p->nch, p->L, X + 4 * F, S.GZ, (int)lvl, c.nz, nullptr, S.stretch, 0, st);
-        if (e == cudaSuccess && mhd) {  // flux, d flux/dx, d flux/dz, d b_z/dx, d b_x/dz
-            e = launch_s12_flux<T>(a, S.bg, X, S.FLUX, st);
-            if (e == cudaSuccess) e = launch_ddx<T>(S.FLUX, S.DXF, nrows, c.nx, (T)c.stretchx, S.fx.twr, S.fx.twi, S.fx.kap, st);
-            if (e == cudaSuccess) e = launch_ddx<T>(X + 7 * F, S.DXBZ, nrows, c.nx, (T)c.stretchx, S.fx.twr, S.fx.twi, S.fx.kap, st);
-            if (e == cudaSuccess) e = launch_ddz<T>(S.z1.tab, p->nch, p->L, S.FLUX, S.DZF, (int)lvl, c.nz, nullptr, S.stretch, 0, st);
-            if (e == cudaSuccess) e = launch_ddz<T>(S.z1.tab, p->nch, p->L, X + 5 * F, S.DZBX, (int)lvl, c.nz, nullptr, S.stretch, 0, st);
-        }
-        if (e == cudaSuccess)
-            e = mhd ? launch_s12_rhs<T>(a, S.bg, X, S.SCR, S.DVX, S.DVZ, S.GX, S.GZ, S.DZBX, S.DZF, S.DXF, S.DXBZ, PSI,
-                                        S.SPV, S.pat, amp, st)
-                : pml ? launch_s6_rhs<T>(a, S.bg, X, S.SCR, S.DVX, S.DVZ, S.GX, S.GZ, PSI, S.SPV, S.pat, amp, st)
-                      : launch_s5_rhs<T>(a, S.bg, X, S.SCR, S.DVX, S.DVZ, S.GX, S.GZ, S.pat, amp, st);
+        a.first = s == 0;
+        a.b = (T)c.betas[s];
+        e = launch_s5x<T>(a, fx, st);
+        if (e == cudaSuccess) e = launch_s5z<T>(a, S.z1.tab, p->nch, p->L, p->cw, st);
         if (e != cudaSuccess) return e;
     }
-    e = launch_s5_end<T>(a, S.A, S.SCR, (T)c.deltat, pml ? S.PV : nullptr, S.SPV, st);
+    e = launch_s5_end<T>(a, pml ? (long long)npa5(c) * npml5(c) * lvl : 0, st);
     if (e != cudaSuccess) return e;
     if (c.steps_out > 0 && p->time % c.steps_out == 0) {
         if (seis && nrec < cap) {
@@ -2318,8 +2304,8 @@ int set_bg5(sparc5_plan *p, const sparc5_background_t *bg, cudaStream_t st)
         CK(cast_to<T>(bg->box, box, NM, st));
         CK(cast_to<T>(bg->boz, boz, NM, st));
         CK(launch_ddz<T>(S.z1.tab, p->nch, p->L, box, curl, nx, nz, nullptr, S.stretch, 0, st));
-        CK(launch_ddx<T>(boz, S.DXBZ, nz, nx, (T)p->cfg.stretchx, S.fx.twr, S.fx.twi, S.fx.kap, st));
-        CK(launch_s5_axpy<T>((long long)NM, curl, S.DXBZ, T(-1), st));
+        CK(launch_ddx<T>(boz, S.DX, nz, nx, (T)p->cfg.stretchx, S.fx.twr, S.fx.twi, S.fx.kap, st));
+        CK(launch_s5_axpy<T>((long long)NM, curl, S.DX, T(-1), st));
     }
     return SPARC_OK;
 }
@@ -2344,7 +2330,12 @@ int sparc5_plan_create(const sparc5_config_t *cfg, sparc5_plan_t **out)
     sparc5_plan *p = new sparc5_plan();
     p->cfg = *cfg;
     p->F = (long long)cfg->nx * cfg->nbatch * cfg->nz;
-    if (!chunking(cfg->nz, 16, p->nch, p->L) || !build_ztab(cfg->nz, 1, p->nch, p->L, p->hz1)) {
+    // blocks of 32 columns where they fill the SMs (FP32), as column_geometry for FP64
+    const long long ncols = (long long)cfg->nx * cfg->nbatch;
+    const bool chunked = chunking(cfg->nz, 16, p->nch, p->L);
+    p->cw = cfg->precision == 32 && ncols >= 32 * 152 ? 32 : 8;
+    if (chunked && cfg->precision == 64) column_geometry(cfg->nz, ncols, cfg->nx, p->cw, p->nch, p->L);
+    if (!chunked || !build_ztab(cfg->nz, 1, p->nch, p->L, p->hz1)) {
         delete p;
         return fail(SPARC_ERR_SIZE, "sparc5_plan_create: nz too large for the column chunking");
     }

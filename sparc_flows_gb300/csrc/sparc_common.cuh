@@ -488,9 +488,6 @@ bool ddy_size_supported(int ny);
 template <typename T>
 cudaError_t launch_ddy(const T *var, T *dvar, int nplanes, int nx, int ny, T stretchy, const T *twr, const T *twi,
                        const T *kap, cudaStream_t st);
-template <typename T>
-cudaError_t launch_s3_stage_in(long long n6, const T *A, const T *SCR, T *X, T beta, long long np, const T *PV,
-                               const T *SPV, T *PSI, cudaStream_t st);
 struct S3Lagr {  // the 7 LAGRANGE_INTERP weights of one step
     double w[7];
 };
@@ -516,30 +513,31 @@ template <typename T>
 cudaError_t launch_s3_kacc_v(long long F, const T *D1, const T *D2, const T *D3, const T *va, double *out,
                              cudaStream_t st);
 // 2-D sponge step (option 5, sparc_sponge.cu).  Fields [nz][nb][nx].
-struct S5Args {
-    int nx, nz, nb, e_rad, i0, i1;  // filter columns [i0, i1]
-    int npmlbot, npmltop;           // options 6 and 12
-    int nf, npa;                    // fields of the state (5 or 8), PML auxiliaries (0, 2 or 4)
-};
 template <typename T>
 struct S5Bg {  // profiles in z; az, bz [npmlbot + npmltop] (options 6, 12)
     const T *rhoinv, *rho0, *c2rho0, *gradp0_z, *gradrho0_z, *g, *source_dep, *sponge, *az, *bz;
     const T *box, *boz, *curl;  // option 12: background field and curlboy, [nz][nx]
 };
 template <typename T>
-cudaError_t launch_s5_rhs(const S5Args &a, const S5Bg<T> &bg, const T *X, T *SCR, const T *DVX, const T *DVZ,
-                          const T *GX, const T *GZ, const T *PAT, T amp, cudaStream_t st);
+struct S5Step {  // one pass of a stage
+    int nx, nz, nb, option, e_rad, i0, i1;  // filter columns [i0, i1]
+    int npmlbot, npmltop, first;            // first: the first stage (stage input = A)
+    long long lvl, F;                       // nb nx, nz lvl
+    S5Bg<T> bg;
+    const T *stretch;
+    T b, dt, amp;
+    T *A, *SCR;     // state and RHS [nf][F]
+    T *DX;          // x-derivatives [2 or 4][F]: of v_x, p, flux, b_z
+    T *PV, *SPV;    // PML auxiliaries and their RHS
+    const T *PAT;
+};
 template <typename T>
-cudaError_t launch_s6_rhs(const S5Args &a, const S5Bg<T> &bg, const T *X, T *SCR, const T *DVX, const T *DVZ,
-                          const T *GX, const T *GZ, const T *PSI, T *SPSI, const T *PAT, T amp, cudaStream_t st);
+cudaError_t launch_s5x(const S5Step<T> &a, const S3Fft<T> &f, cudaStream_t st);
+// cw: columns of a block (FP32 32 or 8; FP64 8, 4 or 2)
 template <typename T>
-cudaError_t launch_s5_end(const S5Args &a, T *A, const T *SCR, T dt, T *PV, const T *SPV, cudaStream_t st);
+cudaError_t launch_s5z(const S5Step<T> &a, const ZTab<T> &z1, int nch, int L, int cw, cudaStream_t st);
 template <typename T>
-cudaError_t launch_s12_flux(const S5Args &a, const S5Bg<T> &bg, const T *X, T *FLUX, cudaStream_t st);
-template <typename T>
-cudaError_t launch_s12_rhs(const S5Args &a, const S5Bg<T> &bg, const T *X, T *SCR, const T *DVX, const T *DVZ,
-                           const T *GX, const T *GZ, const T *DZBX, const T *DZF, const T *DXF, const T *DXBZ,
-                           const T *PSI, T *SPSI, const T *PAT, T amp, cudaStream_t st);
+cudaError_t launch_s5_end(const S5Step<T> &a, long long npv, cudaStream_t st);
 template <typename T>
 cudaError_t launch_s5_axpy(long long n, T *Y, const T *X, T a, cudaStream_t st);
 

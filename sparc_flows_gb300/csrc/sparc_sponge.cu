@@ -5,88 +5,219 @@
 // the Lorentz force, and the magnetic part of PML_BOUNDARY_ACCOUNTING_2D, 1162-1200).
 //
 // Fields are [nz][nb][nx] (level-major, the batch inside a level, as the 3-D step), the state
-// five of them: rho, v_x, v_y (zero in 2-D), v_z, p (initialize.f90:500-504).  One RK stage:
-// X = A + beta SCR (s3_stage_in), x passes of v_x and p (the spectral row pass), z passes of
-// v_z and p (the compact column solve, ibc 1), then s5_rhs_kernel: continuity, momentum with
-// pressure gradient, buoyancy, sponge and source, pressure; the top and bottom rows of the
-// momentum and pressure RHS zero.  End of step: s5_end_kernel, a += dt scr and FILTER_VARS_2D
-// (physics2d.f90:509-560) down each column from a register window, in place.
-#include "sparc_common.cuh"
+// five of them: rho, v_x, v_y, v_z, p (initialize.f90:500-504); with option 12 also b_x, b_y, b_z.  v_y and b_y
+// are zero in 2-D and have no RHS: no pass touches them.  One RK stage is two passes, each forming the stage
+// input A + beta SCR of the fields it needs as it reads them:
+//   x pass (s5x_kernel)  d v_x/dx and d p/dx in one transform; with option 12 d flux/dx and d b_z/dx, the flux
+//                        -(v_x boz - v_z box) formed on the way in
+//   z pass (s5z_kernel)  the compact derivatives (ibc 1) of p and v_z (and of the flux and b_x) of a column tile in
+//                        shared memory, then the whole right-hand side of the tile's rows, SCR in place
+// End of step (s5_end_kernel): a += dt scr and FILTER_VARS_2D (physics2d.f90:509-560) from a column tile of one
+// field in shared memory, in place.
+#include "sparc_wfft.cuh"
 
 namespace sparc {
 
-constexpr int S5_THREADS = 256;
+constexpr int S5_THREADS = 256, S5X_WARPS = 2;
 
-template <typename T>
-__global__ void __launch_bounds__(S5_THREADS) s5_rhs_kernel(S5Args a, S5Bg<T> bg, const T *__restrict__ X,
-                                                            T *__restrict__ SCR, const T *__restrict__ DVX,
-                                                            const T *__restrict__ DVZ, const T *__restrict__ GX,
-                                                            const T *__restrict__ GZ, const T *__restrict__ PAT, T amp)
+// ---- x pass: a unit of WFft lanes is one row and one pair of fields (pair 1: option 12)
+template <typename T, int N>
+__global__ void __launch_bounds__(S5X_WARPS *WARP) s5x_kernel(S5Step<T> a, S3Fft<T> f)
 {
-    const long long lvl = (long long)a.nb * a.nx, n = lvl * a.nz, F = n;
-    const long long stride = (long long)gridDim.x * S5_THREADS;
-    for (long long i = (long long)blockIdx.x * S5_THREADS + threadIdx.x; i < n; i += stride) {
-        const int k = (int)(i / lvl);
-        const long long r = i - (long long)k * lvl;
-        const T rho = X[i], vx = X[F + i], vz = X[3 * F + i], p = X[4 * F + i];
-        const T sp = bg.sponge[k], ri = bg.rhoinv[k];
-        const T div = DVX[i] + DVZ[i];
-        SCR[i] = -bg.gradrho0_z[k] * vz - bg.rho0[k] * div - sp * rho;
-        T rx = -ri * GX[i] - sp * vx;
-        T rz = -ri * GZ[i] - sp * vz;
-        rz = rz - rho * bg.g[k] * ri;
-        if (abs(k - a.e_rad) <= 4) rz = rz + (PAT[r] * amp) * bg.source_dep[k];
-        T rp = -bg.c2rho0[k] * div - vz * bg.gradp0_z[k] - sp * p;
-        if (k == 0 || k == a.nz - 1) rx = rz = rp = T(0);
-        SCR[F + i] = rx;
-        SCR[2 * F + i] = T(0);
-        SCR[3 * F + i] = rz;
-        SCR[4 * F + i] = rp;
+    using W = WFft<T, N>;
+    constexpr int V = W::V, L = W::L;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int t = (threadIdx.x & 31) % L, slot = threadIdx.x / L;
+    const int rows = a.nz * a.nb, units = rows * (a.option == 12 ? 2 : 1);
+    const int first = blockIdx.x * (S5X_WARPS * W::ROWS) + slot;
+    const bool valid = first < units;
+    const int unit = valid ? first : units - 1, pair = unit / rows, row = unit - pair * rows;
+    const RowExchange<T, N> ex{reinterpret_cast<T *>(smem_raw) + (size_t)slot * W::REGION};
+    const long long F = a.F, o = (long long)row * N + t;
+    T re[V], im[V];
+    auto load = [&](int fld, T(&v)[V]) {
+#pragma unroll
+        for (int m = 0; m < V; m++) v[m] = __ldg(a.A + fld * F + o + L * m);
+        if (!a.first) {
+#pragma unroll
+            for (int m = 0; m < V; m++) v[m] = v[m] + a.b * __ldg(a.SCR + fld * F + o + L * m);
+        }
+    };
+    load(1, re);  // v_x
+    if (pair == 0) {
+        load(4, im);  // p
+    } else {
+        T vz[V];
+        load(3, vz);
+        load(7, im);  // b_z
+        const long long q = (long long)(row / a.nb) * N + t;
+#pragma unroll
+        for (int m = 0; m < V; m++) re[m] = -(re[m] * __ldg(a.bg.boz + q + L * m) - vz[m] * __ldg(a.bg.box + q + L * m));
+    }
+    RowMax<T> mr, mi;
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        mr.add(re[m]);
+        mi.add(im[m]);
+    }
+    mr.template reduce<L>();
+    mi.template reduce<L>();
+    const RowScale<T> sr = row_scale<T>(mr), si = row_scale<T>(mi);
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        re[m] = scale_in(re[m], sr);
+        im[m] = scale_in(im[m], si);
+    }
+    wfft_deriv<T, N, V, W::RADIX4>(re, im, ex, f.twr, f.twi, f.kap, f.stretch, t);
+    if (!valid) return;
+    T *d = a.DX + 2 * pair * F + o;
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        d[L * m] = scale_out(re[m], sr);
+        d[F + L * m] = scale_out(im[m], si);
     }
 }
 
-// Option 6, MP_QUIET_PML_2D (physics2d.f90:662-713): the same formulation with the vertical PML
-// (PML_BOUNDARY_ACCOUNTING_2D, physics2d.f90:1142-1160: psi_p and psi_vz on the PML rows,
-// stored [2][npml][nb][nx]) and no sponge; the top and bottom rows of all four RHS zero.
-template <typename T>
-__global__ void __launch_bounds__(S5_THREADS) s6_rhs_kernel(S5Args a, S5Bg<T> bg, const T *__restrict__ X,
-                                                            T *__restrict__ SCR, const T *__restrict__ DVX,
-                                                            const T *__restrict__ DVZ, const T *__restrict__ GX,
-                                                            const T *__restrict__ GZ, const T *__restrict__ PSI,
-                                                            T *__restrict__ SPSI, const T *__restrict__ PAT, T amp)
+// ---- z pass.  OPT 5: sponge (physics2d.f90:1099-1137), 6: vertical PML (662-713, 1142-1160), 12: with the
+// magnetic field (411-474, 1162-1200: dv_z/dz with its PML term replaced on the PML rows 1..npmlbot-1 and
+// nz-npmltop..nz-2 (0-based) by the mean of its two neighbours).  PML auxiliaries [npa][npml][nb][nx]: psi_p,
+// psi_vz, psi_flux, psi_dzbx.  The top and bottom rows: zero RHS of momentum and pressure (5) or of all (6, 12).
+// Thread (c, j): column c of the tile, the rows of chunk j.  The tiles hold the fields, then their derivatives.
+constexpr int S5Z_LMAX = 16, S5Z_ROWS = 4;
+template <typename T, int CW>
+constexpr int s5z_nch() { return sizeof(T) == 8 && CW <= 8 ? 32 : 20; }
+
+template <typename T, int CW, int OPT>
+__global__ void __launch_bounds__(CW *s5z_nch<T, CW>()) s5z_kernel(S5Step<T> a, ZTab<T> z1, int nch, int LC)
 {
-    const long long lvl = (long long)a.nb * a.nx, n = lvl * a.nz, F = n;
-    const long long P = (long long)(a.npmlbot + a.npmltop) * lvl;
-    const long long stride = (long long)gridDim.x * S5_THREADS;
-    for (long long i = (long long)blockIdx.x * S5_THREADS + threadIdx.x; i < n; i += stride) {
-        const int k = (int)(i / lvl);
-        const long long r = i - (long long)k * lvl;
-        T gz = GZ[i], dvz = DVZ[i];
-        int pi = -1;
-        if (k < a.npmlbot) pi = k;
-        else if (k >= a.nz - a.npmltop) pi = a.npmlbot + (k - (a.nz - a.npmltop));
-        if (pi >= 0) {
-            const long long m = (long long)pi * lvl + r;
-            const T pp = PSI[m], pv = PSI[P + m];
-            SPSI[m] = bg.az[pi] * gz + bg.bz[pi] * pp;
-            gz = gz + pp;
-            SPSI[P + m] = bg.az[pi] * dvz + bg.bz[pi] * pv;
-            dvz = dvz + pv;
+    constexpr int NQ = OPT == 12 ? 4 : 2, LMAX = S5Z_LMAX, R = S5Z_ROWS;
+    constexpr int NFLD = OPT == 12 ? 6 : 4;
+    constexpr int fld[6] = {0, 1, 3, 4, 5, 7};  // rho, v_x, v_z, p, b_x, b_z
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *B = reinterpret_cast<T *>(smem_raw);
+    const int nz = a.nz, c = threadIdx.x % CW, j = threadIdx.x / CW, k0 = j * LC, n = min(LC, nz - k0);
+    const size_t tile = (size_t)nz * CW;
+    T *YB = B + NQ * tile;
+    const long long lvl = a.lvl, F = a.F, r = (long long)blockIdx.x * CW + c;
+    const int x = (int)(r % a.nx);
+    auto input = [&](int q, long long o) {
+        const T v = a.A[q * F + o];
+        return a.first ? v : v + a.b * a.SCR[q * F + o];
+    };
+#pragma unroll
+    for (int m = 0; m < LMAX; m++) {
+        if (m < n) {
+            const int k = k0 + m;
+            const long long o = (long long)k * lvl + r;
+            const T vz = input(3, o);
+            B[k * CW + c] = input(4, o);
+            B[tile + k * CW + c] = vz;
+            if (OPT == 12) {
+                const long long q = (long long)k * a.nx + x;
+                B[2 * tile + k * CW + c] = -(input(1, o) * __ldg(a.bg.boz + q) - vz * __ldg(a.bg.box + q));
+                B[3 * tile + k * CW + c] = input(5, o);
+            }
         }
-        const T rho = X[i], vz = X[3 * F + i];
-        const T ri = bg.rhoinv[k];
-        const T div = DVX[i] + dvz;
-        T rc = -bg.rho0[k] * div - bg.gradrho0_z[k] * vz;
-        T rp = -bg.c2rho0[k] * div - vz * bg.gradp0_z[k];
-        T rx = -ri * GX[i];
-        T rz = -ri * (gz + rho * bg.g[k]);
-        if (abs(k - a.e_rad) <= 4) rz = rz + (PAT[r] * amp) * bg.source_dep[k];
-        if (k == 0 || k == a.nz - 1) rc = rp = rx = rz = T(0);
-        SCR[i] = rc;
-        SCR[F + i] = rx;
-        SCR[2 * F + i] = T(0);
-        SCR[3 * F + i] = rz;
-        SCR[4 * F + i] = rp;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int q = 0; q < NQ; q++) {
+        T y[LMAX], xl, xr;
+        T *yb = YB + (size_t)(q & 1) * 2 * nch * CW;
+        const T last = zlocal<T, LMAX>(z1, B + q * tile, CW, c, k0, n, nz, T(0), y);
+        yb[(2 * j) * CW + c] = y[0];
+        yb[(2 * j + 1) * CW + c] = last;
+        __syncthreads();  // the tile is read, the boundary values are there
+        zcouple(z1, yb, CW, c, j, nch, xl, xr);
+#pragma unroll
+        for (int m = 0; m < LMAX; m++)
+            if (m < n) B[q * tile + (k0 + m) * CW + c] = zcorrect(z1, y[m], k0 + m, xl, xr) * __ldg(a.stretch + k0 + m);
+    }
+    if (OPT != 5) {  // PML terms of the thread's rows
+        const long long P = (long long)(a.npmlbot + a.npmltop) * lvl;
+        for (int m = 0; m < n; m++) {
+            const int k = k0 + m;
+            const int pi = k < a.npmlbot ? k : k >= nz - a.npmltop ? a.npmlbot + (k - (nz - a.npmltop)) : -1;
+            if (pi < 0) continue;
+            const T az = __ldg(a.bg.az + pi), bz = __ldg(a.bg.bz + pi);
+            for (int q = 0; q < NQ; q++) {
+                const long long o = q * P + (long long)pi * lvl + r;
+                T ps = a.PV[o];
+                if (!a.first) ps = ps + a.b * a.SPV[o];
+                T &d = B[q * tile + k * CW + c];
+                a.SPV[o] = az * d + bz * ps;
+                d = d + ps;
+            }
+        }
+    }
+    if (OPT == 12) __syncthreads();  // the smoothing reads the rows of the neighbouring chunks
+#pragma unroll 1
+    for (int m0 = 0; m0 < n; m0 += R) {
+        T X[NFLD][R], D[NQ][R];
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            if (m0 + i < n) {
+                const long long o = (long long)(k0 + m0 + i) * lvl + r;
+#pragma unroll
+                for (int v = 0; v < NFLD; v++) X[v][i] = input(fld[v], o);
+#pragma unroll
+                for (int q = 0; q < NQ; q++) D[q][i] = __ldg(a.DX + q * F + o);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < R; i++) {
+            if (m0 + i < n) {
+                const int k = k0 + m0 + i;
+                const long long o = (long long)k * lvl + r;
+                const T *b = B + k * CW + c;
+                const T rho = X[0][i], vz = X[2][i], gx = D[1][i];
+                const T gz = b[0];
+                T dvz = b[tile];
+                if (OPT == 12 && ((k >= 1 && k <= a.npmlbot - 1) || (k >= nz - a.npmltop && k <= nz - 2)))
+                    dvz = T(0.5) * (b[tile - CW] + b[tile + CW]);
+                const T ri = __ldg(a.bg.rhoinv + k), g = __ldg(a.bg.g + k);
+                const T div = D[0][i] + dvz;
+                const bool rim = k == 0 || k == nz - 1;
+                T rc, rx, rz, rp;
+                if (OPT == 5) {
+                    const T sp = __ldg(a.bg.sponge + k);
+                    rc = -__ldg(a.bg.gradrho0_z + k) * vz - __ldg(a.bg.rho0 + k) * div - sp * rho;
+                    rx = -ri * gx - sp * X[1][i];
+                    rz = -ri * gz - sp * vz;
+                    rz = rz - rho * g * ri;
+                    rp = -__ldg(a.bg.c2rho0 + k) * div - vz * __ldg(a.bg.gradp0_z + k) - sp * X[3][i];
+                } else if (OPT == 6) {
+                    rc = -__ldg(a.bg.rho0 + k) * div - __ldg(a.bg.gradrho0_z + k) * vz;
+                    rp = -__ldg(a.bg.c2rho0 + k) * div - vz * __ldg(a.bg.gradp0_z + k);
+                    rx = -ri * gx;
+                    rz = -ri * (gz + rho * g);
+                } else {
+                    const long long q = (long long)k * a.nx + x;
+                    const T bxs = X[4 % NFLD][i], bzs = X[5 % NFLD][i], cu = __ldg(a.bg.curl + q);
+                    const T cur = b[3 % NQ * tile] - D[3 % NQ][i];
+                    const T t1 = __ldg(a.bg.boz + q) * cur + bzs * cu;
+                    const T t3 = -__ldg(a.bg.box + q) * cur - bxs * cu;
+                    rc = -__ldg(a.bg.gradrho0_z + k) * vz - __ldg(a.bg.rho0 + k) * div;
+                    rx = ri * (t1 - gx);
+                    rz = ri * (t3 - gz);
+                    rz = rz - ri * rho * g;
+                    rp = -__ldg(a.bg.c2rho0 + k) * div - vz * __ldg(a.bg.gradp0_z + k);
+                }
+                if (abs(k - a.e_rad) <= 4) rz = rz + (__ldg(a.PAT + r) * a.amp) * __ldg(a.bg.source_dep + k);
+                if (rim) {
+                    if (OPT != 5) rc = T(0);
+                    rx = rz = rp = T(0);
+                }
+                a.SCR[o] = rc;
+                a.SCR[F + o] = rx;
+                a.SCR[3 * F + o] = rz;
+                a.SCR[4 * F + o] = rp;
+                if (OPT == 12) {
+                    a.SCR[5 * F + o] = rim ? T(0) : -b[2 % NQ * tile];
+                    a.SCR[7 * F + o] = rim ? T(0) : D[2 % NQ][i];
+                }
+            }
+        }
     }
 }
 
@@ -98,135 +229,39 @@ __global__ void __launch_bounds__(S5_THREADS) s5_axpy_kernel(long long n, T *__r
     for (long long i = (long long)blockIdx.x * S5_THREADS + threadIdx.x; i < n; i += stride) Y[i] = Y[i] + a * X[i];
 }
 
-// One thread per (field, column): a += dt scr, then FILTER_VARS_2D: the 11-point filter on rows
-// 5 .. nz-6 and two-point means on rows nz-5 .. nz-2 (0-based) of the updated column, written
-// to rows 5 .. nz-2 for x in [i0, i1] (HORIZONTAL_PMLS) from an 11-value register window.
-template <typename T>
-__global__ void __launch_bounds__(S5_THREADS) s5_end_kernel(S5Args a, T *__restrict__ A, const T *__restrict__ SCR,
-                                                            T dt)
+// End of step: a block takes CW columns of one field (those with a RHS), a += dt scr into a tile, then
+// FILTER_VARS_2D in place: the 11-point filter on rows 5 .. nz-6 and two-point means on rows nz-5 .. nz-2 (0-based)
+// for x in [i0, i1] (HORIZONTAL_PMLS).  One thread walking a column took 206 us at 8 x 512 x 300 FP32 (80 blocks).
+template <typename T, int CW>
+__global__ void __launch_bounds__(S5_THREADS) s5_end_kernel(S5Step<T> a)
 {
-    const long long lvl = (long long)a.nb * a.nx;
-    const long long cols = (long long)a.nf * lvl, F = lvl * a.nz;
-    const long long c = (long long)blockIdx.x * S5_THREADS + threadIdx.x;
-    if (c >= cols) return;
-    const int v = (int)(c / lvl);
-    const long long r = c - (long long)v * lvl;
+    constexpr int ROWS = S5_THREADS / CW;
+    constexpr int fld[6] = {0, 1, 3, 4, 5, 7};
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *B = reinterpret_cast<T *>(smem_raw);
+    const int c = threadIdx.x % CW, w = threadIdx.x / CW, nz = a.nz, v = fld[blockIdx.y];
+    const long long lvl = a.lvl, r = (long long)blockIdx.x * CW + c;
     const int x = (int)(r % a.nx);
-    T *col = A + (long long)v * F + r;
-    const T *sc = SCR + (long long)v * F + r;
-    const int nz = a.nz;
-    for (int k = 0; k < nz; k++) col[(long long)k * lvl] = col[(long long)k * lvl] + dt * sc[(long long)k * lvl];
-    if (x < a.i0 || x > a.i1 || nz < 11) return;
+    T *col = a.A + v * a.F + r;
+    const T *sc = a.SCR + v * a.F + r;
+#pragma unroll 4
+    for (int k = w; k < nz; k += ROWS) B[k * CW + c] = col[(long long)k * lvl] + a.dt * __ldg(sc + (long long)k * lvl);
+    __syncthreads();
+    const bool xf = x >= a.i0 && x <= a.i1;
     const T c0 = T(0.75390625), h1 = T(0.5 * 0.41015625), h2 = T(0.5 * -0.234375), h3 = T(0.5 * 0.087890625),
             h4 = T(0.5 * -0.01953125), h5 = T(0.5 * 0.001953125);
-    T w[11];  // rows k-5 .. k+5 of the updated column, for the row k being written
-#pragma unroll
-    for (int j = 0; j < 11; j++) w[j] = col[(long long)j * lvl];
-    for (int k = 5; k <= nz - 2; k++) {
-        T out;
-        if (k <= nz - 6)
-            out = c0 * w[5] + h1 * (w[4] + w[6]) + h2 * (w[3] + w[7]) + h3 * (w[2] + w[8]) + h4 * (w[1] + w[9]) +
-                  h5 * (w[0] + w[10]);
-        else
-            out = T(0.5) * (w[6] + w[4]);
-#pragma unroll
-        for (int j = 0; j < 10; j++) w[j] = w[j + 1];
-        if (k + 6 < nz) w[10] = col[(long long)(k + 6) * lvl];
+#pragma unroll 2
+    for (int k = w; k < nz; k += ROWS) {
+        const T *b = B + k * CW + c;
+        T out = b[0];
+        if (xf && k >= 5 && k <= nz - 2) {
+            if (k <= nz - 6)
+                out = c0 * b[0] + h1 * (b[-CW] + b[CW]) + h2 * (b[-2 * CW] + b[2 * CW]) + h3 * (b[-3 * CW] + b[3 * CW]) +
+                      h4 * (b[-4 * CW] + b[4 * CW]) + h5 * (b[-5 * CW] + b[5 * CW]);
+            else
+                out = T(0.5) * (b[CW] + b[-CW]);
+        }
         col[(long long)k * lvl] = out;
-    }
-}
-
-// Option 12: the induction flux -(v_x boz - v_z box) of the stage input (physics2d.f90:421).
-template <typename T>
-__global__ void __launch_bounds__(S5_THREADS) s12_flux_kernel(S5Args a, S5Bg<T> bg, const T *__restrict__ X,
-                                                              T *__restrict__ FLUX)
-{
-    const long long lvl = (long long)a.nb * a.nx, n = lvl * a.nz, F = n;
-    const long long stride = (long long)gridDim.x * S5_THREADS;
-    for (long long i = (long long)blockIdx.x * S5_THREADS + threadIdx.x; i < n; i += stride) {
-        const int k = (int)(i / lvl);
-        const int x = (int)((i - (long long)k * lvl) % a.nx);
-        const long long q = (long long)k * a.nx + x;
-        FLUX[i] = -(X[F + i] * bg.boz[q] - X[3 * F + i] * bg.box[q]);
-    }
-}
-
-// Option 12, MP_MHD_PML_2d (physics2d.f90:411-474) with PML_BOUNDARY_ACCOUNTING_2D (1142-1200):
-// psi_p, psi_vz as option 6; dv_z/dz (with its PML term) replaced on the PML rows 1..npmlbot-1
-// and nz-npmltop..nz-2 (0-based) by the mean of its two neighbours; psi of d flux/dz and of
-// d b_x/dz.  PML auxiliaries [4][npml][nb][nx]: psi_p, psi_vz, psi_flux, psi_dzbx.  The top and
-// bottom rows of all eight RHS zero.
-template <typename T>
-__global__ void __launch_bounds__(S5_THREADS) s12_rhs_kernel(S5Args a, S5Bg<T> bg, const T *__restrict__ X,
-                                                             T *__restrict__ SCR, const T *__restrict__ DVX,
-                                                             const T *__restrict__ DVZ, const T *__restrict__ GX,
-                                                             const T *__restrict__ GZ, const T *__restrict__ DZBX,
-                                                             const T *__restrict__ DZF, const T *__restrict__ DXF,
-                                                             const T *__restrict__ DXBZ, const T *__restrict__ PSI,
-                                                             T *__restrict__ SPSI, const T *__restrict__ PAT, T amp)
-{
-    const long long lvl = (long long)a.nb * a.nx, n = lvl * a.nz, F = n;
-    const long long P = (long long)(a.npmlbot + a.npmltop) * lvl;
-    const long long stride = (long long)gridDim.x * S5_THREADS;
-    auto pml = [&](int k) {
-        if (k < a.npmlbot) return k;
-        if (k >= a.nz - a.npmltop) return a.npmlbot + (k - (a.nz - a.npmltop));
-        return -1;
-    };
-    for (long long i = (long long)blockIdx.x * S5_THREADS + threadIdx.x; i < n; i += stride) {
-        const int k = (int)(i / lvl);
-        const long long r = i - (long long)k * lvl;
-        const int x = (int)(r % a.nx);
-        T gz = GZ[i], dzf = DZF[i], dzbx = DZBX[i];
-        T dvz = DVZ[i];
-        const int pi = pml(k);
-        if (pi >= 0) {
-            const long long m = (long long)pi * lvl + r;
-            const T pp = PSI[m], pv = PSI[P + m], pf = PSI[2 * P + m], pb = PSI[3 * P + m];
-            SPSI[m] = bg.az[pi] * gz + bg.bz[pi] * pp;
-            gz = gz + pp;
-            SPSI[P + m] = bg.az[pi] * dvz + bg.bz[pi] * pv;
-            dvz = dvz + pv;
-            SPSI[2 * P + m] = bg.az[pi] * dzf + bg.bz[pi] * pf;
-            dzf = dzf + pf;
-            SPSI[3 * P + m] = bg.az[pi] * dzbx + bg.bz[pi] * pb;
-            dzbx = dzbx + pb;
-        }
-        if ((k >= 1 && k <= a.npmlbot - 1) || (k >= a.nz - a.npmltop && k <= a.nz - 2)) {
-            T nb2[2];
-#pragma unroll
-            for (int j = 0; j < 2; j++) {
-                const int kk = j == 0 ? k - 1 : k + 1;
-                const int pk = pml(kk);
-                T v = DVZ[i + (j == 0 ? -lvl : lvl)];
-                if (pk >= 0) v = v + PSI[P + (long long)pk * lvl + r];
-                nb2[j] = v;
-            }
-            dvz = T(0.5) * (nb2[0] + nb2[1]);
-        }
-        const long long q = (long long)k * a.nx + x;
-        const T rho = X[i], vz = X[3 * F + i], bxs = X[5 * F + i], bzs = X[7 * F + i];
-        const T ri = bg.rhoinv[k], cu = bg.curl[q];
-        const T div = DVX[i] + dvz;
-        const T cur = dzbx - DXBZ[i];
-        const T t1 = bg.boz[q] * cur + bzs * cu;
-        const T t3 = -bg.box[q] * cur - bxs * cu;
-        T rc = -bg.gradrho0_z[k] * vz - bg.rho0[k] * div;
-        T rx = ri * (t1 - GX[i]);
-        T rz = ri * (t3 - gz);
-        rz = rz - ri * rho * bg.g[k];
-        if (abs(k - a.e_rad) <= 4) rz = rz + (PAT[r] * amp) * bg.source_dep[k];
-        T rp = -bg.c2rho0[k] * div - vz * bg.gradp0_z[k];
-        T rbx = -dzf, rbz = DXF[i];
-        if (k == 0 || k == a.nz - 1) rc = rx = rz = rp = rbx = rbz = T(0);
-        SCR[i] = rc;
-        SCR[F + i] = rx;
-        SCR[2 * F + i] = T(0);
-        SCR[3 * F + i] = rz;
-        SCR[4 * F + i] = rp;
-        SCR[5 * F + i] = rbx;
-        SCR[6 * F + i] = T(0);
-        SCR[7 * F + i] = rbz;
     }
 }
 
@@ -236,40 +271,79 @@ static unsigned s5_grid(long long n)
     return (unsigned)(g < 152LL * 16 ? g : 152LL * 16);
 }
 
-template <typename T>
-cudaError_t launch_s5_rhs(const S5Args &a, const S5Bg<T> &bg, const T *X, T *SCR, const T *DVX, const T *DVZ,
-                          const T *GX, const T *GZ, const T *PAT, T amp, cudaStream_t st)
+template <typename T, int N>
+static cudaError_t s5x_n(const S5Step<T> &a, const S3Fft<T> &f, cudaStream_t st)
 {
-    const long long n = (long long)a.nb * a.nx * a.nz;
-    s5_rhs_kernel<T><<<s5_grid(n), S5_THREADS, 0, st>>>(a, bg, X, SCR, DVX, DVZ, GX, GZ, PAT, amp);
+    using W = WFft<T, N>;
+    const int units = a.nz * a.nb * (a.option == 12 ? 2 : 1), slots = S5X_WARPS * W::ROWS;
+    const size_t smem = (size_t)slots * W::REGION * sizeof(T);
+    auto k = s5x_kernel<T, N>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<(units + slots - 1) / slots, S5X_WARPS * WARP, smem, st>>>(a, f);
     return cudaGetLastError();
 }
 
 template <typename T>
-cudaError_t launch_s6_rhs(const S5Args &a, const S5Bg<T> &bg, const T *X, T *SCR, const T *DVX, const T *DVZ,
-                          const T *GX, const T *GZ, const T *PSI, T *SPSI, const T *PAT, T amp, cudaStream_t st)
+cudaError_t launch_s5x(const S5Step<T> &a, const S3Fft<T> &f, cudaStream_t st)
 {
-    const long long n = (long long)a.nb * a.nx * a.nz;
-    s6_rhs_kernel<T><<<s5_grid(n), S5_THREADS, 0, st>>>(a, bg, X, SCR, DVX, DVZ, GX, GZ, PSI, SPSI, PAT, amp);
+#define CASE(n_) if (a.nx == n_) return s5x_n<T, n_>(a, f, st);
+    CASE(64) CASE(128) CASE(192) CASE(256) CASE(384) CASE(512) CASE(768) CASE(1024)
+#undef CASE
+    return cudaErrorInvalidValue;
+}
+
+template <typename T, int CW, int OPT>
+static cudaError_t s5z_cw(const S5Step<T> &a, const ZTab<T> &z1, int nch, int L, cudaStream_t st)
+{
+    if (a.lvl % CW || L > S5Z_LMAX || nch > s5z_nch<T, CW>()) return cudaErrorInvalidValue;
+    const size_t smem = ((size_t)(OPT == 12 ? 4 : 2) * a.nz * CW + (size_t)4 * nch * CW) * sizeof(T);
+    auto k = s5z_kernel<T, CW, OPT>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<(unsigned)(a.lvl / CW), CW * nch, smem, st>>>(a, z1, nch, L);
     return cudaGetLastError();
 }
 
-template <typename T>
-cudaError_t launch_s12_flux(const S5Args &a, const S5Bg<T> &bg, const T *X, T *FLUX, cudaStream_t st)
+template <typename T, int CW>
+static cudaError_t s5z_option(const S5Step<T> &a, const ZTab<T> &z1, int nch, int L, cudaStream_t st)
 {
-    const long long n = (long long)a.nb * a.nx * a.nz;
-    s12_flux_kernel<T><<<s5_grid(n), S5_THREADS, 0, st>>>(a, bg, X, FLUX);
-    return cudaGetLastError();
+    return a.option == 12 ? s5z_cw<T, CW, 12>(a, z1, nch, L, st)
+                          : a.option == 6 ? s5z_cw<T, CW, 6>(a, z1, nch, L, st) : s5z_cw<T, CW, 5>(a, z1, nch, L, st);
 }
 
 template <typename T>
-cudaError_t launch_s12_rhs(const S5Args &a, const S5Bg<T> &bg, const T *X, T *SCR, const T *DVX, const T *DVZ,
-                           const T *GX, const T *GZ, const T *DZBX, const T *DZF, const T *DXF, const T *DXBZ,
-                           const T *PSI, T *SPSI, const T *PAT, T amp, cudaStream_t st)
+cudaError_t launch_s5z(const S5Step<T> &a, const ZTab<T> &z1, int nch, int L, int cw, cudaStream_t st)
 {
-    const long long n = (long long)a.nb * a.nx * a.nz;
-    s12_rhs_kernel<T><<<s5_grid(n), S5_THREADS, 0, st>>>(a, bg, X, SCR, DVX, DVZ, GX, GZ, DZBX, DZF, DXF, DXBZ, PSI,
-                                                         SPSI, PAT, amp);
+    if constexpr (sizeof(T) == 8) {
+        if (cw == 2) return s5z_option<T, 2>(a, z1, nch, L, st);
+        if (cw == 4) return s5z_option<T, 4>(a, z1, nch, L, st);
+    } else {
+        if (cw == 32) return s5z_option<T, 32>(a, z1, nch, L, st);
+    }
+    return cw == 8 ? s5z_option<T, 8>(a, z1, nch, L, st) : cudaErrorInvalidValue;
+}
+
+template <typename T, int CW>
+static cudaError_t s5_end_cw(const S5Step<T> &a, cudaStream_t st)
+{
+    const size_t smem = (size_t)a.nz * CW * sizeof(T);
+    auto k = s5_end_kernel<T, CW>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<dim3((unsigned)(a.lvl / CW), a.option == 12 ? 6 : 4), S5_THREADS, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
+// Tile width: one 128-byte row segment where that gives two blocks per SM, else one 32-byte sector.
+template <typename T>
+cudaError_t launch_s5_end(const S5Step<T> &a, long long npv, cudaStream_t st)
+{
+    constexpr int WIDE = 128 / sizeof(T), NARROW = 32 / sizeof(T);
+    const long long wide = a.lvl / WIDE * (a.option == 12 ? 6 : 4);
+    const cudaError_t e = a.lvl % WIDE == 0 && wide >= 2 * 152 ? s5_end_cw<T, WIDE>(a, st) : s5_end_cw<T, NARROW>(a, st);
+    if (e != cudaSuccess || npv == 0) return e;
+    s5_axpy_kernel<T><<<s5_grid(npv), S5_THREADS, 0, st>>>(npv, a.PV, a.SPV, a.dt);
     return cudaGetLastError();
 }
 
@@ -280,40 +354,13 @@ cudaError_t launch_s5_axpy(long long n, T *Y, const T *X, T a, cudaStream_t st)
     return cudaGetLastError();
 }
 
-template <typename T>
-cudaError_t launch_s5_end(const S5Args &a, T *A, const T *SCR, T dt, T *PV, const T *SPV, cudaStream_t st)
-{
-    const long long cols = (long long)a.nf * a.nb * a.nx;
-    s5_end_kernel<T><<<(unsigned)((cols + S5_THREADS - 1) / S5_THREADS), S5_THREADS, 0, st>>>(a, A, SCR, dt);
-    const long long np = (long long)a.npa * (a.npmlbot + a.npmltop) * a.nb * a.nx;
-    if (PV && np > 0) s5_axpy_kernel<T><<<s5_grid(np), S5_THREADS, 0, st>>>(np, PV, SPV, dt);
-    return cudaGetLastError();
-}
-
-template cudaError_t launch_s5_rhs<float>(const S5Args &, const S5Bg<float> &, const float *, float *, const float *,
-                                          const float *, const float *, const float *, const float *, float,
-                                          cudaStream_t);
-template cudaError_t launch_s5_rhs<double>(const S5Args &, const S5Bg<double> &, const double *, double *,
-                                           const double *, const double *, const double *, const double *,
-                                           const double *, double, cudaStream_t);
-template cudaError_t launch_s6_rhs<float>(const S5Args &, const S5Bg<float> &, const float *, float *, const float *,
-                                          const float *, const float *, const float *, const float *, float *,
-                                          const float *, float, cudaStream_t);
-template cudaError_t launch_s6_rhs<double>(const S5Args &, const S5Bg<double> &, const double *, double *,
-                                           const double *, const double *, const double *, const double *,
-                                           const double *, double *, const double *, double, cudaStream_t);
-#define SPARC_S12_INST(T)                                                                                      \
-    template cudaError_t launch_s12_flux<T>(const S5Args &, const S5Bg<T> &, const T *, T *, cudaStream_t);          \
-    template cudaError_t launch_s12_rhs<T>(const S5Args &, const S5Bg<T> &, const T *, T *, const T *, const T *,    \
-                                           const T *, const T *, const T *, const T *, const T *, const T *,        \
-                                           const T *, T *, const T *, T, cudaStream_t);                             \
+#define S5_INST(T)                                                                                                   \
+    template cudaError_t launch_s5x<T>(const S5Step<T> &, const S3Fft<T> &, cudaStream_t);                           \
+    template cudaError_t launch_s5z<T>(const S5Step<T> &, const ZTab<T> &, int, int, int, cudaStream_t);             \
+    template cudaError_t launch_s5_end<T>(const S5Step<T> &, long long, cudaStream_t);                               \
     template cudaError_t launch_s5_axpy<T>(long long, T *, const T *, T, cudaStream_t);
-SPARC_S12_INST(float)
-SPARC_S12_INST(double)
-#undef SPARC_S12_INST
-template cudaError_t launch_s5_end<float>(const S5Args &, float *, const float *, float, float *, const float *,
-                                          cudaStream_t);
-template cudaError_t launch_s5_end<double>(const S5Args &, double *, const double *, double, double *,
-                                           const double *, cudaStream_t);
+S5_INST(float)
+S5_INST(double)
+#undef S5_INST
 
 }  // namespace sparc
