@@ -8,22 +8,27 @@
 // receiver.  The sum over receivers is linear, and exp(-2 pi i k (i-1)/nx) is the forward DFT
 // kernel of a point at x_i, so it equals one transform per mode:
 //     adj_mode = Re IDFT2( filter * DFT2(c) ),  c(x_i, t) = con_i w_i(t) ccdot(x_i, t),
-// with c zero at unmeasured x.  Per mode and batch: three inverse 2-D transforms (filtered
-// synthetic, filtered data, time derivative), the Gizon-Birch derivative of the synthetic along
-// t, per-receiver reductions (window pick, travel time, normalisation), and one forward plus
-// one inverse 2-D transform of c.
+// with c zero at unmeasured x.  The filters are real and even in k and f, so real records stay real:
+//   - synthetic and data share one transform as real and imaginary part (the data times a power of two of
+//     each source, which keeps the rounding of either relative to itself);
+//   - per mode one inverse transform gives both filtered records; a second, of the synthetic's spectrum, the
+//     time derivative ccdot and, as imaginary part, the Gizon-Birch derivative.  With an even record count the
+//     middle frequency makes ccdot complex, and the two derivatives take a transform each;
+//   - only Re c enters adj_mode, and the filtered spectra of all modes are summed: one inverse transform at the end;
+//   - only measured columns are transformed along t (their tiles of a few columns, listed on the host).
+// Per mode 3 transforms along x and 3 along t of the measured columns, where 4 and 7 of every column were taken.
 //
-// Fields are complex [nb][nt][nx] (x fastest).  x transforms: one warp per row, the shared-
-// memory Stockham FFT of the wave solver (nx in its table).  t transforms: any nt (the record
-// count, 240 or 241 for 3600 steps -- 241 is prime): Bluestein's chirp-z transform on two
-// power-of-two FFTs of length M >= 2 nt - 1 (nt <= 512), a direct DFT over 16-column tiles above
-// that.  FFTW's transforms are unnormalised, and so are these.
+// Fields are complex [nb][nt][nx] (x fastest).  x transforms: the register transforms of sparc_wfft.cuh (nx in
+// the FFT table).  t transforms: any nt (the record count, 240 or 241 for 3600 steps -- 241 is prime): Bluestein's
+// chirp-z transform on two power-of-two FFTs of length M >= 2 nt - 1 (nt <= 512), a direct DFT over 16-column tiles
+// above that.  FFTW's transforms are unnormalised, and so are these.  FP64 throughout: bound by the
+// double-precision pipe.
 #include <cmath>
 #include <string>
 #include <vector>
 
-#include "sparc_common.cuh"
 #include "sparc_gb300.h"
+#include "sparc_wfft.cuh"
 
 namespace sparc {
 int report_error(int code, const std::string &msg);
@@ -38,39 +43,46 @@ constexpr int TT_XWPB = 2;       // rows (warps) per block of the x transform
 constexpr double TT_PI = 3.141592653589793;
 
 // x transform of complex rows in place, sign -1 forward, +1 inverse (unnormalised).
-template <int N>
+template <int N, bool INV>
 __global__ void __launch_bounds__(TT_XWPB *WARP) tt_fft_x_kernel(double2 *data, long long nrows, const double *twr,
-                                                                 const double *twi, int inverse)
+                                                                 const double *twi)
 {
+    using W = WFft<double, N, false>;
+    constexpr int V = W::V, L = W::L;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    double *sm = reinterpret_cast<double *>(smem_raw);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long row = (long long)blockIdx.x * TT_XWPB + warp;
-    if (row >= nrows) return;
-    double *xr = sm + (size_t)warp * 4 * N, *xi = xr + N, *yr = xi + N, *yi = yr + N;
-    double2 *d = data + row * N;
-    for (int x = lane; x < N; x += WARP) {
-        const double2 v = d[x];
-        xr[x] = v.x;
-        xi[x] = v.y;
+    const int t = (threadIdx.x & 31) % L, slot = threadIdx.x / L;
+    const long long first = (long long)blockIdx.x * (TT_XWPB * W::ROWS) + slot;
+    const bool valid = first < nrows;
+    const RowExchange<double, N> ex{reinterpret_cast<double *>(smem_raw) + (size_t)slot * W::REGION};
+    double2 *d = data + (valid ? first : nrows - 1) * N + t;
+    double re[V], im[V];
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        const double2 v = d[L * m];
+        re[m] = v.x;
+        im[m] = v.y;
     }
-    __syncwarp();
-    double *orr, *oi;
-    FFTRun<double, N, 0, 1>::run(xr, xi, yr, yi, twr, twi, lane, inverse != 0, 1.0, 1.0, orr, oi);
-    __syncwarp();
-    for (int x = lane; x < N; x += WARP) d[x] = make_double2(orr[x], oi[x]);
+    wfft_stages<double, N, V, false, 0, 1, INV, 0>(re, im, ex, twr, twi, t);
+    if (!valid) return;
+#pragma unroll
+    for (int m = 0; m < V; m++) d[L * m] = make_double2(re[m], im[m]);
 }
+
+// A tile of columns that a t transform covers: source b, columns x0 .. x0 + width - 1.
+struct TTTile {
+    int b, x0;
+};
 
 // t transform of complex columns in place: column (b, x) of length nt, stride nx.
 // wt[m] = exp(-2 pi i m / nt); inverse uses the conjugate.
-__global__ void __launch_bounds__(TT_THREADS) tt_dft_t_kernel(double2 *data, int nt, int nx, const double2 *wt,
-                                                              int inverse)
+__global__ void __launch_bounds__(TT_THREADS) tt_dft_t_kernel(double2 *data, const TTTile *tiles, int nt, int nx,
+                                                              const double2 *wt, int inverse)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double2 *tile = reinterpret_cast<double2 *>(smem_raw);  // [nt][TT_COLS]
     double2 *w = tile + (size_t)nt * TT_COLS;                // [nt]
-    const int x0 = blockIdx.x * TT_COLS;
-    double2 *base = data + (size_t)blockIdx.y * nt * nx + x0;
+    const int x0 = tiles[blockIdx.x].x0;
+    double2 *base = data + (size_t)tiles[blockIdx.x].b * nt * nx + x0;
     for (int idx = threadIdx.x; idx < nt * TT_COLS; idx += TT_THREADS) {
         const int t = idx / TT_COLS, c = idx % TT_COLS;
         tile[idx] = (x0 + c < nx) ? base[(size_t)t * nx + c] : make_double2(0.0, 0.0);
@@ -100,121 +112,177 @@ __global__ void __launch_bounds__(TT_THREADS) tt_dft_t_kernel(double2 *data, int
 // DFT into a convolution with the chirp b_m = exp(+i pi m^2 / nt), evaluated with two power-of-two
 // FFTs of length M >= 2 nt - 1 (Bluestein, IEEE Trans. Audio Electroacoust. 18 (1970) 451-455):
 //   X_k = w_k IFFT_M( FFT_M(x_n w_n) * FFT_M(b) )_k / M,   w_n = exp(-i pi n^2 / nt).
-// The inverse transform is the conjugate of the forward one of the conjugate.  A block of WPB warps
-// takes WPB consecutive columns (b, x0 .. x0 + WPB - 1): the tile [nt][WPB] is loaded and stored
-// row-contiguously (WPB x 16 bytes per record) through shared memory, each warp transforms one
-// column with the Stockham FFT of the x transforms.
-template <int M, int WPB>
-__global__ void __launch_bounds__(WPB *WARP) tt_bluestein_t_kernel(double2 *data, int nt, int nx, const double2 *chirp,
-                                                                   const double2 *bhat, const double *twr,
-                                                                   const double *twi, int inverse)
+// The inverse transform is the conjugate of the forward one of the conjugate.  A block takes the COLS consecutive
+// columns of a tile, WFft<M>::L threads each: the tile [nt][COLS] is loaded and stored row-contiguously (COLS x 16
+// bytes per record) through the columns' exchange regions.
+template <int M, int COLS>
+__global__ void __launch_bounds__(COLS *WFft<double, M, false>::L)
+    tt_bluestein_t_kernel(double2 *data, const TTTile *tiles, int nt, int nx, const double2 *chirp, const double2 *bhat,
+                          const double *twr, const double *twi, int inverse)
 {
+    using W = WFft<double, M, false>;
+    constexpr int V = W::V, L = W::L, SW = W::REGION + 1;  // odd: the columns' equal elements on distinct banks
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *sm = reinterpret_cast<double *>(smem_raw);
-    constexpr int SW = 4 * M + 2;  // per-warp stride: the tile rows of 8 warps land on distinct banks
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int x0 = blockIdx.x * WPB;
-    double2 *base = data + (size_t)blockIdx.y * nt * nx + x0;
+    const int t = threadIdx.x % L, col = threadIdx.x / L;
+    const int x0 = tiles[blockIdx.x].x0;
+    double2 *base = data + (size_t)tiles[blockIdx.x].b * nt * nx + x0;
     const double cs = inverse ? -1.0 : 1.0;  // conjugation of the input and output for the inverse
-    for (int idx = threadIdx.x; idx < nt * WPB; idx += WPB * WARP) {
-        const int t = idx / WPB, c = idx % WPB;
-        double *xr = sm + (size_t)c * SW, *xi = xr + M;
-        double2 v = (x0 + c < nx) ? base[(size_t)t * nx + c] : make_double2(0.0, 0.0);
+    for (int idx = threadIdx.x; idx < nt * COLS; idx += COLS * L) {
+        const int k = idx / COLS, c = idx % COLS;
+        const RowExchange<double, M> ex{sm + (size_t)c * SW};
+        double2 v = (x0 + c < nx) ? base[(size_t)k * nx + c] : make_double2(0.0, 0.0);
         v.y *= cs;
-        const double2 w = chirp[t];
-        xr[t] = v.x * w.x - v.y * w.y;
-        xi[t] = v.x * w.y + v.y * w.x;
-    }
-    double *xr = sm + (size_t)warp * SW, *xi = xr + M, *yr = xi + M, *yi = yr + M;
-    for (int t = nt + lane; t < M; t += WARP) {
-        xr[t] = 0.0;
-        xi[t] = 0.0;
-    }
-    __syncthreads();
-    double *fr, *fi;
-    FFTRun<double, M, 0, 1>::run(xr, xi, yr, yi, twr, twi, lane, false, 1.0, 1.0, fr, fi);
-    for (int k = lane; k < M; k += WARP) {
-        const double2 b = bhat[k];
-        const double ar = fr[k], ai = fi[k];
-        fr[k] = ar * b.x - ai * b.y;
-        fi[k] = ar * b.y + ai * b.x;
-    }
-    __syncwarp();
-    double *gr = (fr == xr) ? yr : xr, *gi = (fr == xr) ? yi : xi;
-    double *cr, *ci;
-    FFTRun<double, M, 0, 1>::run(fr, fi, gr, gi, twr, twi, lane, true, 1.0, 1.0, cr, ci);
-    __syncwarp();
-    const double inv_m = 1.0 / (double)M;
-    for (int k = lane; k < nt; k += WARP) {  // X_k = w_k c_k / M, back into the warp's own buffer
         const double2 w = chirp[k];
-        const double ar = cr[k] * inv_m, ai = ci[k] * inv_m;
-        const double rr = ar * w.x - ai * w.y, ri = ar * w.y + ai * w.x;
-        cr[k] = rr;
-        ci[k] = ri * cs;
+        ex.put<0>(k, v.x * w.x - v.y * w.y, v.x * w.y + v.y * w.x);
     }
-    if (lane == 0) reinterpret_cast<int *>(sm + (size_t)WPB * SW)[warp] = (int)(cr - (sm + (size_t)warp * SW));
     __syncthreads();
-    for (int idx = threadIdx.x; idx < nt * WPB; idx += WPB * WARP) {
-        const int t = idx / WPB, c = idx % WPB;
-        if (x0 + c >= nx) continue;
-        const double *wb = sm + (size_t)c * SW;
-        const int off = reinterpret_cast<const int *>(sm + (size_t)WPB * SW)[c];
-        base[(size_t)t * nx + c] = make_double2(wb[off + t], wb[off + M + t]);
+    const RowExchange<double, M> ex{sm + (size_t)col * SW};
+    double re[V], im[V];
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        re[m] = im[m] = 0.0;
+        if (t + L * m < nt) ex.get<0>(t + L * m, re[m], im[m]);
     }
-}
-
-// out = in * filter[t][x] (real), optionally times i 2 pi freqnu(t) (the time derivative of
-// driver.f90:2015-2017, freqnu = distmat(nt) / (nt dt 60)).
-__global__ void __launch_bounds__(TT_THREADS) tt_filter_kernel(const double2 *in, double2 *out, const double *filter,
-                                                               int nt, int nx, long long n, int deriv, double dt_min)
-{
-    const long long stride = (long long)gridDim.x * TT_THREADS;
-    for (long long i = (long long)blockIdx.x * TT_THREADS + threadIdx.x; i < n; i += stride) {
-        const long long tx = i % ((long long)nt * nx);
-        const int t = (int)(tx / nx);
-        const double f = filter[tx];
-        double2 v = in[i];
-        v.x *= f;
-        v.y *= f;
-        if (deriv) {
-            const int d = (t > nt - t) ? -(nt - t) : t;  // distmat: index 0 at 0, upper half negative
-            const double om = 2.0 * TT_PI * ((double)d / ((double)nt * dt_min * 60.0));
-            v = make_double2(-om * v.y, om * v.x);  // times i om
+    wfft_stages<double, M, V, false, 0, 1, false, 0>(re, im, ex, twr, twi, t);
+#pragma unroll
+    for (int m = 0; m < V; m++) {
+        const double2 b = bhat[t + L * m];
+        const double ar = re[m], ai = im[m];
+        re[m] = ar * b.x - ai * b.y;
+        im[m] = ar * b.y + ai * b.x;
+    }
+    wfft_stages<double, M, V, false, 0, 1, true, 0>(re, im, ex, twr, twi, t);
+    __syncwarp();  // the transform's last reads of the region are done
+    const double inv_m = 1.0 / (double)M;
+#pragma unroll
+    for (int m = 0; m < V; m++) {  // X_k = w_k c_k / M, back into the column's region
+        const int k = t + L * m;
+        if (k < nt) {
+            const double2 w = chirp[k];
+            const double ar = re[m] * inv_m, ai = im[m] * inv_m;
+            ex.put<0>(k, ar * w.x - ai * w.y, (ar * w.y + ai * w.x) * cs);
         }
-        out[i] = v;
+    }
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < nt * COLS; idx += COLS * L) {
+        const int k = idx / COLS, c = idx % COLS;
+        if (x0 + c >= nx) continue;
+        const RowExchange<double, M> ec{sm + (size_t)c * SW};
+        double2 v;
+        ec.get<0>(k, v.x, v.y);
+        base[(size_t)k * nx + c] = v;
     }
 }
 
-// Real records into complex planes.
-__global__ void __launch_bounds__(TT_THREADS) tt_load_kernel(const double *in, double2 *out, long long n)
+// Angular frequencies of spectral row t: of the time derivative of driver.f90:2015-2017 (freqnu = distmat(nt) /
+// (nt dt 60): index 0 at 0, upper half negative) and of COMPUTE_TT_GIZONBIRCH's derivative (driver.f90:913-917: zero
+// at q = nt/2 and its mirror).
+__device__ __forceinline__ double tt_omega(int t, int nt, double dt_min)
 {
-    const long long stride = (long long)gridDim.x * TT_THREADS;
-    for (long long i = (long long)blockIdx.x * TT_THREADS + threadIdx.x; i < n; i += stride)
-        out[i] = make_double2(in[i], 0.0);
+    const int d = (t > nt - t) ? -(nt - t) : t;
+    return 2.0 * TT_PI * ((double)d / ((double)nt * dt_min * 60.0));
+}
+__device__ __forceinline__ double tt_omega_gb(int t, int nt, double dt_min)
+{
+    const int h = nt / 2, q = t < h ? t : t > nt - h ? -(nt - t) : 0;
+    return 2.0 * TT_PI * (double)q / ((double)nt * dt_min);
 }
 
-// Real part into a complex buffer (imaginary part zero), optional scale.
-__global__ void __launch_bounds__(TT_THREADS) tt_real_kernel(const double2 *in, double2 *out, long long n, double s)
+// Per source: the power of two that brings the data's largest value to the synthetic's binary exponent (1 where
+// either is zero or not finite), its inverse, and whether the data have a value that is not finite.
+struct TTScale {
+    double s, inv;
+    int bad, pad;
+};
+
+__global__ void __launch_bounds__(TT_THREADS) tt_max_kernel(const double *synth, const double *data, unsigned *top,
+                                                            long long plane)
 {
-    const long long stride = (long long)gridDim.x * TT_THREADS;
-    for (long long i = (long long)blockIdx.x * TT_THREADS + threadIdx.x; i < n; i += stride)
-        out[i] = make_double2(in[i].x * s, 0.0);
+    const int b = blockIdx.y;
+    unsigned ms = 0u, md = 0u;
+    for (long long i = (long long)blockIdx.x * TT_THREADS + threadIdx.x; i < plane; i += (long long)gridDim.x * TT_THREADS) {
+        ms = max(ms, (unsigned)__double2hiint(synth[b * plane + i]) & 0x7fffffffu);
+        md = max(md, (unsigned)__double2hiint(data[b * plane + i]) & 0x7fffffffu);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        ms = max(ms, __shfl_xor_sync(0xffffffffu, ms, o));
+        md = max(md, __shfl_xor_sync(0xffffffffu, md, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(top + 2 * b, ms);
+        atomicMax(top + 2 * b + 1, md);
+    }
 }
 
-// Multiplier of COMPUTE_TT_GIZONBIRCH's derivative (driver.f90:913-917) on the full spectrum:
-// i 2 pi q / (nt dt) below nt/2, zero at q = nt/2 (and its mirror), the conjugate mirror above.
-__global__ void __launch_bounds__(TT_THREADS) tt_gb_kernel(double2 *data, int nt, int nx, long long n, double dt_min)
+__global__ void tt_scale_kernel(const unsigned *top, TTScale *scale, int nb)
 {
-    const int h = nt / 2;
+    const int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= nb) return;
+    const int es = (int)(top[2 * b] >> 20), ed = (int)(top[2 * b + 1] >> 20);  // biased exponents (0: zero or subnormal)
+    const int d = (es == 0 || ed == 0 || es == 0x7ff || ed == 0x7ff) ? 0 : max(-1000, min(1000, es - ed));
+    scale[b] = TTScale{__hiloint2double((1023 + d) << 20, 0), __hiloint2double((1023 - d) << 20, 0), ed == 0x7ff, 0};
+}
+
+// Real records into one complex plane: synthetic + i scale data (data that are not finite stay out of it).
+__global__ void __launch_bounds__(TT_THREADS) tt_load_kernel(const double *synth, const double *data, double2 *out,
+                                                             const TTScale *scale, long long n, long long plane)
+{
     const long long stride = (long long)gridDim.x * TT_THREADS;
     for (long long i = (long long)blockIdx.x * TT_THREADS + threadIdx.x; i < n; i += stride) {
-        const int q = (int)((i / nx) % nt);
-        int s = 0;
-        if (q < h) s = q;
-        else if (q > nt - h) s = -(nt - q);
-        const double om = 2.0 * TT_PI * (double)s / ((double)nt * dt_min);
-        const double2 v = data[i];
-        data[i] = make_double2(-om * v.y, om * v.x);
+        const TTScale c = scale[i / plane];
+        out[i] = make_double2(synth[i], c.bad ? 0.0 : data[i] * c.s);
+    }
+}
+
+// The spectra of one mode from Z = DFT2(synth + i data): acc = filter Z (both filtered records after the
+// inverse), and of the synthetic's spectrum S(k) = (Z(k) + conj Z(-k)) / 2: ccd = filter (i om S - om_gb S / 64),
+// whose inverse is ccdot + i u0dot / 64 where both are real (odd nt), or (u0d given) ccdot and u0dot apart.  (In
+// minutes u0dot is 60 times ccdot: the power of two keeps the rounding of either relative to itself.)  One block
+// per spectral row: its two frequencies cost a division each.
+constexpr double TT_GB_SCALE = 64.0;
+__global__ void __launch_bounds__(TT_THREADS) tt_mode_kernel(const double2 *Z, double2 *acc, double2 *ccd, double2 *u0d,
+                                                             const double *filter, int nt, int nx, double dt_min,
+                                                             int derivatives)
+{
+    __shared__ double w[2];
+    const int b = blockIdx.x / nt, t = blockIdx.x - b * nt;
+    if (threadIdx.x == 0) {
+        w[0] = tt_omega(t, nt, dt_min);
+        w[1] = tt_omega_gb(t, nt, dt_min);
+    }
+    __syncthreads();
+    const double om = w[0], gb = u0d ? w[1] : w[1] * (1.0 / TT_GB_SCALE);
+    const size_t row = ((size_t)b * nt + t) * nx, mirror = ((size_t)b * nt + (t ? nt - t : 0)) * nx;
+    for (int x = threadIdx.x; x < nx; x += TT_THREADS) {
+        const size_t i = row + x;
+        const double f = filter[(size_t)t * nx + x];
+        const double2 z = Z[i];
+        acc[i] = make_double2(z.x * f, z.y * f);
+        if (!derivatives) continue;
+        const double2 m = Z[mirror + (x ? nx - x : 0)];
+        const double sr = 0.5 * (z.x + m.x) * f, si = 0.5 * (z.y - m.y) * f;
+        if (u0d) {
+            ccd[i] = make_double2(-om * si, om * sr);
+            u0d[i] = make_double2(-gb * si, gb * sr);
+        } else {
+            ccd[i] = make_double2(-om * si - gb * sr, om * sr - gb * si);
+        }
+    }
+}
+
+// sum += filter * in.
+__global__ void __launch_bounds__(TT_THREADS) tt_sum_kernel(const double2 *in, double2 *sum, const double *filter,
+                                                            long long n, long long plane)
+{
+    const long long stride = (long long)gridDim.x * TT_THREADS;
+    for (long long i = (long long)blockIdx.x * TT_THREADS + threadIdx.x; i < n; i += stride) {
+        const double f = filter[i % plane];
+        const double2 v = in[i];
+        double2 o = sum[i];
+        o.x += v.x * f;
+        o.y += v.y * f;
+        sum[i] = o;
     }
 }
 
@@ -228,10 +296,10 @@ struct TTRow {
 // One warp per measured receiver (driver.f90:2040-2100): window pick (first maximum of
 // |Re acc| over the search range), travel time by Simpson sums (SIMPSON_REGULAR weights over
 // the whole record, integrals.f90:107-130) of w u0dot (u0 - u) and w u0dot^2, and the
-// normalisation con = Re(-tau / (sum_{lef..rig} ccdot^2 dt)).  u0dot holds nt times the
-// derivative (the c2r transform is unnormalised).
+// normalisation con = Re(-tau / (sum_{lef..rig} ccdot^2 dt)).  acc holds u0 + i scale u; ccdot the time
+// derivative and, where u0dot is null, u0dot / TT_GB_SCALE as imaginary part.
 __global__ void __launch_bounds__(TT_THREADS) tt_rows_kernel(TTRow *rows, int nrows, const double2 *acc,
-                                                             const double2 *dat, const double2 *u0dot,
+                                                             const TTScale *scale, const double2 *u0dot,
                                                              const double2 *ccdot, int nt, int nx, int halftime,
                                                              int given, double dt_min)
 {
@@ -259,14 +327,21 @@ __global__ void __launch_bounds__(TT_THREADS) tt_rows_kernel(TTRow *rows, int nr
         r.rig = min(bi + halftime, nt);
     }
     double num = 0.0, den = 0.0, sr = 0.0, si = 0.0;
-    const double inv_nt = 1.0 / (double)nt;
+    const TTScale sc = scale[r.b];
     for (int t = r.lef + lane; t <= r.rig; t += WARP) {  // 1-based t
         const double wgt = (t == 1 || t == nt) ? 1.0 : ((t % 2 == 0) ? 4.0 : 2.0);
-        const double ud = at(u0dot, t - 1).x * inv_nt;
-        const double u0 = at(acc, t - 1).x, u = at(dat, t - 1).x;
+        double2 c = at(ccdot, t - 1);
+        const double2 z = at(acc, t - 1);
+        double ud;
+        if (u0dot) {
+            ud = at(u0dot, t - 1).x;
+        } else {
+            ud = c.y * TT_GB_SCALE;
+            c.y = 0.0;
+        }
+        const double u0 = z.x, u = sc.bad ? nan("") : z.y * sc.inv;
         num += wgt * (ud * (u0 - u));
         den += wgt * (ud * ud);
-        const double2 c = at(ccdot, t - 1);
         sr += c.x * c.x - c.y * c.y;
         si += 2.0 * c.x * c.y;
     }
@@ -293,20 +368,22 @@ __global__ void __launch_bounds__(TT_THREADS) tt_rows_kernel(TTRow *rows, int nr
 // around it.  tau = NaN marks a receiver that is not measured: a window leaving the record or a
 // peak at the end of the lag range (the reference reads past its arrays there).
 __global__ void __launch_bounds__(TT_THREADS) tt_cc_kernel(TTRow *rows, int nrows, const double2 *acc,
-                                                           const double2 *dat, int nt, int nx, int halftime,
+                                                           const TTScale *scale, int nt, int nx, int halftime,
                                                            int given, double dt_min)
 {
     const int warp = (blockIdx.x * TT_THREADS + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= nrows) return;
     TTRow r = rows[warp];
     const size_t base = (size_t)r.b * nt * nx + r.x;
-    auto re = [&](const double2 *f, int t0) { return f[base + (size_t)t0 * nx].x; };  // 0-based record index
+    const TTScale sc = scale[r.b];
+    auto u0 = [&](int t0) { return acc[base + (size_t)t0 * nx].x; };  // 0-based record index
+    auto u = [&](int t0) { return sc.bad ? nan("") : acc[base + (size_t)t0 * nx].y * sc.inv; };
     if (!given) {
         const int a = max(r.timest, 1), e = min(r.timefin, nt);  // 1-based, clipped
         double best = -1.0;
         int bi = a;
         for (int t = a + lane; t <= e; t += WARP) {
-            const double v = fabs(re(acc, t - 1));
+            const double v = fabs(u0(t - 1));
             if (v > best) { best = v; bi = t; }
         }
 #pragma unroll
@@ -327,9 +404,9 @@ __global__ void __launch_bounds__(TT_THREADS) tt_cc_kernel(TTRow *rows, int nrow
             const int i = j - (n - 1);
             double c = 0.0;
             if (i <= 0) {
-                for (int k = 1; k <= n + i; k++) c += re(acc, w0 + k - i - 1) * re(dat, w0 + k - 1);
+                for (int k = 1; k <= n + i; k++) c += u0(w0 + k - i - 1) * u(w0 + k - 1);
             } else {
-                for (int k = 1; k <= n - i; k++) c += re(acc, w0 + k - 1) * re(dat, w0 + k + i - 1);
+                for (int k = 1; k <= n - i; k++) c += u0(w0 + k - 1) * u(w0 + k + i - 1);
             }
             return c * dt_min;
         };
@@ -360,7 +437,7 @@ __global__ void __launch_bounds__(TT_THREADS) tt_cc_kernel(TTRow *rows, int nrow
     }
 }
 
-// c(x_i, t) = con_i w_i(t) ccdot(x_i, t) at the measured receivers (the buffer is zeroed first).
+// Re c(x_i, t) = con_i w_i(t) Re ccdot(x_i, t) at the measured receivers (the buffer is zeroed first).
 __global__ void __launch_bounds__(TT_THREADS) tt_scatter_kernel(const TTRow *rows, int nrows, const double2 *ccdot,
                                                                 double2 *c, int nt, int nx)
 {
@@ -369,30 +446,21 @@ __global__ void __launch_bounds__(TT_THREADS) tt_scatter_kernel(const TTRow *row
     const TTRow r = rows[warp];
     const size_t base = (size_t)r.b * nt * nx + r.x;
     for (int t = r.lef + lane; t <= r.rig; t += WARP) {
-        const double2 v = ccdot[base + (size_t)(t - 1) * nx];
-        double2 &o = c[base + (size_t)(t - 1) * nx];
-        o.x += r.con * v.x;
-        o.y += r.con * v.y;
+        c[base + (size_t)(t - 1) * nx].x += r.con * ccdot[base + (size_t)(t - 1) * nx].x;
     }
 }
 
-// adj[b][nt-1-t][x] += Re(field[b][t][x]) (time reversal, driver.f90:2097-2099).
-__global__ void __launch_bounds__(TT_THREADS) tt_accum_kernel(const double2 *f, double *adj, int nt, int nx,
-                                                              long long n)
+// out[b][nt-1-t][x] = s Re(field[b][t][x]) (time reversal, driver.f90:2097-2099).
+__global__ void __launch_bounds__(TT_THREADS) tt_out_kernel(const double2 *f, double *out, int nt, int nx, long long n,
+                                                            double s)
 {
     const long long stride = (long long)gridDim.x * TT_THREADS;
     for (long long i = (long long)blockIdx.x * TT_THREADS + threadIdx.x; i < n; i += stride) {
         const long long plane = (long long)nt * nx;
         const long long b = i / plane, r = i - b * plane;
         const int t = (int)(r / nx), x = (int)(r - (long long)t * nx);
-        adj[b * plane + (long long)(nt - 1 - t) * nx + x] += f[i].x;
+        out[b * plane + (long long)(nt - 1 - t) * nx + x] = f[i].x * s;
     }
-}
-
-__global__ void __launch_bounds__(TT_THREADS) tt_scale_out_kernel(const double *adj, double *out, long long n, double s)
-{
-    const long long stride = (long long)gridDim.x * TT_THREADS;
-    for (long long i = (long long)blockIdx.x * TT_THREADS + threadIdx.x; i < n; i += stride) out[i] = adj[i] * s;
 }
 
 unsigned tt_grid(long long n)
@@ -406,8 +474,12 @@ unsigned tt_grid(long long n)
 struct sparc_tt_plan {
     int nx = 0, nt = 0, nb = 0;
     std::vector<void *> allocs;
-    double2 *S = nullptr, *D = nullptr, *ACC = nullptr, *DAT = nullptr, *CCD = nullptr, *U0D = nullptr, *C = nullptr;
-    double *adj = nullptr, *twr = nullptr, *twi = nullptr;
+    double2 *Z = nullptr, *ACC = nullptr, *CCD = nullptr, *U0D = nullptr, *C = nullptr, *ADJ = nullptr;
+    double *twr = nullptr, *twi = nullptr;
+    TTScale *scale = nullptr;
+    unsigned *top = nullptr;
+    TTTile *all = nullptr, *tiles = nullptr;  // every tile; those of the mode's measured columns
+    int width = 0, nall = 0;                  // columns of a tile, tiles of the batch
     double2 *wt = nullptr;
     TTRow *rows = nullptr;
     int cap = 0;
@@ -422,11 +494,13 @@ template <int N>
 cudaError_t fft_x_n(sparc_tt_plan *p, double2 *f, int inverse, cudaStream_t st)
 {
     const long long nrows = (long long)p->nb * p->nt;
-    const size_t smem = (size_t)TT_XWPB * 4 * N * sizeof(double);
-    auto k = tt_fft_x_kernel<N>;
+    using W = WFft<double, N, false>;
+    const int slots = TT_XWPB * W::ROWS;
+    const size_t smem = (size_t)slots * W::REGION * sizeof(double);
+    auto k = inverse ? tt_fft_x_kernel<N, true> : tt_fft_x_kernel<N, false>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k<<<(unsigned)((nrows + TT_XWPB - 1) / TT_XWPB), TT_XWPB * WARP, smem, st>>>(f, nrows, p->twr, p->twi, inverse);
+    k<<<(unsigned)((nrows + slots - 1) / slots), TT_XWPB * WARP, smem, st>>>(f, nrows, p->twr, p->twi);
     return cudaGetLastError();
 }
 
@@ -440,42 +514,70 @@ cudaError_t fft_x(sparc_tt_plan *p, double2 *f, int inverse, cudaStream_t st)
 
 size_t dft_t_smem(int nt) { return ((size_t)nt * TT_COLS + nt) * sizeof(double2); }
 
-template <int M, int WPB>
-cudaError_t bluestein_t(sparc_tt_plan *p, double2 *f, int inverse, cudaStream_t st)
+template <int M, int COLS>
+cudaError_t bluestein_t(sparc_tt_plan *p, double2 *f, int inverse, const TTTile *tiles, int n, cudaStream_t st)
 {
-    const size_t smem = (size_t)WPB * (4 * M + 2) * sizeof(double) + WPB * sizeof(int) + 16;
-    auto k = tt_bluestein_t_kernel<M, WPB>;
+    using W = WFft<double, M, false>;
+    const size_t smem = (size_t)COLS * (W::REGION + 1) * sizeof(double);
+    auto k = tt_bluestein_t_kernel<M, COLS>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    dim3 grid((p->nx + WPB - 1) / WPB, p->nb);
-    k<<<grid, WPB * WARP, smem, st>>>(f, p->nt, p->nx, p->chirp, p->bhat, p->btwr, p->btwi, inverse);
+    k<<<n, COLS * W::L, smem, st>>>(f, tiles, p->nt, p->nx, p->chirp, p->bhat, p->btwr, p->btwi, inverse);
     return cudaGetLastError();
 }
 
-cudaError_t dft_t(sparc_tt_plan *p, double2 *f, int inverse, cudaStream_t st)
+// Columns of a t transform's tile: Bluestein of length bm (0: the direct DFT).
+// Bound by the double-precision pipe, so blocks of a few warps that spread evenly over the SMs: 155 tiles of 8
+// columns (8 x 141 measured columns, length 512) took two waves of 152 SMs, 166 us; 2 columns are one 32-byte sector.
+int tile_width(int bm) { return bm == 0 ? TT_COLS : bm >= 512 ? 2 : bm == 256 ? 4 : 8; }
+
+cudaError_t dft_t(sparc_tt_plan *p, double2 *f, int inverse, const TTTile *tiles, int n, cudaStream_t st)
 {
+    if (n <= 0) return cudaSuccess;
     switch (p->bm) {
-        case 64: return bluestein_t<64, 8>(p, f, inverse, st);
-        case 128: return bluestein_t<128, 8>(p, f, inverse, st);
-        case 256: return bluestein_t<256, 8>(p, f, inverse, st);
-        case 512: return bluestein_t<512, 8>(p, f, inverse, st);
-        case 1024: return bluestein_t<1024, 4>(p, f, inverse, st);
+        case 64: return bluestein_t<64, 8>(p, f, inverse, tiles, n, st);
+        case 128: return bluestein_t<128, 8>(p, f, inverse, tiles, n, st);
+        case 256: return bluestein_t<256, 4>(p, f, inverse, tiles, n, st);
+        case 512: return bluestein_t<512, 2>(p, f, inverse, tiles, n, st);
+        case 1024: return bluestein_t<1024, 2>(p, f, inverse, tiles, n, st);
         default: break;
     }
     const size_t smem = dft_t_smem(p->nt);
     cudaError_t e = cudaFuncSetAttribute(tt_dft_t_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    dim3 grid((p->nx + TT_COLS - 1) / TT_COLS, p->nb);
-    tt_dft_t_kernel<<<grid, TT_THREADS, smem, st>>>(f, p->nt, p->nx, p->wt, inverse);
+    tt_dft_t_kernel<<<n, TT_THREADS, smem, st>>>(f, tiles, p->nt, p->nx, p->wt, inverse);
     return cudaGetLastError();
 }
 
-// 2-D transform over (x, t) of every source's plane.
-cudaError_t dft2(sparc_tt_plan *p, double2 *f, int inverse, cudaStream_t st)
+// Spectra and records of one mode: acc (and with derivatives ccdot, u0dot) along x everywhere, along t on the tiles.
+cudaError_t mode_records(sparc_tt_plan *p, const double *filter, double dt_min, bool derivatives, int ntiles, cudaStream_t st)
 {
-    cudaError_t e = fft_x(p, f, inverse, st);
-    if (e == cudaSuccess) e = dft_t(p, f, inverse, st);
+    double2 *u0d = derivatives && p->nt % 2 == 0 ? p->U0D : nullptr;
+    tt_mode_kernel<<<p->nb * p->nt, TT_THREADS, 0, st>>>(p->Z, p->ACC, p->CCD, u0d, filter, p->nt, p->nx, dt_min, derivatives);
+    cudaError_t e = cudaGetLastError();
+    double2 *f[3] = {p->ACC, derivatives ? p->CCD : nullptr, u0d};
+    for (double2 *q : f) {
+        if (!q) continue;
+        if (e == cudaSuccess) e = fft_x(p, q, 1, st);
+        if (e == cudaSuccess) e = dft_t(p, q, 1, p->tiles, ntiles, st);
+    }
     return e;
+}
+
+// The tiles of the rows' columns (rows [nrows][7] as the caller gives them), uploaded; their number.
+int row_tiles(sparc_tt_plan *p, const int *rows, int nrows, std::vector<TTTile> &list, cudaStream_t st, cudaError_t &e)
+{
+    const int per = (p->nx + p->width - 1) / p->width;
+    std::vector<char> on((size_t)p->nb * per, 0);
+    for (int r = 0; r < nrows; r++) on[(size_t)rows[7 * r] * per + rows[7 * r + 1] / p->width] = 1;
+    list.clear();
+    for (int b = 0; b < p->nb; b++)
+        for (int i = 0; i < per; i++)
+            if (on[(size_t)b * per + i]) list.push_back(TTTile{b, i * p->width});
+    e = cudaSuccess;
+    if (!list.empty())
+        e = cudaMemcpyAsync(p->tiles, list.data(), list.size() * sizeof(TTTile), cudaMemcpyHostToDevice, st);
+    return (int)list.size();
 }
 
 int tt_fail(const char *what, cudaError_t e)
@@ -506,12 +608,18 @@ int sparc_tt_plan_create(int nx, int nt, int nbatch, int max_rows, sparc_tt_plan
     p->nb = nbatch;
     p->cap = max_rows;
     const size_t n = (size_t)nbatch * nt * nx;
+    // Bluestein length: the smallest power of two M >= 2 nt - 1 in the FFT table (64..1024)
+    int M = 64;
+    while (M < 2 * nt - 1) M *= 2;
+    p->width = tile_width(M <= 1024 ? M : 0);
+    p->nall = (nx + p->width - 1) / p->width * nbatch;
     struct Req { void **ptr; size_t bytes; };
     std::vector<Req> reqs = {
-        {(void **)&p->S, n * sizeof(double2)}, {(void **)&p->D, n * sizeof(double2)},
-        {(void **)&p->ACC, n * sizeof(double2)}, {(void **)&p->DAT, n * sizeof(double2)},
-        {(void **)&p->CCD, n * sizeof(double2)}, {(void **)&p->U0D, n * sizeof(double2)},
-        {(void **)&p->C, n * sizeof(double2)}, {(void **)&p->adj, n * sizeof(double)},
+        {(void **)&p->Z, n * sizeof(double2)}, {(void **)&p->ACC, n * sizeof(double2)},
+        {(void **)&p->CCD, n * sizeof(double2)}, {(void **)&p->U0D, nt % 2 == 0 ? n * sizeof(double2) : 16},
+        {(void **)&p->C, n * sizeof(double2)}, {(void **)&p->ADJ, n * sizeof(double2)},
+        {(void **)&p->scale, nbatch * sizeof(TTScale)}, {(void **)&p->top, 2 * nbatch * sizeof(unsigned)},
+        {(void **)&p->all, p->nall * sizeof(TTTile)}, {(void **)&p->tiles, p->nall * sizeof(TTTile)},
         {(void **)&p->twr, nx * sizeof(double)}, {(void **)&p->twi, nx * sizeof(double)},
         {(void **)&p->wt, nt * sizeof(double2)}, {(void **)&p->rows, (size_t)max_rows * sizeof(TTRow)},
     };
@@ -534,10 +642,12 @@ int sparc_tt_plan_create(int nx, int nt, int nbatch, int max_rows, sparc_tt_plan
     cudaError_t e = cudaMemcpy(p->twr, tr.data(), nx * sizeof(double), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(p->twi, ti.data(), nx * sizeof(double), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(p->wt, w.data(), nt * sizeof(double2), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(p->adj, 0, n * sizeof(double));
-    // Bluestein tables: the smallest power of two M >= 2 nt - 1 in the FFT table (64..1024)
-    int M = 64;
-    while (M < 2 * nt - 1) M *= 2;
+    if (e == cudaSuccess) e = cudaMemset(p->ADJ, 0, n * sizeof(double2));
+    std::vector<TTTile> every;
+    for (int b = 0; b < nbatch; b++)
+        for (int x0 = 0; x0 < nx; x0 += p->width) every.push_back(TTTile{b, x0});
+    if (e == cudaSuccess) e = cudaMemcpy(p->all, every.data(), every.size() * sizeof(TTTile), cudaMemcpyHostToDevice);
+    // Bluestein tables
     if (e == cudaSuccess && M <= 1024) {
         p->bm = M;
         std::vector<double2> ch(nt), bext(M, make_double2(0.0, 0.0)), bh(M);
@@ -597,13 +707,17 @@ int sparc_tt_set_records(sparc_tt_plan_t *p, const double *synth, const double *
     if (!p || !synth || !data) return report_error(SPARC_ERR_ARG, "sparc_tt_set_records: null argument");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long long n = (long long)p->nb * p->nt * p->nx;
-    // real records into complex planes, then forward 2-D transforms (driver.f90:1840-1844)
-    tt_load_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(synth, p->S, n);
-    tt_load_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(data, p->D, n);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = dft2(p, p->S, 0, st);
-    if (e == cudaSuccess) e = dft2(p, p->D, 0, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(p->adj, 0, (size_t)n * sizeof(double), st);
+    // real records into one complex plane, then its forward 2-D transform (driver.f90:1840-1844)
+    const long long plane = (long long)p->nt * p->nx;
+    cudaError_t e = cudaMemsetAsync(p->top, 0, 2 * p->nb * sizeof(unsigned), st);
+    if (e != cudaSuccess) return tt_fail("sparc_tt_set_records", e);
+    tt_max_kernel<<<dim3(16, p->nb), TT_THREADS, 0, st>>>(synth, data, p->top, plane);
+    tt_scale_kernel<<<(p->nb + 127) / 128, 128, 0, st>>>(p->top, p->scale, p->nb);
+    tt_load_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(synth, data, p->Z, p->scale, n, plane);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = fft_x(p, p->Z, 0, st);
+    if (e == cudaSuccess) e = dft_t(p, p->Z, 0, p->all, p->nall, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(p->ADJ, 0, (size_t)n * sizeof(double2), st);
     return e == cudaSuccess ? SPARC_OK : tt_fail("sparc_tt_set_records", e);
 }
 
@@ -628,48 +742,28 @@ int sparc_tt_mode(sparc_tt_plan_t *p, const double *filter, int nrows, int *rows
         h[r] = TTRow{q[0], q[1], q[2], q[3], q[4], q[5], 0, 0, 0.0, 0.0};
     }
     cudaError_t e = cudaSuccess;
-    // filtered synthetic and data, the time derivative of the filtered synthetic (driver.f90:1990-2017)
-    tt_filter_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(p->S, p->ACC, filter, nt, nx, n, 0, dt_min);
-    tt_filter_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(p->D, p->DAT, filter, nt, nx, n, 0, dt_min);
-    tt_filter_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(p->S, p->CCD, filter, nt, nx, n, 1, dt_min);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = dft2(p, p->ACC, 1, st);
-    if (e == cudaSuccess) e = dft2(p, p->DAT, 1, st);
-    if (e == cudaSuccess) e = dft2(p, p->CCD, 1, st);
-    // Gizon-Birch derivative of every synthetic column along t (driver.f90:905-923)
-    if (e == cudaSuccess) {
-        tt_real_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(p->ACC, p->U0D, n, 1.0);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = dft_t(p, p->U0D, 0, st);
-    if (e == cudaSuccess) {
-        tt_gb_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(p->U0D, nt, nx, n, dt_min);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = dft_t(p, p->U0D, 1, st);
+    std::vector<TTTile> list;
+    const int ntiles = row_tiles(p, rows, nrows, list, st, e);
     if (e == cudaSuccess && nrows > 0) {
-        e = cudaMemcpyAsync(p->rows, h.data(), nrows * sizeof(TTRow), cudaMemcpyHostToDevice, st);
+        // filtered synthetic and data, the derivatives of the filtered synthetic (driver.f90:1990-2017, 905-923)
+        e = mode_records(p, filter, dt_min, true, ntiles, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(p->rows, h.data(), nrows * sizeof(TTRow), cudaMemcpyHostToDevice, st);
+        const unsigned g = (unsigned)(((long long)nrows * WARP + TT_THREADS - 1) / TT_THREADS);
         if (e == cudaSuccess) {
-            const unsigned g = (unsigned)(((long long)nrows * WARP + TT_THREADS - 1) / TT_THREADS);
-            tt_rows_kernel<<<g, TT_THREADS, 0, st>>>(p->rows, nrows, p->ACC, p->DAT, p->U0D, p->CCD, nt, nx, halftime,
-                                                     given, dt_min);
+            tt_rows_kernel<<<g, TT_THREADS, 0, st>>>(p->rows, nrows, p->ACC, p->scale, nt % 2 == 0 ? p->U0D : nullptr,
+                                                     p->CCD, nt, nx, halftime, given, dt_min);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaMemsetAsync(p->C, 0, (size_t)n * sizeof(double2), st);
         if (e == cudaSuccess) {
-            const unsigned g = (unsigned)(((long long)nrows * WARP + TT_THREADS - 1) / TT_THREADS);
             tt_scatter_kernel<<<g, TT_THREADS, 0, st>>>(p->rows, nrows, p->CCD, p->C, nt, nx);
             e = cudaGetLastError();
         }
-        // adj_mode = Re IDFT2(filter * DFT2(c)), accumulated time-reversed
-        if (e == cudaSuccess) e = dft2(p, p->C, 0, st);
+        // adj_mode = Re IDFT2(filter * DFT2(Re c)): its spectrum is summed (columns that are not measured are zero)
+        if (e == cudaSuccess) e = dft_t(p, p->C, 0, p->tiles, ntiles, st);
+        if (e == cudaSuccess) e = fft_x(p, p->C, 0, st);
         if (e == cudaSuccess) {
-            tt_filter_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(p->C, p->C, filter, nt, nx, n, 0, dt_min);
-            e = cudaGetLastError();
-        }
-        if (e == cudaSuccess) e = dft2(p, p->C, 1, st);
-        if (e == cudaSuccess) {
-            tt_accum_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(p->C, p->adj, nt, nx, n);
+            tt_sum_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(p->C, p->ADJ, filter, n, (long long)nt * nx);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), p->rows, nrows * sizeof(TTRow), cudaMemcpyDeviceToHost, st);
@@ -703,16 +797,15 @@ int sparc_tt_misfit_mode(sparc_tt_plan_t *p, const double *filter, int nrows, in
             return report_error(SPARC_ERR_ARG, "sparc_tt_misfit_mode: empty search range");
         h[r] = TTRow{q[0], q[1], q[2], q[3], q[4], q[5], 0, 0, 0.0, 0.0};
     }
-    tt_filter_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(p->S, p->ACC, filter, nt, nx, n, 0, dt_min);
-    tt_filter_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(p->D, p->DAT, filter, nt, nx, n, 0, dt_min);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) e = dft2(p, p->ACC, 1, st);
-    if (e == cudaSuccess) e = dft2(p, p->DAT, 1, st);
+    cudaError_t e = cudaSuccess;
+    std::vector<TTTile> list;
+    const int ntiles = row_tiles(p, rows, nrows, list, st, e);
+    if (e == cudaSuccess && nrows > 0) e = mode_records(p, filter, dt_min, false, ntiles, st);
     if (e == cudaSuccess && nrows > 0) {
         e = cudaMemcpyAsync(p->rows, h.data(), nrows * sizeof(TTRow), cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) {
             const unsigned g = (unsigned)(((long long)nrows * WARP + TT_THREADS - 1) / TT_THREADS);
-            tt_cc_kernel<<<g, TT_THREADS, 0, st>>>(p->rows, nrows, p->ACC, p->DAT, nt, nx, halftime, given, dt_min);
+            tt_cc_kernel<<<g, TT_THREADS, 0, st>>>(p->rows, nrows, p->ACC, p->scale, nt, nx, halftime, given, dt_min);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), p->rows, nrows * sizeof(TTRow), cudaMemcpyDeviceToHost, st);
@@ -734,8 +827,13 @@ int sparc_tt_adjoint(sparc_tt_plan_t *p, double *adj, void *stream)
     if (!p || !adj) return report_error(SPARC_ERR_ARG, "sparc_tt_adjoint: null argument");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const long long n = (long long)p->nb * p->nt * p->nx;
-    tt_scale_out_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(p->adj, adj, n, (double)p->nt / 60.0);  // driver.f90:2201
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = cudaMemcpyAsync(p->C, p->ADJ, (size_t)n * sizeof(double2), cudaMemcpyDeviceToDevice, st);
+    if (e == cudaSuccess) e = fft_x(p, p->C, 1, st);
+    if (e == cudaSuccess) e = dft_t(p, p->C, 1, p->all, p->nall, st);
+    if (e == cudaSuccess) {
+        tt_out_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(p->C, adj, p->nt, p->nx, n, (double)p->nt / 60.0);  // driver.f90:2201
+        e = cudaGetLastError();
+    }
     return e == cudaSuccess ? SPARC_OK : tt_fail("sparc_tt_adjoint", e);
 }
 
