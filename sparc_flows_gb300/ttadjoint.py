@@ -56,37 +56,30 @@ def _grid(nx, nt, xlength_cm, outputcad):
 
 def ridge_filters(nx: int, nt: int, xlength_cm: float, outputcad: float) -> np.ndarray:
     """(9, nt, nx): f, p1..p7 ridges and the all-p-mode filter (driver.f90:1148-1718)."""
-    k, f = _grid(nx, nt, xlength_cm, outputcad)
-    out = np.zeros((9, nt, nx))
+    return _ridge_filters(nx, nt, xlength_cm, outputcad, "cpu").numpy()
+
+
+def _ridge_filters(nx: int, nt: int, xlength_cm: float, outputcad: float, device) -> torch.Tensor:
+    """ridge_filters as FP64 tensors on a device: all nine ridges in one pass of whole-array operations."""
+    k, f = (torch.as_tensor(v, dtype=torch.float64, device=device) for v in _grid(nx, nt, xlength_cm, outputcad))
+    poly = lambda c: _f(c[0]) + _f(c[1]) * k + _f(c[2]) * k ** 2  # noqa: E731
     df = 0.5
-    for p in range(9):
-        if p == 8:
-            m = np.ones((nt, nx))
-            flow = _f(1.6)
-        else:
-            low, high, flow = _RIDGE[p]
-            flow = _f(flow)
-            ph = [_f(v) for v in high]
-            f1 = ph[0] + ph[1] * k + ph[2] * k ** 2
-            if low == "sqrt":
-                f0 = _f(_P2_CONST) * np.sqrt(np.abs(k))
-            else:
-                pl = [_f(v) for v in low]
-                f0 = pl[0] + pl[1] * k + pl[2] * k ** 2
-            delta = (f1 - f0)[None, :]
-            d = f[:, None] - f0[None, :]
-            inside = (d < delta) & (d > 0)
-            with np.errstate(invalid="ignore", divide="ignore"):
-                if p == 0:
-                    shape = 0.5 * (1.0 + np.cos(PI * (d - delta / 2.0) / (delta / 2.0)))
-                else:
-                    shape = 0.5 * (1.0 + np.cos(PI * (np.abs(d) - np.abs(delta) * 0.5) / (np.abs(delta) * 0.5)))
-            m = np.where(inside, shape, 0.0)
-        taper = np.where(f < flow + df, 0.5 * (1.0 + np.cos(PI * (f - (flow + df)) / df)), 1.0)
-        m = m * taper[:, None]
-        m[f < flow] = 0.0
-        out[p] = m
-    return out
+    edge = []
+    for p in range(8):
+        low, high, _ = _RIDGE[p]
+        f0 = _f(_P2_CONST) * torch.sqrt(torch.abs(k)) if low == "sqrt" else poly(low)
+        edge.append(torch.stack((f0, poly(high) - f0)))
+    f0, delta = (e[:, None, :] for e in torch.stack(edge).unbind(1))
+    d = f[None, :, None] - f0
+    half = delta / 2.0
+    # the f mode's ridge is written without the absolute values of the p modes' (the same inside a ridge)
+    shape = 0.5 * (1.0 + torch.cos(PI * (d - half) / half))
+    m = torch.ones((9, nt, nx), dtype=torch.float64, device=device)
+    m[:8] = torch.where((d < delta) & (d > 0), shape, torch.zeros_like(shape))
+    flow = torch.tensor([_f(_RIDGE[p][2]) for p in range(8)] + [_f(1.6)], dtype=torch.float64, device=device)[:, None]
+    ft = f[None, :]
+    taper = torch.where(ft < flow + df, 0.5 * (1.0 + torch.cos(PI * (ft - (flow + df)) / df)), torch.ones_like(flow + ft))
+    return m * torch.where(ft < flow, torch.zeros_like(taper), taper)[:, :, None]
 
 
 def freq_filter(f1: float, f2: float, nt: int, outputcad: float) -> np.ndarray:
@@ -101,16 +94,20 @@ def mode_filters(nx, nt, xlength_cm, outputcad, freq: dict) -> np.ndarray:
     (f1, f2) of the filter.params.allmodes / .0 / .1 / .2 files present ('allmodes', 0, 1, 2);
     as in the reference, a mode whose own file is absent is multiplied by the last frequency
     filter read (the all-modes one, a second time, or 1)."""
-    filt = ridge_filters(nx, nt, xlength_cm, outputcad)
+    return _mode_filters(nx, nt, xlength_cm, outputcad, freq, "cpu").numpy()
+
+
+def _mode_filters(nx, nt, xlength_cm, outputcad, freq: dict, device) -> torch.Tensor:
+    filt = _ridge_filters(nx, nt, xlength_cm, outputcad, device)
     ff = np.ones(nt)
     if "allmodes" in freq:
         ff = freq_filter(*freq["allmodes"], nt, outputcad)
-    filt *= ff[None, :, None]
+    every = [ff] * 9
     for p in (0, 1, 2):
         if p in freq:
             ff = freq_filter(*freq[p], nt, outputcad)
-        filt[p] *= ff[:, None]
-    return filt
+        every[p] = every[p] * ff
+    return filt * torch.as_tensor(np.stack(every), dtype=torch.float64, device=device)[:, :, None]
 
 
 def _read_floats(path: str, n: int) -> list[float]:
@@ -143,24 +140,33 @@ def read_measurement_files(directory: str):
 BANDS = [(2.0, 3.5), (3.5, 4.5), (4.5, 6.0)]  # MISFIT_ALL's frequency bands, driver.f90:2376-2385
 
 
+# first-bounce polynomials in distance (minutes): window pick of ADJOINT_SOURCE_FILT and of MISFIT_ALL
+_BOUNCE = ((-0.000417147774671, 0.313350998096, 17.9609631186), (-0.00028361249034, 0.29270337114, 36.4398734578))
+_BOUNCE_MISFIT = ((-1.45511095e-04, 2.72140632e-01, 2.16331969e+01), (3.85746516e-08, 2.21324786e-01, 4.36702155e+01))
+
+
+def _bounce_range(poly, dist, dt_min):
+    return tuple(np.floor((_f(c[0]) * dist ** 2 + _f(c[1]) * dist + _f(c[2])) * (1.0 / dt_min)).astype(np.int64)
+                 for c in poly)
+
+
+def _search_ranges(pord: int, dist: np.ndarray, dt_min: float, misfit: bool = False):
+    """timest, timefin of the window picks at distances dist (driver.f90:2046-2053, 2436-2446), 1-based."""
+    if pord != 8:
+        ts = np.floor(dist / _f(MODE_SPEED[pord]) * (1.0 / dt_min)).astype(np.int64)
+        return ts, ts + 40
+    return _bounce_range(_BOUNCE_MISFIT if misfit else _BOUNCE, dist, dt_min)
+
+
 def misfit_search_range(pord: int, dist: float, dt_min: float) -> tuple[int, int]:
     """timest, timefin of MISFIT_ALL's window pick (driver.f90:2436-2446): the f/p modes as in
     ADJOINT_SOURCE_FILT, the first bounce (pord 8) with its own polynomials."""
-    if pord != 8:
-        return search_range(pord, dist, dt_min)
-    ts = math.floor((_f(-1.45511095e-04) * dist ** 2 + _f(2.72140632e-01) * dist + _f(2.16331969e+01)) * (1.0 / dt_min))
-    tf = math.floor((_f(3.85746516e-08) * dist ** 2 + _f(2.21324786e-01) * dist + _f(4.36702155e+01)) * (1.0 / dt_min))
-    return ts, tf
+    return tuple(int(v) for v in _search_ranges(pord, np.float64(dist), dt_min, misfit=True))
 
 
 def search_range(pord: int, dist: float, dt_min: float) -> tuple[int, int]:
     """timest, timefin of the window pick (driver.f90:2046-2053), 1-based."""
-    if pord != 8:
-        ts = math.floor(dist / _f(MODE_SPEED[pord]) * (1.0 / dt_min))
-        return ts, ts + 40
-    ts = math.floor((_f(-0.000417147774671) * dist ** 2 + _f(0.313350998096) * dist + _f(17.9609631186)) * (1.0 / dt_min))
-    tf = math.floor((_f(-0.00028361249034) * dist ** 2 + _f(0.29270337114) * dist + _f(36.4398734578)) * (1.0 / dt_min))
-    return ts, tf
+    return tuple(int(v) for v in _search_ranges(pord, np.float64(dist), dt_min))
 
 
 class TTAdjoint:
@@ -183,6 +189,28 @@ class TTAdjoint:
         x = np.arange(self.nx) / self.nx
         return np.abs((x - 0.5) * self.xlength_cm * _f(1e-8) - x00)
 
+    def _rows(self, pord, x00s, modes, dt, windows, misfit=False) -> np.ndarray:
+        """The measured receivers of a mode, (n, 7) int32 rows (b, i, timest, timefin, lef, rig, 0) by source and
+        column; windows {b: [(lef, rig), ...]} in that order, or None to pick."""
+        mindist, maxdist, _ = modes[pord]
+        out = []
+        for b in range(self.nb):
+            dist = self.distances(x00s[b])
+            i = np.flatnonzero((dist > mindist) & (dist < maxdist))
+            ts, tf = _search_ranges(pord, dist[i], dt, misfit)
+            rows = np.zeros((len(i), 7), dtype=np.int32)
+            rows[:, 0], rows[:, 1], rows[:, 2], rows[:, 3] = b, i, ts, tf
+            if windows is None:
+                # a search range outside the record: the reference reads out of bounds
+                rows = rows[np.maximum(ts, 1) <= np.minimum(tf, self.nt)]
+            elif len(i):
+                given = windows.get(b, [])
+                if len(given) < len(i):
+                    raise StopIteration("fewer windows than measured receivers")
+                rows[:, 4:6] = np.asarray(given[:len(i)])
+            out.append(rows)
+        return np.ascontiguousarray(np.concatenate(out) if out else np.zeros((0, 7), dtype=np.int32))
+
     def run(self, synth, data, x00s, t_min: np.ndarray, modes: dict, freq: dict | None = None,
             windows: dict | None = None):
         """synth, data: (nb, nt, nx) records; x00s: source positions in Mm (master.pixels); t_min:
@@ -198,41 +226,31 @@ class TTAdjoint:
         capi.check(self.L.sparc_tt_set_records(self.plan, s.data_ptr(), d.data_ptr(), self._stream()),
                    "sparc_tt_set_records")
         dt = float(t_min[1] - t_min[0])
-        filt = torch.as_tensor(mode_filters(nx, nt, self.xlength_cm, self.outputcad, freq or {}),
-                               dtype=torch.float64, device=self.dev).contiguous()
+        filt = _mode_filters(nx, nt, self.xlength_cm, self.outputcad, freq or {}, self.dev).contiguous()
         misfit = np.zeros(nb)
         nmeas = np.zeros(nb, dtype=int)
         rows_out, wins_out = {}, {}
         for pord in sorted(modes):
-            mindist, maxdist, window = modes[pord]
-            halftime = int(math.floor(window / (2.0 * dt) + 0.5))
+            halftime = int(math.floor(modes[pord][2] / (2.0 * dt) + 0.5))
             given = windows is not None and pord in windows
-            rows = []
-            for b in range(nb):
-                dist = self.distances(x00s[b])
-                it = iter(windows[pord].get(b, [])) if given else None
-                for i in range(nx):
-                    if not (dist[i] > mindist and dist[i] < maxdist):
-                        continue
-                    ts, tf = search_range(pord, dist[i], dt)
-                    lef, rig = next(it) if given else (0, 0)
-                    if not given and max(ts, 1) > min(tf, nt):
-                        continue  # search range outside the record: the reference reads out of bounds
-                    rows.append((b, i, ts, tf, lef, rig, 0))
-            arr = np.ascontiguousarray(np.array(rows, dtype=np.int32).reshape(-1, 7))
-            tau = np.zeros(max(len(rows), 1))
-            capi.check(self.L.sparc_tt_mode(self.plan, filt[pord].data_ptr(), len(rows),
+            arr = self._rows(pord, x00s, modes, dt, windows[pord] if given else None)
+            tau = np.zeros(max(len(arr), 1))
+            capi.check(self.L.sparc_tt_mode(self.plan, filt[pord].data_ptr(), len(arr),
                                             arr.ctypes.data_as(ctypes.POINTER(ctypes.c_int)), halftime, int(given),
                                             dt, tau.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), self._stream()),
                        "sparc_tt_mode")
+            if given:
+                arr[:, [2, 3, 6]] = 0
             per_b, per_w = {}, {}
-            for r, (b, i, ts, tf, lef, rig, loc) in enumerate(arr.tolist()):
-                if given:
-                    loc = ts = tf = 0
-                per_b.setdefault(b, []).append((i + 1, tau[r] * 60.0, lef, rig, loc, ts, tf))
-                per_w.setdefault(b, []).append((lef, rig))
-                misfit[b] += tau[r] ** 2
-                nmeas[b] += 1
+            for b in np.unique(arr[:, 0]).tolist():
+                one = arr[:, 0] == b
+                q, tt = arr[one], tau[:len(arr)][one]
+                lef, rig = q[:, 4].tolist(), q[:, 5].tolist()
+                per_b[b] = list(zip((q[:, 1] + 1).tolist(), (tt * 60.0).tolist(), lef, rig, q[:, 6].tolist(),
+                                    q[:, 2].tolist(), q[:, 3].tolist()))
+                per_w[b] = list(zip(lef, rig))
+                misfit[b] = np.cumsum(np.concatenate(([misfit[b]], tt ** 2)))[-1]  # in the order of the receivers
+                nmeas[b] += len(q)
             rows_out[pord], wins_out[pord] = per_b, per_w
         adj = torch.empty((nb, nt, nx), dtype=torch.float64, device=self.dev)
         capi.check(self.L.sparc_tt_adjoint(self.plan, adj.data_ptr(), self._stream()), "sparc_tt_adjoint")
@@ -250,42 +268,31 @@ class TTAdjoint:
         capi.check(self.L.sparc_tt_set_records(self.plan, s.data_ptr(), d.data_ptr(), self._stream()),
                    "sparc_tt_set_records")
         dt = float(t_min[1] - t_min[0])
-        ridges = ridge_filters(nx, nt, self.xlength_cm, self.outputcad)
+        ridges = _ridge_filters(nx, nt, self.xlength_cm, self.outputcad, self.dev)
         out = []
         for fb, (left, right) in enumerate(BANDS, start=1):
-            ff = freq_filter(left, right, nt, self.outputcad)
+            ff = torch.as_tensor(freq_filter(left, right, nt, self.outputcad), device=self.dev)
             nmeas = np.zeros((nb, 11), dtype=int)
             mis = np.zeros((nb, 11))
             wins = {}
             for pord in sorted(modes):
-                mindist, maxdist, window = modes[pord]
-                halftime = int(math.floor(window / (2.0 * dt) + 0.5))
+                halftime = int(math.floor(modes[pord][2] / (2.0 * dt) + 0.5))
                 given = windows is not None and fb in windows and pord in windows[fb]
-                rows = []
-                for b in range(nb):
-                    dist = self.distances(x00s[b])
-                    it = iter(windows[fb][pord].get(b, [])) if given else None
-                    for i in range(nx):
-                        if not (dist[i] > mindist and dist[i] < maxdist):
-                            continue
-                        ts, tf = misfit_search_range(pord, dist[i], dt)
-                        lef, rig = next(it) if given else (0, 0)
-                        if not given and max(ts, 1) > min(tf, nt):
-                            continue
-                        rows.append((b, i, ts, tf, lef, rig, 0))
-                arr = np.ascontiguousarray(np.array(rows, dtype=np.int32).reshape(-1, 7))
-                tau = np.zeros(max(len(rows), 1))
-                filt = torch.as_tensor(ridges[pord] * ff[:, None], dtype=torch.float64, device=self.dev).contiguous()
-                capi.check(self.L.sparc_tt_misfit_mode(self.plan, filt.data_ptr(), len(rows),
+                arr = self._rows(pord, x00s, modes, dt, windows[fb][pord] if given else None, misfit=True)
+                tau = np.zeros(max(len(arr), 1))
+                filt = (ridges[pord] * ff[:, None]).contiguous()
+                capi.check(self.L.sparc_tt_misfit_mode(self.plan, filt.data_ptr(), len(arr),
                                                        arr.ctypes.data_as(ctypes.POINTER(ctypes.c_int)), halftime,
                                                        int(given), dt, tau.ctypes.data_as(ctypes.POINTER(ctypes.c_double)),
                                                        self._stream()), "sparc_tt_misfit_mode")
                 per_w = {}
-                for r, (b, i, ts, tf, lef, rig, loc) in enumerate(arr.tolist()):
-                    per_w.setdefault(b, []).append((lef, rig))
-                    if np.isfinite(tau[r]):
-                        mis[b, pord] += tau[r] ** 2
-                        nmeas[b, pord] += 1
+                for b in np.unique(arr[:, 0]).tolist():
+                    one = arr[:, 0] == b
+                    q, tt = arr[one], tau[:len(arr)][one]
+                    per_w[b] = list(zip(q[:, 4].tolist(), q[:, 5].tolist()))
+                    tt = tt[np.isfinite(tt)]
+                    mis[b, pord] += np.cumsum(np.concatenate(([0.0], tt ** 2)))[-1]
+                    nmeas[b, pord] += len(tt)
                 wins[pord] = per_w
             out.append({"band": (left, right), "nmeas": nmeas, "misfit": 0.5 * mis, "windows": wins})
         return out
