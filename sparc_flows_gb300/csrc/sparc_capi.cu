@@ -743,8 +743,8 @@ int alloc_solver(sparc_plan *p)
             for (int d = 0; d < BAND_NPOW; d++) { S.band.rpow[d] = (float)rp; rp *= hb[0].r; }
             S.band_R = R;
             S.band_cw = bcw;
-            // specialised grids: the first phase's inputs staged by TMA (boxes of 32 columns x nz/2 rows)
-            S.have_maps32 = col_band_specialised(nx, nz, bcw, R) && nz % 2 == 0 && nz / 2 <= 256 &&
+            // 32-column blocks: the inputs of two phases staged by TMA (boxes of 32 columns x half the depth)
+            S.have_maps32 = bcw == 32 && nz / 2 <= 256 &&
                             encode_map(&S.maps32.A, A, nx, (long long)nb * 4 * nz, nz / 2, sizeof(float), 32) &&
                             encode_map(&S.maps32.SV, SV, nx, (long long)3 * nb * 2 * nz, nz / 2, sizeof(float), 32) &&
                             encode_map(&S.maps32.DX, DX, nx, (long long)nb * nz, nz / 2, sizeof(float), 32);

@@ -8,7 +8,7 @@
 // two field columns F[nz][CW], two right-hand-side columns [nz][CW], the carries of two
 // derivatives and seven depth profiles.
 //
-// On the specialised grids (TMA1) the first phase's three input tiles (xi_z and v_z of the state,
+// In 32-column blocks (TMA1) the first phase's three input tiles (xi_z and v_z of the state,
 // the RHS of v_z two stages back) are staged by 2-D bulk tensor copies into the two RHS tiles and
 // the second field tile, which are idle until phase 2: one thread issues them at kernel start,
 // and the block stages its PML rows and depth profiles while they are in flight.  Once phase 1
@@ -39,24 +39,26 @@ __device__ __forceinline__ bool band_tma_wait(uint64_t *bar, uint32_t &par, int 
     return true;
 }
 
-// One [nz][32] tile (two boxes of nz/2 rows) from rows row0 .. row0 + nz - 1 of map at x0.
-template <int NZ>
-__device__ __forceinline__ void band_tma_tile(float *dst, const CUtensorMap *map, int x0, int row0, uint64_t *bar)
+// One [nz][32] tile from rows row0 .. row0 + nz - 1 of map at x0 (field: row row0 of the array): two boxes of nz/2
+// rows and, where nz is odd, the last row as a copy of 128 bytes.
+__device__ __forceinline__ void band_tma_tile(float *dst, const CUtensorMap *map, const float *field, int nx, int x0,
+                                              int row0, int nz, uint64_t *bar)
 {
+    const int h = nz / 2;
     tma_load_2d(dst, map, x0, row0, bar);
-    tma_load_2d(dst + (NZ / 2) * 32, map, x0, row0 + NZ / 2, bar);
+    tma_load_2d(dst + (size_t)h * 32, map, x0, row0 + h, bar);
+    if (nz & 1) bulk_load(dst + (size_t)(nz - 1) * 32, field + (size_t)(nz - 1) * nx + x0, 128u, bar);
 }
 
 // NX, NZ: the grid as compile-time constants (0: taken from the arguments).  With them every
 // global and shared-memory offset of the unrolled row loops is an immediate, and with NZ a
 // multiple of R every thread group is full; the generic instantiation serves other grids.
-// TMA1 (CW = 32, even NZ with NZ/2 <= 256): the inputs of phases 1 and 3 staged by TMA through
-// the maps m.
+// TMA1 (CW = 32, nz <= 512): the inputs of phases 1 and 3 staged by TMA through the maps m.
 template <int CW, int R, int NX, int NZ, bool TMA1>
 __global__ void __launch_bounds__(CW *band_maxg<CW>(), band_minb<CW>())
     col_band_kernel(StepArgs<float> a, BandDev bd, const __grid_constant__ ColMaps32 m)
 {
-    static_assert(!TMA1 || (CW == 32 && NZ > 0 && NZ % 2 == 0 && NZ / 2 <= 256), "TMA1 geometry");
+    static_assert(!TMA1 || CW == 32, "TMA1 geometry");
     // tiles of nz x 32 floats are nz * 128 bytes long: with a 128-byte aligned base every tile and
     // half tile is a valid TMA destination
     extern __shared__ __align__(128) float smb[];
@@ -96,11 +98,13 @@ __global__ void __launch_bounds__(CW *band_maxg<CW>(), band_minb<CW>())
         __syncthreads();
         if (threadIdx.x == 0) {
             const uint32_t nt = 1 + (s >= 2 ? 1 : 0) + (s >= 3 ? 1 : 0);
-            mbar_arrive_expect_tx(bar, nt * (uint32_t)NZ * CW * sizeof(float));
+            mbar_arrive_expect_tx(bar, nt * (uint32_t)nz * CW * sizeof(float));
             const int x0 = blockIdx.x * CW;
-            band_tma_tile<NZ>(RA, &m.A, x0, (b * 4 + F_XIZ) * NZ, bar);
-            if (s >= 2) band_tma_tile<NZ>(RB, &m.A, x0, (b * 4 + F_VZ) * NZ, bar);
-            if (s >= 3) band_tma_tile<NZ>(FB, &m.SV, x0, ((a.slot_sm2 * a.nb + b) * 2 + 1) * NZ, bar);
+            const float *Af = a.A + (size_t)b * 4 * nz * nx;
+            band_tma_tile(RA, &m.A, Af + (size_t)F_XIZ * nz * nx, nx, x0, (b * 4 + F_XIZ) * nz, nz, bar);
+            if (s >= 2) band_tma_tile(RB, &m.A, Af + (size_t)F_VZ * nz * nx, nx, x0, (b * 4 + F_VZ) * nz, nz, bar);
+            if (s >= 3)
+                band_tma_tile(FB, &m.SV, svp(a, a.slot_sm2, b, 1), nx, x0, ((a.slot_sm2 * a.nb + b) * 2 + 1) * nz, nz, bar);
         }
     }
     for (int k = threadIdx.x; k < nz; k += blockDim.x) {  // depth profiles
@@ -188,10 +192,10 @@ __global__ void __launch_bounds__(CW *band_maxg<CW>(), band_minb<CW>())
         // ordered before the copies by the barrier above and the proxy fence
         if (threadIdx.x == 0) {
             fence_proxy_async_smem();
-            mbar_arrive_expect_tx(bar, 2u * NZ * CW * sizeof(float));
+            mbar_arrive_expect_tx(bar, 2u * nz * CW * sizeof(float));
             const int x0 = blockIdx.x * CW;
-            band_tma_tile<NZ>(RB, &m.DX, x0, b * NZ, bar);
-            band_tma_tile<NZ>(FB, &m.A, x0, (b * 4 + F_VX) * NZ, bar);
+            band_tma_tile(RB, &m.DX, a.DX + (size_t)b * F, nx, x0, b * nz, nz, bar);
+            band_tma_tile(FB, &m.A, Ab + F_VX * F, nx, x0, (b * 4 + F_VX) * nz, nz, bar);
         }
     }
     // L2 prefetch of phase 3's per-point inputs of this thread group's rows (one 128-byte line
@@ -474,6 +478,8 @@ cudaError_t launch_col_stage_band(const StepArgs<float> &a, const BandDev &bd, c
             }
         }
     }
+    if constexpr (CW == 32)
+        if (m32) return launch_band<CW, R, 0, 0, true>(a, bd, *m32, st);
     return launch_band<CW, R, 0, 0, false>(a, bd, ColMaps32{}, st);
 }
 
