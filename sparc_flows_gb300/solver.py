@@ -410,7 +410,7 @@ class WaveSolver:
 
     def describe(self) -> dict:
         """Kernels of the column and end-of-step passes of this plan and whether the row pass
-        overlaps the column pass's last wave (sparc_plan_describe)."""
+        may overlap the column pass's last wave (sparc_plan_describe)."""
         buf = ctypes.create_string_buffer(256)
         capi.check(self.L.sparc_plan_describe(self.plan, buf, 256), "sparc_plan_describe")
         return dict(kv.split("=", 1) for kv in buf.value.decode().split())
