@@ -242,8 +242,13 @@ int sparc_colmat_apply(const double *W, int nz, const double *in, double *out, i
  * [nb][2][nz][2 npmlhor] with forcing [nb][nx] added to RHS v_z at the injection row (the plan's state is left as
  * it is, its stage buffers are used), then takes la, lZ, lW, the adjoints of the step's outputs, to those of its
  * inputs in place and adds the gradients with respect to v0x, v0z and c2rho0 of each solve to gx, gz, gc
- * [nb][nz][nx].  work: sparc_adjoint_step_bytes device bytes.  Device pointers; no allocation, no synchronisation. */
+ * [nb][nz][nx].  work: sparc_adjoint_step_bytes device bytes, the first sparc_adjoint_cache_bytes of them what the
+ * stages leave for their transposes.  sparc_adjoint_replay advances the plan by one step and writes that to cache;
+ * with it in work and a0 NULL, sparc_adjoint_step recomputes nothing.  Device pointers; no allocation, no
+ * synchronisation. */
 size_t sparc_adjoint_step_bytes(const sparc_plan_t *p);
+size_t sparc_adjoint_cache_bytes(const sparc_plan_t *p);
+int sparc_adjoint_replay(sparc_plan_t *p, double *cache, void *stream);
 int sparc_adjoint_prepare(sparc_plan_t *p);
 int sparc_adjoint_step(sparc_plan_t *p, const double *a0, const double *Pz, const double *Px, const double *forcing,
                        double *la, double *lZ, double *lW, double *gx, double *gz, double *gc, void *work, void *stream);

@@ -36,6 +36,8 @@ SIGNATURES = {
     "sparc_checkpoint_bytes": (ctypes.c_size_t, [_vp]),
     "sparc_adjoint_step_bytes": (ctypes.c_size_t, [_vp]),
     "sparc_adjoint_prepare": (ctypes.c_int, [_vp]),
+    "sparc_adjoint_cache_bytes": (ctypes.c_size_t, [_vp]),
+    "sparc_adjoint_replay": (ctypes.c_int, [_vp, _vp, _vp]),
     "sparc_adjoint_step": (ctypes.c_int, [_vp] * 13),
     "sparc_colmat_apply": (ctypes.c_int, [_vp, ctypes.c_int, _vp, _vp, ctypes.c_int, ctypes.c_int, ctypes.c_int,
                                           ctypes.c_int, ctypes.c_int, _vp]),

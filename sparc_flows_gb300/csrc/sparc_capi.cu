@@ -1566,10 +1566,50 @@ int sparc_adjoint_prepare(sparc_plan_t *p)
     return SPARC_OK;
 }
 
+size_t sparc_adjoint_cache_bytes(const sparc_plan_t *p)
+{
+    return p ? (size_t)25 * p->cfg.nbatch * p->cfg.nx * p->cfg.nz * sizeof(double) : 0;
+}
+
+int sparc_adjoint_replay(sparc_plan_t *p, double *cache, void *stream)
+{
+    if (!p || !cache) return fail(SPARC_ERR_ARG, "sparc_adjoint_replay: null argument");
+    if (!p->have_zT || !p->have_bg || !p->have_src)
+        return fail(SPARC_ERR_STATE, "sparc_adjoint_replay: sparc_adjoint_prepare, background and source come first");
+    const cudaStream_t st = (cudaStream_t)stream;
+    const double *B = p->cfg.betas;
+    const size_t NF = (size_t)p->cfg.nbatch * p->cfg.nx * p->cfg.nz;
+    StepArgs<double> a = p->s64.a;  // the plan's step (enqueue_step), its stages' caches kept
+    a.fsign = 1.0;
+    a.unstretch_top = p->unstretch_top;
+    a.seis = a.snaps = nullptr;
+    a.nrec_cap = 0;
+    a.tile_cnt = nullptr;
+    for (int s = 1; s <= 5; s++) {
+        a.stage = s;
+        a.bs = B[s - 1];
+        a.bsm1 = s >= 2 ? B[s - 2] : 0.0;
+        a.slot_s = s % 3; a.slot_sm1 = (s - 1) % 3; a.slot_sm2 = (s + 1) % 3;
+        a.cache = cache + (size_t)(s - 1) * 5 * NF;
+        CK(launch_row_stage<double>(a, st));
+        CK(launch_col_stage<double>(a, st));
+    }
+    a.cache = nullptr;
+    a.stage = 6;
+    a.bs = 0.0; a.bsm1 = B[4];
+    a.slot_s = 0; a.slot_sm1 = 5 % 3; a.slot_sm2 = 4 % 3;
+    CK(launch_row_stage<double>(a, st));
+    a.stage = 7;
+    a.bs = B[4];
+    a.slot_s = 5 % 3; a.slot_sm1 = 4 % 3;
+    CK(end_step(p, a, st));
+    return SPARC_OK;
+}
+
 int sparc_adjoint_step(sparc_plan_t *p, const double *a0, const double *Pz, const double *Px, const double *forcing,
                        double *la, double *lZ, double *lW, double *gx, double *gz, double *gc, void *work, void *stream)
 {
-    if (!p || !a0 || !Pz || !Px || !forcing || !la || !lZ || !lW || !gx || !gz || !gc || !work)
+    if (!p || !la || !lZ || !lW || !gx || !gz || !gc || !work || (a0 && (!Pz || !Px || !forcing)))
         return fail(SPARC_ERR_ARG, "sparc_adjoint_step: null argument");
     if (!p->have_zT || !p->have_bg) return fail(SPARC_ERR_STATE, "sparc_adjoint_step: sparc_adjoint_prepare and the background come first");
     const cudaStream_t st = (cudaStream_t)stream;
@@ -1581,33 +1621,34 @@ int sparc_adjoint_step(sparc_plan_t *p, const double *a0, const double *Pz, cons
     AdjArgs g{};
     StepArgs<double> &a = g.a;
     a = p->s64.a;
-    double *inj = w + at[6], *tab = w + at[7];
-    int *time = (int *)(tab + 8), *idx = (int *)(tab + 9);
-    CK(launch_adj_tables(time, idx, tab, inj, c.nbatch * c.nx, st));
-    // the five stages of the step from (a0, Pz, Px), keeping what the transposed stages need
-    a.A = const_cast<double *>(a0);
-    a.PZ = const_cast<double *>(Pz);
-    a.PX = const_cast<double *>(Px);
-    a.fsign = 1.0;
-    a.unstretch_top = p->unstretch_top;
-    a.seis = a.snaps = nullptr;
-    a.nrec_cap = 0;
-    a.d_time = time;
-    a.src_until = 0;
-    a.ntab = 1;
-    a.src_w = tab;
-    a.src_idx = idx;
-    a.src_rows = forcing;
-    a.nrows = 1;
-    a.inj_scale = inj;
-    for (int s = 1; s <= 5; s++) {
-        a.stage = s;
-        a.bs = c.betas[s - 1];
-        a.bsm1 = s >= 2 ? c.betas[s - 2] : 0.0;
-        a.slot_s = s % 3; a.slot_sm1 = (s - 1) % 3; a.slot_sm2 = (s + 1) % 3;
-        a.cache = w + at[0] + (size_t)(s - 1) * 5 * NF;
-        CK(launch_row_stage<double>(a, st));
-        CK(launch_col_stage<double>(a, st));
+    if (a0) {  // the five stages of the step from (a0, Pz, Px), keeping what the transposed stages need
+        double *inj = w + at[6], *tab = w + at[7];
+        int *time = (int *)(tab + 8), *idx = (int *)(tab + 9);
+        CK(launch_adj_tables(time, idx, tab, inj, c.nbatch * c.nx, st));
+        a.A = const_cast<double *>(a0);
+        a.PZ = const_cast<double *>(Pz);
+        a.PX = const_cast<double *>(Px);
+        a.fsign = 1.0;
+        a.unstretch_top = p->unstretch_top;
+        a.seis = a.snaps = nullptr;
+        a.nrec_cap = 0;
+        a.d_time = time;
+        a.src_until = 0;
+        a.ntab = 1;
+        a.src_w = tab;
+        a.src_idx = idx;
+        a.src_rows = forcing;
+        a.nrows = 1;
+        a.inj_scale = inj;
+        for (int s = 1; s <= 5; s++) {
+            a.stage = s;
+            a.bs = c.betas[s - 1];
+            a.bsm1 = s >= 2 ? c.betas[s - 2] : 0.0;
+            a.slot_s = s % 3; a.slot_sm1 = (s - 1) % 3; a.slot_sm2 = (s + 1) % 3;
+            a.cache = w + at[0] + (size_t)(s - 1) * 5 * NF;
+            CK(launch_row_stage<double>(a, st));
+            CK(launch_col_stage<double>(a, st));
+        }
     }
     a.cache = nullptr;
     g.la = la; g.lZ = lZ; g.lW = lW;

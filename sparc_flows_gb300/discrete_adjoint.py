@@ -7,8 +7,8 @@ The reference has no discrete adjoint: its adjoint run is a time-reversed forwar
 flow negated (driver.f90:144-147) whose kernels match finite differences only to discretisation
 accuracy.  Here the forward solve is the device step of the plan (fused kernels, sparc_forward);
 the backward pass replays it segment by segment from HBM checkpoints (sparc_checkpoint_save /
-load), recomputes the five stage inputs of each step and applies the transposed stages in reverse
-order:
+load), keeping what the five stages of each step leave for their transposes, and applies the
+transposed stages in reverse order:
 
   x-derivative  D_x (spectral, Nyquist bin dropped) is real antisymmetric: D_x^T = -D_x, applied
                 with the device ddx;
@@ -30,8 +30,9 @@ The sound speed enters through p = -c^2 rho0 div - ...: dL/d(c^2 rho0) = -sum la
 stages and steps (the exact counterpart of kernel_c, with the PML profiles held fixed).
 StepOperators applies every operator one at a time (pointwise algebra as device tensor arithmetic,
 each derivative, transposed derivative and transposed filter one kernel): the form the tests take
-apart.  ExactGradient runs the fused reverse step (sparc_adjoint_step): the plan's own row and column
-passes recompute the stages, one x and one z pass per stage transpose them.
+apart.  ExactGradient runs the fused passes: the replay is the plan's own step with its stage caches
+kept (sparc_adjoint_replay; where they would not fit, sparc_adjoint_step runs the stages again), one x
+and one z pass per stage transpose them.
 """
 from __future__ import annotations
 
@@ -43,6 +44,10 @@ from .config import RSUN_CM
 from .solver import WaveSolver, _ptr, _stream
 
 F64 = torch.float64
+# Device bytes that a segment's stage caches may take (15 MB a step for one solve of 256 x 300, six times its state):
+# up to there the replay of a segment keeps them, above it keeps the states and the reverse steps run their five
+# stages again.  Kept: 76.1 ms for records and gradient of 30 steps at 256 x 300; run again: 92.4 ms.
+CACHE_BYTES = 2 << 30
 # FILTER_VARS_2D coefficients (physics2d.f90:509-583): c0 and the half-weights of neighbours 1..5
 FILTER_C = (0.75390625, 0.41015625, -0.234375, 0.087890625, -0.01953125, 0.001953125)
 
@@ -270,7 +275,7 @@ class ExactGradient:
     """Seismograms at receiver columns as a function of the stream function, with the exact
     gradient of any loss of them by the discrete adjoint.  The forward solve is the plan's device
     step; states are checkpointed every `segment` steps in HBM and each segment is replayed once
-    during the backward pass."""
+    during the backward pass, its stage caches kept where they fit CACHE_BYTES."""
 
     def __init__(self, ws: WaveSolver, receivers, segment: int = 25, use_graph: bool = True):
         self.ws, self.ops = ws, StepOperators(ws)
@@ -289,7 +294,17 @@ class ExactGradient:
             raise RuntimeError("unexpected checkpoint layout")
         self.row = -(-nbytes // 256) * 256
         self.ckpt = torch.empty((self.nseg, self.row), dtype=torch.uint8, device=ws.dev)
-        self.segbuf = torch.empty((self.seg, self.row), dtype=torch.uint8, device=ws.dev)
+        self._cache_row = int(ws.L.sparc_adjoint_cache_bytes(ws.plan))
+        steps = min(self.seg, n)
+        self._keep_caches = steps * self._cache_row <= CACHE_BYTES
+        self.segbuf = None
+        if self._keep_caches:
+            try:
+                self.segbuf = torch.empty((steps, self._cache_row), dtype=torch.uint8, device=ws.dev)
+            except torch.cuda.OutOfMemoryError:
+                self._keep_caches = False
+        if self.segbuf is None:
+            self.segbuf = torch.empty((self.seg, self.row), dtype=torch.uint8, device=ws.dev)
         self.seis = torch.zeros((nb, self.nrec, nx), dtype=F64, device=ws.dev)
         ws_rows = getattr(ws, "src_rows", None)
         if ws_rows is None:
@@ -337,12 +352,13 @@ class ExactGradient:
             capi.check(self.ws.L.sparc_adjoint_prepare(self.ws.plan), "sparc_adjoint_prepare")
         return self._s
 
-    def _reverse_step(self):
-        """Recompute the stages of one step from the static state and apply the transposed step
-        to the static adjoints in place, accumulating the gradients (sparc_adjoint_step: the fused
-        counterpart of StepOperators.step and step_T)."""
+    def _reverse_step(self, cached: bool = False):
+        """Recompute the stages of one step from the static state (cached: take them from the work's
+        cache) and apply the transposed step to the static adjoints in place, accumulating the gradients
+        (sparc_adjoint_step: the fused counterpart of StepOperators.step and step_T)."""
         S = self._s
-        args = [_ptr(S[k]) for k in ("a", "Pz", "Px", "f", "la", "lZ", "lW", "gx", "gz", "gc")]
+        args = [None if cached and k in ("a", "Pz", "Px", "f") else _ptr(S[k])
+                for k in ("a", "Pz", "Px", "f", "la", "lZ", "lW", "gx", "gz", "gc")]
         capi.check(self.ws.L.sparc_adjoint_step(self.ws.plan, *args, _ptr(self._work), _stream()), "sparc_adjoint_step")
 
     def _run_reverse_step(self):
@@ -356,11 +372,11 @@ class ExactGradient:
                 side.wait_stream(torch.cuda.current_stream(self.ws.dev))
                 with torch.cuda.stream(side):
                     for _ in range(2):
-                        self._reverse_step()
+                        self._reverse_step(self._keep_caches)
                 torch.cuda.current_stream(self.ws.dev).wait_stream(side)
                 g = torch.cuda.CUDAGraph()
                 with torch.cuda.graph(g):
-                    self._reverse_step()
+                    self._reverse_step(self._keep_caches)
                 self._graph = g
             except RuntimeError:
                 self.use_graph = False
@@ -369,7 +385,7 @@ class ExactGradient:
         if self._graph is not None:
             self._graph.replay()
         else:
-            self._reverse_step()
+            self._reverse_step(self._keep_caches)
 
     def gradient(self, psi: torch.Tensor, grad_rec: torch.Tensor) -> torch.Tensor:
         """dL/dpsi for dL/d(records at the receivers) = grad_rec (nb, nrec, nrcv), at the psi of
@@ -383,19 +399,25 @@ class ExactGradient:
         for m in range(self.nseg - 1, -1, -1):
             n0, n1 = m * self.seg, min((m + 1) * self.seg, n)
             ws.checkpoint_load(self.ckpt[m])
-            for j in range(n1 - n0):  # replay the segment, keeping the state before each step
-                ws.checkpoint_save(self.segbuf[j])
-                ws.run_steps(1, None, None, 0)
+            for j in range(n1 - n0):  # replay the segment, keeping each step's stage caches or the state before it
+                if self._keep_caches:
+                    capi.check(ws.L.sparc_adjoint_replay(ws.plan, _ptr(self.segbuf[j]), _stream()), "sparc_adjoint_replay")
+                else:
+                    ws.checkpoint_save(self.segbuf[j])
+                    ws.run_steps(1, None, None, 0)
             for step in range(n1 - 1, n0 - 1, -1):
                 if step % so == 0 and step // so < self.nrec:  # record taken after this step
                     S["la"][:, 3, ops.k_obs, self.rcv] += grad_rec[:, step // so, :]
-                for dst, src in zip((S["a"], S["Pz"], S["Px"]), self._views(self.segbuf[step - n0])):
-                    dst.copy_(src)
-                fc = self._forcing(step)
-                if fc is None:
-                    S["f"].zero_()
+                if self._keep_caches:
+                    self._work[:self._cache_row].copy_(self.segbuf[step - n0])
                 else:
-                    S["f"].copy_(fc)
+                    for dst, src in zip((S["a"], S["Pz"], S["Px"]), self._views(self.segbuf[step - n0])):
+                        dst.copy_(src)
+                    fc = self._forcing(step)
+                    if fc is None:
+                        S["f"].zero_()
+                    else:
+                        S["f"].copy_(fc)
                 self._run_reverse_step()
         self.last = {"v0x": S["gx"].sum(0), "v0z": S["gz"].sum(0), "c2rho0": S["gc"].sum(0)}
         return self.psi_gradient(self.last["v0x"], self.last["v0z"])

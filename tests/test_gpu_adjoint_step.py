@@ -42,3 +42,28 @@ def test_matches_operators(nx, nz, nb, bump, wide):
         err = float((x - y).norm() / y.norm())
         assert np.isfinite(err) and err <= 1e-11, (name, err)
     ws.close()
+
+
+@pytest.mark.parametrize("graph", [True, False])
+def test_kept_caches_equal_recomputed_stages(monkeypatch, graph):
+    """A segment's stage caches kept by its replay, or the states kept and every reverse step's stages recomputed:
+    the same kernels on values that differ by the rounding of the forcing (its two products in another order, 2 ulp),
+    which 37 steps carry on: far below 1e-12 of the norm."""
+    from sparc_flows_gb300 import discrete_adjoint as D
+    from sparc_flows_gb300.solver import WaveSolver
+    run = RunConfig(nx=128, nz=157, xlength_cm=100e8, nsteps=37, flows=True)
+    model = M.polytrope(157)
+    psi = torch.as_tensor(M.gaussian_psi(run, model, M.psi_amplitude_for_peak(run, model, 240.0)), device="cuda")
+    out = []
+    for limit in (1 << 40, 0):
+        monkeypatch.setattr(D, "CACHE_BYTES", limit)
+        ws = WaveSolver(run, model, nbatch=2, precision=64, psi=psi.cpu().numpy())
+        ws.set_forward_sources([M.SourceSpec(-5.0), M.SourceSpec(8.0)])
+        eg = D.ExactGradient(ws, receivers=[30, 64, 90], segment=10, use_graph=graph)
+        assert eg._keep_caches == (limit > 0)
+        rec = eg.forward(psi).clone()
+        g = eg.gradient(psi, rec)
+        out.append([rec, g] + [eg.last[k] for k in ("v0x", "v0z", "c2rho0")])
+        ws.close()
+    for a, b in zip(*out):
+        assert torch.isfinite(a).all() and float((a - b).norm()) <= 1e-12 * float(b.norm()) and float(b.norm()) > 0
