@@ -171,7 +171,9 @@ int sparc_get_time(sparc_plan_t *plan, int *time, void *stream);
  * leaves idle, as "column=<kernel> end=<kernel> stage_overlap=<0|1>" (NUL-terminated, at most len
  * bytes).  FP32 plans of 512 columns with the banded column pass have the overlap unless
  * SPARC_STAGE_OVERLAP=0 is set when the plan is created; it is taken where the column pass has a partial
- * last wave behind a full one (SPARC_STAGE_OVERLAP=1: everywhere). */
+ * last wave behind a full one (SPARC_STAGE_OVERLAP=1: everywhere).  Of a banded column kernel the first five
+ * template arguments are named: the fifth is 1 on a grid with compiled sizes whose inputs are bulk-copied, 0 on
+ * every other grid, bulk-copied or not. */
 int sparc_plan_describe(const sparc_plan_t *plan, char *buf, int len);
 
 /* Kernel construction from paired snapshots (kernels.f90:209-358): for record pair

@@ -1371,7 +1371,7 @@ int sparc_plan_describe(const sparc_plan_t *p, char *buf, int len)
                   (col_band_specialised(p->cfg.nx, p->cfg.nz, S.band_cw, S.band_R)
                        ? std::to_string(p->cfg.nx) + "," + std::to_string(p->cfg.nz)
                        : std::string("0,0")) +
-                  (S.have_maps32 ? ",1>" : ",0>");
+                  (S.have_maps32 && col_band_specialised(p->cfg.nx, p->cfg.nz, S.band_cw, S.band_R) ? ",1>" : ",0>");
         else if (S.have_maps && p->cfg.column_impl == 1) col = "col_stage_tma_kernel<float>";
         else col = "col_stage_kernel<float," + std::to_string(S.a.colw) + ">";
         end = S.a.ALO ? (S.end_stream ? "end_step_comp_kernel" : "end_step_kernel<float>")

@@ -8,7 +8,7 @@
 // two field columns F[nz][CW], two right-hand-side columns [nz][CW], the carries of two
 // derivatives and seven depth profiles.
 //
-// In 32-column blocks (TMA1) the first phase's three input tiles (xi_z and v_z of the state,
+// In 32-column blocks (TMA1, TMAG) the first phase's three input tiles (xi_z and v_z of the state,
 // the RHS of v_z two stages back) are staged by 2-D bulk tensor copies into the two RHS tiles and
 // the second field tile, which are idle until phase 2: one thread issues them at kernel start,
 // and the block stages its PML rows and depth profiles while they are in flight.  Once phase 1
@@ -53,12 +53,15 @@ __device__ __forceinline__ void band_tma_tile(float *dst, const CUtensorMap *map
 // NX, NZ: the grid as compile-time constants (0: taken from the arguments).  With them every
 // global and shared-memory offset of the unrolled row loops is an immediate, and with NZ a
 // multiple of R every thread group is full; the generic instantiation serves other grids.
-// TMA1 (CW = 32, nz <= 512): the inputs of phases 1 and 3 staged by TMA through the maps m.
-template <int CW, int R, int NX, int NZ, bool TMA1>
+// TMA1 on a specialised grid, TMAG on any other (CW = 32, nz <= 512): the inputs of phases 1 and 3 staged by TMA
+// through the maps m.
+template <int CW, int R, int NX, int NZ, bool TMA1, bool TMAG>
 __global__ void __launch_bounds__(CW *band_maxg<CW>(), band_minb<CW>())
     col_band_kernel(StepArgs<float> a, BandDev bd, const __grid_constant__ ColMaps32 m)
 {
-    static_assert(!TMA1 || CW == 32, "TMA1 geometry");
+    constexpr bool STAGED = TMA1 || TMAG;
+    static_assert(!STAGED || CW == 32, "staged geometry");
+    static_assert(!TMA1 || NX, "TMA1: a specialised grid");
     // tiles of nz x 32 floats are nz * 128 bytes long: with a 128-byte aligned base every tile and
     // half tile is a valid TMA destination
     extern __shared__ __align__(128) float smb[];
@@ -77,7 +80,7 @@ __global__ void __launch_bounds__(CW *band_maxg<CW>(), band_minb<CW>())
     // (replaced by their new RHS once used), az, bz, fdz
     const int nzp = a.nzpml;
     float *PS = KPB + 7 * nz;
-    // TMA1: the mbarrier, on the first 8-byte boundary after the PML rows
+    // STAGED: the mbarrier, on the first 8-byte boundary after the PML rows
     uint64_t *bar = reinterpret_cast<uint64_t *>(smb + ((PS - smb + 5 * nzp * CW + 1) & ~1));
     uint32_t tma_par = 0;  // parity of the mbarrier phase awaited next
     const int s = a.stage;
@@ -85,7 +88,7 @@ __global__ void __launch_bounds__(CW *band_maxg<CW>(), band_minb<CW>())
     // stage overlap: every block has started once all have passed this point, so the row pass
     // launched as this grid's dependent takes only SMs that no block of this grid still needs
     if (a.tile_cnt) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if constexpr (TMA1) {
+    if constexpr (STAGED) {
         if ((smem_u32(smb) & 127u) != 0) {  // uniform over the block: no copy is issued
             if (threadIdx.x == 0) atomicExch(a.d_err, SPARC_DEV_ERR_TMA_ALIGN);
             return;
@@ -154,7 +157,7 @@ __global__ void __launch_bounds__(CW *band_maxg<CW>(), band_minb<CW>())
     }
 
     // ---- 1: xi_z at stage s (scr xi_z = v_z of stage s-1 with the RHS boundary zeros)
-    if constexpr (TMA1) {
+    if constexpr (STAGED) {
         if (!band_tma_wait(bar, tma_par, a.d_err)) return;
     }
     float xz[R];
@@ -164,7 +167,7 @@ __global__ void __launch_bounds__(CW *band_maxg<CW>(), band_minb<CW>())
         if (m < n) {
             const int k = k0 + m;
             float v;
-            if constexpr (TMA1) {
+            if constexpr (STAGED) {
                 v = RA[k * CW + c];
                 if (s >= 2) {
                     const float avz = RB[k * CW + c];
@@ -187,7 +190,7 @@ __global__ void __launch_bounds__(CW *band_maxg<CW>(), band_minb<CW>())
         }
     }
     __syncthreads();
-    if constexpr (TMA1) {
+    if constexpr (STAGED) {
         // phase 3's tiles: dxi_x/dx -> RB, v_x of the state -> FB: phase 1's generic-proxy reads of both tiles are
         // ordered before the copies by the barrier above and the proxy fence
         if (threadIdx.x == 0) {
@@ -208,8 +211,8 @@ __global__ void __launch_bounds__(CW *band_maxg<CW>(), band_minb<CW>())
             if (m >= n) continue;
             const float *p;
             switch (ai) {
-                case 0: p = TMA1 ? nullptr : a.DX + (size_t)b * F; break;
-                case 1: p = TMA1 ? nullptr : Ab + F_VX * F; break;
+                case 0: p = STAGED ? nullptr : a.DX + (size_t)b * F; break;
+                case 1: p = STAGED ? nullptr : Ab + F_VX * F; break;
                 case 2: p = s >= 2 ? svp(a, a.slot_sm1, b, 0) : nullptr; break;
                 case 3: p = a.c2d ? a.c2rho0 + (size_t)b * a.bg2 : nullptr; break;
                 default: p = nullptr; break;
@@ -246,7 +249,7 @@ __global__ void __launch_bounds__(CW *band_maxg<CW>(), band_minb<CW>())
     {
         float d[R];
         band_eval<CW, R>(bd, bd.uv[2], C0, c, g, G, k0, n, nz, RA, d);
-        if constexpr (TMA1) {
+        if constexpr (STAGED) {
             if (!band_tma_wait(bar, tma_par, a.d_err)) return;
         }
 #pragma unroll
@@ -263,14 +266,14 @@ __global__ void __launch_bounds__(CW *band_maxg<CW>(), band_minb<CW>())
                     dzz += ps;
                     fd = PS[(4 * nzp + pi) * CW + c];
                 }
-                const float div = (TMA1 ? RB[k * CW + c] : __ldg(a.DX + (size_t)b * F + q)) + dzz;
+                const float div = (STAGED ? RB[k * CW + c] : __ldg(a.DX + (size_t)b * F + q)) + dzz;
                 const float c2r = a.c2d ? __ldg(a.c2rho0 + (size_t)b * a.bg2 + q) : Kc2[k];
                 const float gp = Kgp[k] * fd, gr = Kgr[k] * fd;
                 const float p = -c2r * div - gp * xz[m];
                 const float rho = -Kr0[k] * div - gr * xz[m];
                 xz[m] = rho * Kg[k];
                 FA[k * CW + c] = p;
-                float vx = TMA1 ? FB[k * CW + c] : __ldg(Ab + F_VX * F + q);
+                float vx = STAGED ? FB[k * CW + c] : __ldg(Ab + F_VX * F + q);
                 if (s >= 2) vx += bs * __ldg(svp(a, a.slot_sm1, b, 0) + q);
                 FB[k * CW + c] = vx;
             }
@@ -434,14 +437,14 @@ size_t col_band_smem_bytes(int nz, int nzpml, int R, int cw)
     }
 }
 
-template <int CW, int R, int NX, int NZ, bool TMA1>
+template <int CW, int R, int NX, int NZ, bool TMA1, bool TMAG = false>
 static cudaError_t launch_band(const StepArgs<float> &a, const BandDev &bd, const ColMaps32 &m, cudaStream_t st)
 {
     const int G = (a.nz + R - 1) / R;
     if (G > band_maxg<CW>() || a.nx % CW != 0 || R * G - a.nz >= R) return cudaErrorInvalidValue;
     if ((NX && a.nx != NX) || (NZ && a.nz != NZ)) return cudaErrorInvalidValue;
     const size_t smem = band_smem<CW, R>(a.nz, a.nzpml);
-    auto kern = col_band_kernel<CW, R, NX, NZ, TMA1>;
+    auto kern = col_band_kernel<CW, R, NX, NZ, TMA1, TMAG>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     dim3 grid(a.nx / CW, a.nb);
@@ -479,7 +482,7 @@ cudaError_t launch_col_stage_band(const StepArgs<float> &a, const BandDev &bd, c
         }
     }
     if constexpr (CW == 32)
-        if (m32) return launch_band<CW, R, 0, 0, true>(a, bd, *m32, st);
+        if (m32) return launch_band<CW, R, 0, 0, false, true>(a, bd, *m32, st);
     return launch_band<CW, R, 0, 0, false>(a, bd, ColMaps32{}, st);
 }
 

@@ -46,7 +46,7 @@ from .solver import WaveSolver, _ptr, _stream
 F64 = torch.float64
 # Device bytes that a segment's stage caches may take (15 MB a step for one solve of 256 x 300, six times its state):
 # up to there the replay of a segment keeps them, above it keeps the states and the reverse steps run their five
-# stages again.  Kept: 76.1 ms for records and gradient of 30 steps at 256 x 300; run again: 92.4 ms.
+# stages again.  Kept: 76.1 ms for records and gradient of 31 steps at 256 x 300; run again: 92.4 ms.
 CACHE_BYTES = 2 << 30
 # FILTER_VARS_2D coefficients (physics2d.f90:509-583): c0 and the half-weights of neighbours 1..5
 FILTER_C = (0.75390625, 0.41015625, -0.234375, 0.087890625, -0.01953125, 0.001953125)
@@ -296,7 +296,8 @@ class ExactGradient:
         self.ckpt = torch.empty((self.nseg, self.row), dtype=torch.uint8, device=ws.dev)
         self._cache_row = int(ws.L.sparc_adjoint_cache_bytes(ws.plan))
         steps = min(self.seg, n)
-        self._keep_caches = steps * self._cache_row <= CACHE_BYTES
+        # the replay that keeps them is the forward run's step (an adjoint run's has the flow negated)
+        self._keep_caches = not self.run.adjoint and steps * self._cache_row <= CACHE_BYTES
         self.segbuf = None
         if self._keep_caches:
             try:
