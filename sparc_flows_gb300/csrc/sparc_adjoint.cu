@@ -13,7 +13,7 @@
 // tridiagonal system (same chunks, factors of T^T) followed by the transposed stencil, O(nz) per column
 // where the dense product was O(nz^2); the value of the solve at a preset row is the preset's adjoint.  FP64,
 // bound by the double-precision pipe: the dense products alone took 600 operations per point and derivative.
-// One reverse step of 256 x 300 on a GB300: 1.2 ms (0.45 of it the recomputed stages), 5.2 ms as about 2000
+// One reverse step of 256 x 300 on a GB300: 1.2 ms (0.45 of it the stages, where they are run again), 5.2 ms as about 2000
 // kernels of single operators replayed from a graph.
 #include <cuda_runtime.h>
 
