@@ -189,50 +189,79 @@ __device__ __forceinline__ double tt_omega_gb(int t, int nt, double dt_min)
     return 2.0 * TT_PI * (double)q / ((double)nt * dt_min);
 }
 
-// Per source: the power of two that brings the data's largest value to the synthetic's binary exponent (1 where
-// either is zero or not finite), its inverse, and whether the data have a value that is not finite.
+// Per source: the power of two that brings the data's largest value to the synthetic's binary exponent, its inverse,
+// and what stands in the imaginary part.  A transform rounds relative to the larger of its two parts, so a part that
+// separate transforms would keep exactly (zero, or equal to the other one) is not taken from it: a source without a
+// synthetic or without data then has no travel time (0 / 0, or no correlation peak), and data equal to the synthetic
+// have a shift of exactly zero.
+enum { TT_PACKED = 0, TT_NOT_FINITE, TT_ZERO, TT_EQUAL };  // else alone: u NaN, u = 0, u = u0
 struct TTScale {
     double s, inv;
-    int bad, pad;
+    int kind, pad;
+};
+// Largest |value| of both planes as bit patterns, and whether any value differs.
+struct TTTop {
+    unsigned long long synth, data, differ;
 };
 
-__global__ void __launch_bounds__(TT_THREADS) tt_max_kernel(const double *synth, const double *data, unsigned *top,
+__global__ void __launch_bounds__(TT_THREADS) tt_max_kernel(const double *synth, const double *data, TTTop *top,
                                                             long long plane)
 {
     const int b = blockIdx.y;
-    unsigned ms = 0u, md = 0u;
+    const unsigned long long MAG = 0x7fffffffffffffffull;
+    unsigned long long ms = 0, md = 0;
+    bool differ = false;
     for (long long i = (long long)blockIdx.x * TT_THREADS + threadIdx.x; i < plane; i += (long long)gridDim.x * TT_THREADS) {
-        ms = max(ms, (unsigned)__double2hiint(synth[b * plane + i]) & 0x7fffffffu);
-        md = max(md, (unsigned)__double2hiint(data[b * plane + i]) & 0x7fffffffu);
+        const unsigned long long u = (unsigned long long)__double_as_longlong(synth[b * plane + i]),
+                                 v = (unsigned long long)__double_as_longlong(data[b * plane + i]);
+        ms = max(ms, u & MAG);
+        md = max(md, v & MAG);
+        differ |= u != v;
     }
     for (int o = 16; o > 0; o >>= 1) {
         ms = max(ms, __shfl_xor_sync(0xffffffffu, ms, o));
         md = max(md, __shfl_xor_sync(0xffffffffu, md, o));
     }
+    differ = __any_sync(0xffffffffu, differ);
     if ((threadIdx.x & 31) == 0) {
-        atomicMax(top + 2 * b, ms);
-        atomicMax(top + 2 * b + 1, md);
+        atomicMax(&top[b].synth, ms);
+        atomicMax(&top[b].data, md);
+        if (differ) atomicMax(&top[b].differ, 1ull);
     }
 }
 
-__global__ void tt_scale_kernel(const unsigned *top, TTScale *scale, int nb)
+// Biased binary exponent of |v| (bits, not zero), of a subnormal as if it were normalised.
+__device__ __forceinline__ int tt_exponent(unsigned long long bits)
+{
+    const int e = (int)(bits >> 52);
+    return e ? e : 12 - __clzll((long long)bits);
+}
+
+__global__ void tt_scale_kernel(const TTTop *top, TTScale *scale, int nb)
 {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= nb) return;
-    const int es = (int)(top[2 * b] >> 20), ed = (int)(top[2 * b + 1] >> 20);  // biased exponents (0: zero or subnormal)
-    const int d = (es == 0 || ed == 0 || es == 0x7ff || ed == 0x7ff) ? 0 : max(-1000, min(1000, es - ed));
-    scale[b] = TTScale{__hiloint2double((1023 + d) << 20, 0), __hiloint2double((1023 - d) << 20, 0), ed == 0x7ff, 0};
+    const unsigned long long ms = top[b].synth, md = top[b].data, INF = 0x7ffull << 52;
+    const int kind = md >= INF ? TT_NOT_FINITE : ms == 0 || md == 0 ? TT_ZERO : !top[b].differ ? TT_EQUAL : TT_PACKED;
+    const int d = kind == TT_PACKED && ms < INF ? max(-1000, min(1000, tt_exponent(ms) - tt_exponent(md))) : 0;
+    scale[b] = TTScale{__hiloint2double((1023 + d) << 20, 0), __hiloint2double((1023 - d) << 20, 0), kind, 0};
 }
 
-// Real records into one complex plane: synthetic + i scale data (data that are not finite stay out of it).
+// Real records into one complex plane: synthetic + i scale data, the synthetic alone where they are not packed.
 __global__ void __launch_bounds__(TT_THREADS) tt_load_kernel(const double *synth, const double *data, double2 *out,
                                                              const TTScale *scale, long long n, long long plane)
 {
     const long long stride = (long long)gridDim.x * TT_THREADS;
     for (long long i = (long long)blockIdx.x * TT_THREADS + threadIdx.x; i < n; i += stride) {
         const TTScale c = scale[i / plane];
-        out[i] = make_double2(synth[i], c.bad ? 0.0 : data[i] * c.s);
+        out[i] = make_double2(synth[i], c.kind == TT_PACKED ? data[i] * c.s : 0.0);
     }
+}
+
+// The data's value at an element z of the filtered records.
+__device__ __forceinline__ double tt_data(const TTScale &sc, const double2 &z)
+{
+    return sc.kind == TT_PACKED ? z.y * sc.inv : sc.kind == TT_ZERO ? 0.0 : sc.kind == TT_EQUAL ? z.x : nan("");
 }
 
 // The spectra of one mode from Z = DFT2(synth + i data): acc = filter Z (both filtered records after the
@@ -339,7 +368,7 @@ __global__ void __launch_bounds__(TT_THREADS) tt_rows_kernel(TTRow *rows, int nr
             ud = c.y * TT_GB_SCALE;
             c.y = 0.0;
         }
-        const double u0 = z.x, u = sc.bad ? nan("") : z.y * sc.inv;
+        const double u0 = z.x, u = tt_data(sc, z);
         num += wgt * (ud * (u0 - u));
         den += wgt * (ud * ud);
         sr += c.x * c.x - c.y * c.y;
@@ -377,7 +406,7 @@ __global__ void __launch_bounds__(TT_THREADS) tt_cc_kernel(TTRow *rows, int nrow
     const size_t base = (size_t)r.b * nt * nx + r.x;
     const TTScale sc = scale[r.b];
     auto u0 = [&](int t0) { return acc[base + (size_t)t0 * nx].x; };  // 0-based record index
-    auto u = [&](int t0) { return sc.bad ? nan("") : acc[base + (size_t)t0 * nx].y * sc.inv; };
+    auto u = [&](int t0) { return tt_data(sc, acc[base + (size_t)t0 * nx]); };
     if (!given) {
         const int a = max(r.timest, 1), e = min(r.timefin, nt);  // 1-based, clipped
         double best = -1.0;
@@ -477,7 +506,7 @@ struct sparc_tt_plan {
     double2 *Z = nullptr, *ACC = nullptr, *CCD = nullptr, *U0D = nullptr, *C = nullptr, *ADJ = nullptr;
     double *twr = nullptr, *twi = nullptr;
     TTScale *scale = nullptr;
-    unsigned *top = nullptr;
+    TTTop *top = nullptr;
     TTTile *all = nullptr, *tiles = nullptr;  // every tile; those of the mode's measured columns
     int width = 0, nall = 0;                  // columns of a tile, tiles of the batch
     double2 *wt = nullptr;
@@ -618,7 +647,7 @@ int sparc_tt_plan_create(int nx, int nt, int nbatch, int max_rows, sparc_tt_plan
         {(void **)&p->Z, n * sizeof(double2)}, {(void **)&p->ACC, n * sizeof(double2)},
         {(void **)&p->CCD, n * sizeof(double2)}, {(void **)&p->U0D, nt % 2 == 0 ? n * sizeof(double2) : 16},
         {(void **)&p->C, n * sizeof(double2)}, {(void **)&p->ADJ, n * sizeof(double2)},
-        {(void **)&p->scale, nbatch * sizeof(TTScale)}, {(void **)&p->top, 2 * nbatch * sizeof(unsigned)},
+        {(void **)&p->scale, nbatch * sizeof(TTScale)}, {(void **)&p->top, nbatch * sizeof(TTTop)},
         {(void **)&p->all, p->nall * sizeof(TTTile)}, {(void **)&p->tiles, p->nall * sizeof(TTTile)},
         {(void **)&p->twr, nx * sizeof(double)}, {(void **)&p->twi, nx * sizeof(double)},
         {(void **)&p->wt, nt * sizeof(double2)}, {(void **)&p->rows, (size_t)max_rows * sizeof(TTRow)},
@@ -709,7 +738,7 @@ int sparc_tt_set_records(sparc_tt_plan_t *p, const double *synth, const double *
     const long long n = (long long)p->nb * p->nt * p->nx;
     // real records into one complex plane, then its forward 2-D transform (driver.f90:1840-1844)
     const long long plane = (long long)p->nt * p->nx;
-    cudaError_t e = cudaMemsetAsync(p->top, 0, 2 * p->nb * sizeof(unsigned), st);
+    cudaError_t e = cudaMemsetAsync(p->top, 0, p->nb * sizeof(TTTop), st);
     if (e != cudaSuccess) return tt_fail("sparc_tt_set_records", e);
     tt_max_kernel<<<dim3(16, p->nb), TT_THREADS, 0, st>>>(synth, data, p->top, plane);
     tt_scale_kernel<<<(p->nb + 127) / 128, 128, 0, st>>>(p->top, p->scale, p->nb);
