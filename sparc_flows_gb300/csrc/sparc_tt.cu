@@ -8,13 +8,17 @@
 // receiver.  The sum over receivers is linear, and exp(-2 pi i k (i-1)/nx) is the forward DFT
 // kernel of a point at x_i, so it equals one transform per mode:
 //     adj_mode = Re IDFT2( filter * DFT2(c) ),  c(x_i, t) = con_i w_i(t) ccdot(x_i, t),
-// with c zero at unmeasured x.  The filters are real and even in k and f, so real records stay real:
+// with c zero at unmeasured x.  A filter is real; an even one (filter(-f, -k) = filter(f, k), as every ridge is)
+// keeps real records real:
 //   - synthetic and data share one transform as real and imaginary part (the data times a power of two of
 //     each source, which keeps the rounding of either relative to itself);
 //   - per mode one inverse transform gives both filtered records; a second, of the synthetic's spectrum, the
 //     time derivative ccdot and, as imaginary part, the Gizon-Birch derivative.  With an even record count the
 //     middle frequency makes ccdot complex, and the two derivatives take a transform each;
 //   - only Re c enters adj_mode, and the filtered spectra of all modes are summed: one inverse transform at the end;
+//   - with any other filter the picks and travel times see the real part of the filtered records, which is that of
+//     the filter's even part; ccdot is complex and enters adj_mode whole, and the two derivatives take a transform
+//     each.  The spectra's kernel notes such a filter, and the mode is run again for it;
 //   - only measured columns are transformed along t (their tiles of a few columns, listed on the host).
 // Per mode 3 transforms along x and 3 along t of the measured columns, where 4 and 7 of every column were taken.
 //
@@ -266,13 +270,14 @@ __device__ __forceinline__ double tt_data(const TTScale &sc, const double2 &z)
 
 // The spectra of one mode from Z = DFT2(synth + i data): acc = filter Z (both filtered records after the
 // inverse), and of the synthetic's spectrum S(k) = (Z(k) + conj Z(-k)) / 2: ccd = filter (i om S - om_gb S / 64),
-// whose inverse is ccdot + i u0dot / 64 where both are real (odd nt), or (u0d given) ccdot and u0dot apart.  (In
-// minutes u0dot is 60 times ccdot: the power of two keeps the rounding of either relative to itself.)  One block
-// per spectral row: its two frequencies cost a division each.
+// whose inverse is ccdot + i u0dot / 64 where both are real (odd nt, even filter), or (u0d given) ccdot and u0dot
+// apart.  (In minutes u0dot is 60 times ccdot: the power of two keeps the rounding of either relative to itself.)
+// acc and u0dot take the filter's even part, (f + f) / 2 = f of an even one: the real parts of the records.  odd: set
+// where the filter is not even (null: ccd and u0d are not wanted).  One block per spectral row: its two frequencies
+// cost a division each.
 constexpr double TT_GB_SCALE = 64.0;
 __global__ void __launch_bounds__(TT_THREADS) tt_mode_kernel(const double2 *Z, double2 *acc, double2 *ccd, double2 *u0d,
-                                                             const double *filter, int nt, int nx, double dt_min,
-                                                             int derivatives)
+                                                             const double *filter, int *odd, int nt, int nx, double dt_min)
 {
     __shared__ double w[2];
     const int b = blockIdx.x / nt, t = blockIdx.x - b * nt;
@@ -282,28 +287,31 @@ __global__ void __launch_bounds__(TT_THREADS) tt_mode_kernel(const double2 *Z, d
     }
     __syncthreads();
     const double om = w[0], gb = u0d ? w[1] : w[1] * (1.0 / TT_GB_SCALE);
-    const size_t row = ((size_t)b * nt + t) * nx, mirror = ((size_t)b * nt + (t ? nt - t : 0)) * nx;
+    const size_t row = ((size_t)b * nt + t) * nx, mt = t ? nt - t : 0, mirror = ((size_t)b * nt + mt) * nx;
     for (int x = threadIdx.x; x < nx; x += TT_THREADS) {
         const size_t i = row + x;
-        const double f = filter[(size_t)t * nx + x];
+        const int mx = x ? nx - x : 0;
+        const double f = filter[(size_t)t * nx + x], fm = filter[mt * nx + mx], e = 0.5 * (f + fm);
         const double2 z = Z[i];
-        acc[i] = make_double2(z.x * f, z.y * f);
-        if (!derivatives) continue;
-        const double2 m = Z[mirror + (x ? nx - x : 0)];
-        const double sr = 0.5 * (z.x + m.x) * f, si = 0.5 * (z.y - m.y) * f;
+        acc[i] = make_double2(z.x * e, z.y * e);
+        if (!odd) continue;
+        if (b == 0 && __double_as_longlong(f) != __double_as_longlong(fm)) *odd = 1;
+        const double2 m = Z[mirror + mx];
+        const double sr = 0.5 * (z.x + m.x), si = 0.5 * (z.y - m.y), cr = sr * f, ci = si * f;
         if (u0d) {
-            ccd[i] = make_double2(-om * si, om * sr);
-            u0d[i] = make_double2(-gb * si, gb * sr);
+            ccd[i] = make_double2(-om * ci, om * cr);
+            u0d[i] = make_double2(-gb * (si * e), gb * (sr * e));
         } else {
-            ccd[i] = make_double2(-om * si - gb * sr, om * sr - gb * si);
+            ccd[i] = make_double2(-om * ci - gb * cr, om * cr - gb * ci);
         }
     }
 }
 
-// sum += filter * in.
+// sum += filter * in, unless *skip.
 __global__ void __launch_bounds__(TT_THREADS) tt_sum_kernel(const double2 *in, double2 *sum, const double *filter,
-                                                            long long n, long long plane)
+                                                            const int *skip, long long n, long long plane)
 {
+    if (skip && *skip) return;
     const long long stride = (long long)gridDim.x * TT_THREADS;
     for (long long i = (long long)blockIdx.x * TT_THREADS + threadIdx.x; i < n; i += stride) {
         const double f = filter[i % plane];
@@ -466,9 +474,9 @@ __global__ void __launch_bounds__(TT_THREADS) tt_cc_kernel(TTRow *rows, int nrow
     }
 }
 
-// Re c(x_i, t) = con_i w_i(t) Re ccdot(x_i, t) at the measured receivers (the buffer is zeroed first).
+// Re c(x_i, t) = con_i w_i(t) Re ccdot(x_i, t) at the measured receivers (the buffer is zeroed first); whole: c.
 __global__ void __launch_bounds__(TT_THREADS) tt_scatter_kernel(const TTRow *rows, int nrows, const double2 *ccdot,
-                                                                double2 *c, int nt, int nx)
+                                                                double2 *c, int nt, int nx, bool whole)
 {
     const int warp = (blockIdx.x * TT_THREADS + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (warp >= nrows) return;
@@ -476,6 +484,7 @@ __global__ void __launch_bounds__(TT_THREADS) tt_scatter_kernel(const TTRow *row
     const size_t base = (size_t)r.b * nt * nx + r.x;
     for (int t = r.lef + lane; t <= r.rig; t += WARP) {
         c[base + (size_t)(t - 1) * nx].x += r.con * ccdot[base + (size_t)(t - 1) * nx].x;
+        if (whole) c[base + (size_t)(t - 1) * nx].y += r.con * ccdot[base + (size_t)(t - 1) * nx].y;
     }
 }
 
@@ -510,7 +519,7 @@ struct sparc_tt_plan {
     TTTile *all = nullptr, *tiles = nullptr;  // every tile; those of the mode's measured columns
     int width = 0, nall = 0;                  // columns of a tile, tiles of the batch
     double2 *wt = nullptr;
-    TTRow *rows = nullptr;
+    TTRow *rows = nullptr;  // of a call; in front of them one whose pad says that the mode's filter is not even
     int cap = 0;
     int bm = 0;  // Bluestein length (0: direct DFT along t)
     double2 *chirp = nullptr, *bhat = nullptr;
@@ -578,19 +587,57 @@ cudaError_t dft_t(sparc_tt_plan *p, double2 *f, int inverse, const TTTile *tiles
     return cudaGetLastError();
 }
 
-// Spectra and records of one mode: acc (and with derivatives ccdot, u0dot) along x everywhere, along t on the tiles.
-cudaError_t mode_records(sparc_tt_plan *p, const double *filter, double dt_min, bool derivatives, int ntiles, cudaStream_t st)
+// Spectra and records of one mode: acc (and with odd, see tt_mode_kernel, ccdot and, apart, u0dot) along x
+// everywhere, along t on the tiles.
+cudaError_t mode_records(sparc_tt_plan *p, const double *filter, double dt_min, int *odd, bool apart, int ntiles, cudaStream_t st)
 {
-    double2 *u0d = derivatives && p->nt % 2 == 0 ? p->U0D : nullptr;
-    tt_mode_kernel<<<p->nb * p->nt, TT_THREADS, 0, st>>>(p->Z, p->ACC, p->CCD, u0d, filter, p->nt, p->nx, dt_min, derivatives);
+    double2 *u0d = odd && apart ? p->U0D : nullptr;
+    tt_mode_kernel<<<p->nb * p->nt, TT_THREADS, 0, st>>>(p->Z, p->ACC, p->CCD, u0d, filter, odd, p->nt, p->nx, dt_min);
     cudaError_t e = cudaGetLastError();
-    double2 *f[3] = {p->ACC, derivatives ? p->CCD : nullptr, u0d};
+    double2 *f[3] = {p->ACC, odd ? p->CCD : nullptr, u0d};
     for (double2 *q : f) {
         if (!q) continue;
         if (e == cudaSuccess) e = fft_x(p, q, 1, st);
         if (e == cudaSuccess) e = dft_t(p, q, 1, p->tiles, ntiles, st);
     }
     return e;
+}
+
+// One mode of the adjoint source on the tiles of its rows h[1..] (h[0]: see sparc_tt_plan), which come back measured.
+// whole: for a filter that is not even; without it such a filter leaves the adjoint source as it is and sets h[0].pad.
+cudaError_t adjoint_mode(sparc_tt_plan *p, const double *filter, std::vector<TTRow> &h, int ntiles, int halftime, int given,
+                         double dt_min, bool whole, cudaStream_t st)
+{
+    const int nt = p->nt, nx = p->nx, nrows = (int)h.size() - 1;
+    const long long n = (long long)p->nb * nt * nx;
+    const bool apart = whole || nt % 2 == 0;
+    int *odd = &p->rows->pad;
+    TTRow *rows = p->rows + 1;
+    // filtered synthetic and data, the derivatives of the filtered synthetic (driver.f90:1990-2017, 905-923)
+    cudaError_t e = mode_records(p, filter, dt_min, odd, apart, ntiles, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(rows, h.data() + 1, nrows * sizeof(TTRow), cudaMemcpyHostToDevice, st);
+    const unsigned g = (unsigned)(((long long)nrows * WARP + TT_THREADS - 1) / TT_THREADS);
+    if (e == cudaSuccess) {
+        tt_rows_kernel<<<g, TT_THREADS, 0, st>>>(rows, nrows, p->ACC, p->scale, apart ? p->U0D : nullptr, p->CCD, nt, nx,
+                                                 halftime, given, dt_min);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemsetAsync(p->C, 0, (size_t)n * sizeof(double2), st);
+    if (e == cudaSuccess) {
+        tt_scatter_kernel<<<g, TT_THREADS, 0, st>>>(rows, nrows, p->CCD, p->C, nt, nx, whole);
+        e = cudaGetLastError();
+    }
+    // adj_mode = Re IDFT2(filter * DFT2(c)): its spectrum is summed (columns that are not measured are zero)
+    if (e == cudaSuccess) e = dft_t(p, p->C, 0, p->tiles, ntiles, st);
+    if (e == cudaSuccess) e = fft_x(p, p->C, 0, st);
+    if (e == cudaSuccess) {
+        tt_sum_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(p->C, p->ADJ, filter, whole ? nullptr : odd, n, (long long)nt * nx);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), p->rows, h.size() * sizeof(TTRow), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && whole) e = cudaMemsetAsync(odd, 0, sizeof(int), st);  // for the next mode
+    const cudaError_t w = cudaStreamSynchronize(st);
+    return e == cudaSuccess ? w : e;
 }
 
 // The tiles of the rows' columns (rows [nrows][7] as the caller gives them), uploaded; their number.
@@ -645,12 +692,12 @@ int sparc_tt_plan_create(int nx, int nt, int nbatch, int max_rows, sparc_tt_plan
     struct Req { void **ptr; size_t bytes; };
     std::vector<Req> reqs = {
         {(void **)&p->Z, n * sizeof(double2)}, {(void **)&p->ACC, n * sizeof(double2)},
-        {(void **)&p->CCD, n * sizeof(double2)}, {(void **)&p->U0D, nt % 2 == 0 ? n * sizeof(double2) : 16},
+        {(void **)&p->CCD, n * sizeof(double2)}, {(void **)&p->U0D, n * sizeof(double2)},
         {(void **)&p->C, n * sizeof(double2)}, {(void **)&p->ADJ, n * sizeof(double2)},
         {(void **)&p->scale, nbatch * sizeof(TTScale)}, {(void **)&p->top, nbatch * sizeof(TTTop)},
         {(void **)&p->all, p->nall * sizeof(TTTile)}, {(void **)&p->tiles, p->nall * sizeof(TTTile)},
         {(void **)&p->twr, nx * sizeof(double)}, {(void **)&p->twi, nx * sizeof(double)},
-        {(void **)&p->wt, nt * sizeof(double2)}, {(void **)&p->rows, (size_t)max_rows * sizeof(TTRow)},
+        {(void **)&p->wt, nt * sizeof(double2)}, {(void **)&p->rows, ((size_t)max_rows + 1) * sizeof(TTRow)},
     };
     for (auto &r : reqs) {
         cudaError_t e = cudaMalloc(r.ptr, r.bytes);
@@ -672,6 +719,7 @@ int sparc_tt_plan_create(int nx, int nt, int nbatch, int max_rows, sparc_tt_plan
     if (e == cudaSuccess) e = cudaMemcpy(p->twi, ti.data(), nx * sizeof(double), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(p->wt, w.data(), nt * sizeof(double2), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(p->ADJ, 0, n * sizeof(double2));
+    if (e == cudaSuccess) e = cudaMemset(p->rows, 0, sizeof(TTRow));
     std::vector<TTTile> every;
     for (int b = 0; b < nbatch; b++)
         for (int x0 = 0; x0 < nx; x0 += p->width) every.push_back(TTTile{b, x0});
@@ -757,7 +805,6 @@ int sparc_tt_mode(sparc_tt_plan_t *p, const double *filter, int nrows, int *rows
         return report_error(SPARC_ERR_ARG, "sparc_tt_mode: bad argument");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nt = p->nt, nx = p->nx;
-    const long long n = (long long)p->nb * nt * nx;
     for (int r = 0; r < nrows; r++) {
         const int *q = rows + 7 * r;
         if (q[0] < 0 || q[0] >= p->nb || q[1] < 0 || q[1] >= nx || (given && (q[4] < 1 || q[5] > nt || q[4] > q[5])))
@@ -765,46 +812,31 @@ int sparc_tt_mode(sparc_tt_plan_t *p, const double *filter, int nrows, int *rows
         if (!given && (max(q[2], 1) > min(q[3], nt)))
             return report_error(SPARC_ERR_ARG, "sparc_tt_mode: empty search range");
     }
-    std::vector<TTRow> h(nrows);
+    std::vector<TTRow> first(nrows + 1, TTRow{});
     for (int r = 0; r < nrows; r++) {
         const int *q = rows + 7 * r;
-        h[r] = TTRow{q[0], q[1], q[2], q[3], q[4], q[5], 0, 0, 0.0, 0.0};
+        first[r + 1] = TTRow{q[0], q[1], q[2], q[3], q[4], q[5], 0, 0, 0.0, 0.0};
     }
     cudaError_t e = cudaSuccess;
     std::vector<TTTile> list;
     const int ntiles = row_tiles(p, rows, nrows, list, st, e);
-    if (e == cudaSuccess && nrows > 0) {
-        // filtered synthetic and data, the derivatives of the filtered synthetic (driver.f90:1990-2017, 905-923)
-        e = mode_records(p, filter, dt_min, true, ntiles, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(p->rows, h.data(), nrows * sizeof(TTRow), cudaMemcpyHostToDevice, st);
-        const unsigned g = (unsigned)(((long long)nrows * WARP + TT_THREADS - 1) / TT_THREADS);
-        if (e == cudaSuccess) {
-            tt_rows_kernel<<<g, TT_THREADS, 0, st>>>(p->rows, nrows, p->ACC, p->scale, nt % 2 == 0 ? p->U0D : nullptr,
-                                                     p->CCD, nt, nx, halftime, given, dt_min);
-            e = cudaGetLastError();
+    std::vector<TTRow> h = first;
+    if (nrows == 0) {
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    } else {
+        if (e == cudaSuccess) e = adjoint_mode(p, filter, h, ntiles, halftime, given, dt_min, false, st);
+        if (e == cudaSuccess && h[0].pad) {
+            h = first;
+            e = adjoint_mode(p, filter, h, ntiles, halftime, given, dt_min, true, st);
         }
-        if (e == cudaSuccess) e = cudaMemsetAsync(p->C, 0, (size_t)n * sizeof(double2), st);
-        if (e == cudaSuccess) {
-            tt_scatter_kernel<<<g, TT_THREADS, 0, st>>>(p->rows, nrows, p->CCD, p->C, nt, nx);
-            e = cudaGetLastError();
-        }
-        // adj_mode = Re IDFT2(filter * DFT2(Re c)): its spectrum is summed (columns that are not measured are zero)
-        if (e == cudaSuccess) e = dft_t(p, p->C, 0, p->tiles, ntiles, st);
-        if (e == cudaSuccess) e = fft_x(p, p->C, 0, st);
-        if (e == cudaSuccess) {
-            tt_sum_kernel<<<tt_grid(n), TT_THREADS, 0, st>>>(p->C, p->ADJ, filter, n, (long long)nt * nx);
-            e = cudaGetLastError();
-        }
-        if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), p->rows, nrows * sizeof(TTRow), cudaMemcpyDeviceToHost, st);
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return tt_fail("sparc_tt_mode", e);
     for (int r = 0; r < nrows; r++) {
         int *q = rows + 7 * r;
-        q[4] = h[r].lef;
-        q[5] = h[r].rig;
-        q[6] = h[r].loc;
-        tau[r] = h[r].tau;
+        q[4] = h[r + 1].lef;
+        q[5] = h[r + 1].rig;
+        q[6] = h[r + 1].loc;
+        tau[r] = h[r + 1].tau;
     }
     return SPARC_OK;
 }
@@ -829,7 +861,7 @@ int sparc_tt_misfit_mode(sparc_tt_plan_t *p, const double *filter, int nrows, in
     cudaError_t e = cudaSuccess;
     std::vector<TTTile> list;
     const int ntiles = row_tiles(p, rows, nrows, list, st, e);
-    if (e == cudaSuccess && nrows > 0) e = mode_records(p, filter, dt_min, false, ntiles, st);
+    if (e == cudaSuccess && nrows > 0) e = mode_records(p, filter, dt_min, nullptr, false, ntiles, st);
     if (e == cudaSuccess && nrows > 0) {
         e = cudaMemcpyAsync(p->rows, h.data(), nrows * sizeof(TTRow), cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) {
