@@ -161,8 +161,7 @@ __device__ __forceinline__ void s3x_deriv(S3Pair<T, N, V> &p, const RowExchange<
         mr.add(p.re[m]);
         mi.add(p.im[m]);
     }
-    mr.template reduce<L>();
-    mi.template reduce<L>();
+    row_maxima(mr, mi, ex);
     p.sr = row_scale<T>(mr);
     p.si = row_scale<T>(mi);
 #pragma unroll
@@ -181,11 +180,11 @@ __global__ void __launch_bounds__(S3X_WARPS *WARP) s3x_kernel(S3Step<T> a, S3Fft
     using W = WFft<T, N>;
     constexpr int V = W::V, L = W::L;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int t = (threadIdx.x & 31) % L, slot = threadIdx.x / L;
-    const int pairs = a.nz * a.nb * a.ny / 2, first = blockIdx.x * (S3X_WARPS * W::ROWS) + slot;
+    const int t = threadIdx.x % L, slot = threadIdx.x / L;
+    const int pairs = a.nz * a.nb * a.ny / 2, first = blockIdx.x * (W::rows(S3X_WARPS)) + slot;
     const bool valid = first < pairs;
     const int r0 = 2 * (valid ? first : pairs - 1);
-    const RowExchange<T, N> ex{reinterpret_cast<T *>(smem_raw) + (size_t)slot * W::REGION};
+    const RowExchange<T, N> ex{reinterpret_cast<T *>(smem_raw) + (size_t)slot * W::REGION, slot};
     const int k = r0 / (a.nb * a.ny);
     const bool rim = k == 0 || k == a.nz - 1;
     const long long o0 = (long long)r0 * N + t, q0 = (long long)k * a.nxy + (long long)(r0 % a.ny) * N + t, F = a.F;
@@ -679,7 +678,7 @@ template <typename T, int N>
 static cudaError_t s3x_n(const S3Step<T> &a, const S3Fft<T> &f, int mode, cudaStream_t st)
 {
     using W = WFft<T, N>;
-    const int pairs = a.nz * a.nb * a.ny / 2, slots = S3X_WARPS * W::ROWS;
+    const int pairs = a.nz * a.nb * a.ny / 2, slots = W::rows(S3X_WARPS);
     const size_t smem = (size_t)slots * W::REGION * sizeof(T);
     auto k = mode == 0 ? s3x_kernel<T, N, 0> : mode == 1 ? s3x_kernel<T, N, 1> : s3x_kernel<T, N, 2>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -76,11 +76,11 @@ __global__ void __launch_bounds__(ADJ_WARPS *WARP) adj_row_kernel(AdjArgs g)
     constexpr int V = W::V, L = W::L;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const StepArgs<double> &a = g.a;
-    const int t = (threadIdx.x & 31) % L, slot = threadIdx.x / L;
-    const int rows = a.nb * a.nz, first = blockIdx.x * (ADJ_WARPS * W::ROWS) + slot;
+    const int t = threadIdx.x % L, slot = threadIdx.x / L;
+    const int rows = a.nb * a.nz, first = blockIdx.x * (W::rows(ADJ_WARPS)) + slot;
     const bool valid = first < rows;
     const int row = valid ? first : rows - 1, b = row / a.nz, k = row - b * a.nz;
-    const RowExchange<double, N> ex{reinterpret_cast<double *>(smem_raw) + (size_t)slot * W::REGION};
+    const RowExchange<double, N> ex{reinterpret_cast<double *>(smem_raw) + (size_t)slot * W::REGION, slot};
     const size_t F = (size_t)a.nz * N, q0 = (size_t)k * N + t;
     const double *lX = g.lX + (size_t)b * 4 * F + q0;
     double re[V], im[V];
@@ -92,8 +92,7 @@ __global__ void __launch_bounds__(ADJ_WARPS *WARP) adj_row_kernel(AdjArgs g)
             mr.add(re[m]);
             mi.add(im[m]);
         }
-        mr.template reduce<L>();
-        mi.template reduce<L>();
+        row_maxima(mr, mi, ex);
         sr = row_scale<double>(mr);
         si = row_scale<double>(mi);
 #pragma unroll
@@ -380,7 +379,7 @@ template <int N>
 cudaError_t adj_row_n(const AdjArgs &g, int mode, cudaStream_t st)
 {
     using W = WFft<double, N>;
-    const int rows = g.a.nb * g.a.nz, slots = ADJ_WARPS * W::ROWS;
+    const int rows = g.a.nb * g.a.nz, slots = W::rows(ADJ_WARPS);
     const size_t smem = (size_t)slots * W::REGION * sizeof(double);
     auto k = mode == 0 ? adj_row_kernel<N, 0> : mode == 1 ? adj_row_kernel<N, 1> : adj_row_kernel<N, 2>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

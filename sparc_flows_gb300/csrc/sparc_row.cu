@@ -135,21 +135,26 @@ __device__ __forceinline__ void row_mid_store_pml(const StepArgs<T> &a, const Ro
     }
 }
 
-// The row pass with the register transforms of sparc_wfft.cuh: WFft<T, N>::ROWS rows per warp, thread t of a
+// Resident blocks that the registers are limited for (0: no limit): four at 768 columns in FP32, eight rows on an SM (four solves of
+// 300 levels 299 us a step against 309 without the limit); at 1024 the limit costs more than it gives (308 against 294).
+template <typename T, int N>
+constexpr int row_blocks() { return sizeof(T) == 4 && N == 768 ? 4 : 0; }
+
+// The row pass with the register transforms of sparc_wfft.cuh: WFft<T, N>::L threads a row, thread t of a
 // row holding columns t + L m.
 template <typename T, int N, int MODE>
-__global__ void __launch_bounds__(ROW_WPB *WARP) row_stage_kernel(StepArgs<T> a, int region)
+__global__ void __launch_bounds__(ROW_WPB *WARP, row_blocks<T, N>()) row_stage_kernel(StepArgs<T> a, int region)
 {
     using W = WFft<T, N>;
     constexpr int V = W::V, L = W::L;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int t = (threadIdx.x & 31) % L, slot = threadIdx.x / L;  // row of the block
+    const int t = threadIdx.x % L, slot = threadIdx.x / L;  // row of the block
     if (MODE == 0 && blockIdx.x == 0 && threadIdx.x == 0) *a.d_time += 1;  // new step begins
     const int rows = a.nb * a.nz, first = blockIdx.x * (blockDim.x / L) + slot;
     const bool valid = first < rows;
     const int row = valid ? first : rows - 1;  // the warp's other rows need every lane
     T *S = reinterpret_cast<T *>(smem_raw) + (size_t)slot * region;
-    const RowExchange<T, N> ex{S};
+    const RowExchange<T, N> ex{S, slot};
     const RowCtx<T> r(a, row, N);
 
     T re[V], im[V];
@@ -160,8 +165,7 @@ __global__ void __launch_bounds__(ROW_WPB *WARP) row_stage_kernel(StepArgs<T> a,
         mr.add(re[m]);
         mi.add(im[m]);
     }
-    mr.template reduce<L>();
-    mi.template reduce<L>();
+    row_maxima(mr, mi, ex);
     RowScale<T> sr = row_scale<T>(mr), si = row_scale<T>(mi);
 #pragma unroll
     for (int m = 0; m < V; m++) {
@@ -175,7 +179,7 @@ __global__ void __launch_bounds__(ROW_WPB *WARP) row_stage_kernel(StepArgs<T> a,
     constexpr bool DEFER = sizeof(T) == 4 && V < 32;
     constexpr int VD = DEFER ? V : 1;
     T svx[VD], dxo[VD];
-    __syncwarp();  // the transform's last reads of S are done before S holds the x-PML values
+    ex.sync();  // the transform's last reads of S are done before S holds the x-PML values
 #pragma unroll
     for (int m = 0; m < V; m++) {
         const int x = t + L * m, md = DEFER ? m : 0;
@@ -192,7 +196,7 @@ __global__ void __launch_bounds__(ROW_WPB *WARP) row_stage_kernel(StepArgs<T> a,
         mr2.add(vxs);
         mi2.add(vzs);
     }
-    __syncwarp();
+    ex.sync();
     if (valid) row_mid_store_pml<T, MODE, L>(a, r, S, t);
     if (DEFER && valid) {
 #pragma unroll
@@ -203,9 +207,8 @@ __global__ void __launch_bounds__(ROW_WPB *WARP) row_stage_kernel(StepArgs<T> a,
         }
     }
     if (MODE == 2 || !a.flows) return;
-    __syncwarp();  // the x-PML values are read before the next transform reuses S
-    mr2.template reduce<L>();
-    mi2.template reduce<L>();
+    ex.sync();  // the x-PML values are read before the next transform reuses S
+    row_maxima(mr2, mi2, ex);
     sr = row_scale<T>(mr2);
     si = row_scale<T>(mi2);
 #pragma unroll
@@ -344,10 +347,10 @@ __global__ void __launch_bounds__(ROW_WPB *WARP) ddx_kernel(const T *__restrict_
     using W = WFft<T, N, FOUR>;
     constexpr int V = W::V, L = W::L;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int t = (threadIdx.x & 31) % L, slot = threadIdx.x / L;
+    const int t = threadIdx.x % L, slot = threadIdx.x / L;
     const int r0 = 2 * (blockIdx.x * (blockDim.x / L) + slot);
     const bool one = r0 < nrows, two = r0 + 1 < nrows;
-    const RowExchange<T, N> ex{reinterpret_cast<T *>(smem_raw) + (size_t)slot * W::REGION};
+    const RowExchange<T, N, L> ex{reinterpret_cast<T *>(smem_raw) + (size_t)slot * W::REGION, slot};
     const T *src = var + (size_t)r0 * N + t;
     T re[V], im[V];
     RowMax<T> mr, mi;
@@ -361,8 +364,7 @@ __global__ void __launch_bounds__(ROW_WPB *WARP) ddx_kernel(const T *__restrict_
         mr.add(re[m]);
         mi.add(im[m]);
     }
-    mr.template reduce<L>();
-    mi.template reduce<L>();
+    row_maxima(mr, mi, ex);
     const RowScale<T> sr = row_scale<T>(mr), si = row_scale<T>(mi);
 #pragma unroll
     for (int m = 0; m < V; m++) {
@@ -430,8 +432,8 @@ static cudaError_t row_stage_n(const StepArgs<T> &a, cudaStream_t st)
         return cudaGetLastError();
     }
     // four warps a block; two, so that the blocks reach every SM, where the rows are few
-    const int rows = a.nb * a.nz, wpb = rows <= 152 * ROW_WPB * WFft<T, N>::ROWS ? 2 : ROW_WPB;
-    const int slots = wpb * WFft<T, N>::ROWS, grid = (rows + slots - 1) / slots;
+    const int rows = a.nb * a.nz, wpb = rows <= 152 * WFft<T, N>::rows(ROW_WPB) ? 2 : ROW_WPB;
+    const int slots = WFft<T, N>::rows(wpb), grid = (rows + slots - 1) / slots;
     const int region = max(WFft<T, N>::REGION, 3 * a.nhx);  // exchange arrays, or the row's x-PML values
     const size_t smem = (size_t)slots * region * sizeof(T);
     auto k = a.stage == 1 ? row_stage_kernel<T, N, 0> : a.stage <= 5 ? row_stage_kernel<T, N, 1> : row_stage_kernel<T, N, 2>;
@@ -454,8 +456,8 @@ template <typename T, int N, bool FOUR>
 static cudaError_t ddx_n(const T *var, T *dvar, int nrows, T stretchx, const T *twr, const T *twi, const T *kap,
                          cudaStream_t st)
 {
-    const int pairs = (nrows + 1) / 2, wpb = pairs <= 152 * ROW_WPB * WFft<T, N, FOUR>::ROWS ? 1 : ROW_WPB;
-    const int slots = wpb * WFft<T, N, FOUR>::ROWS, grid = (pairs + slots - 1) / slots;
+    const int pairs = (nrows + 1) / 2, wpb = pairs > 152 * WFft<T, N, FOUR>::rows(ROW_WPB) ? ROW_WPB : WFft<T, N, FOUR>::L > WARP ? 2 : 1;
+    const int slots = WFft<T, N, FOUR>::rows(wpb), grid = (pairs + slots - 1) / slots;
     const size_t smem = (size_t)slots * WFft<T, N, FOUR>::REGION * sizeof(T);
     auto k = ddx_kernel<T, N, FOUR>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -486,11 +488,11 @@ __global__ void __launch_bounds__(ROW_WPB *WARP) kacc_row_kernel(KAccArgs<T> a)
     using W = WFft<T, N>;
     constexpr int V = W::V, L = W::L;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int t = (threadIdx.x & 31) % L, slot = threadIdx.x / L;
+    const int t = threadIdx.x % L, slot = threadIdx.x / L;
     const int rows = a.nb * a.nz, first = blockIdx.x * (blockDim.x / L) + slot;
     const bool valid = first < rows;
     const int row = valid ? first : rows - 1;
-    const RowExchange<T, N> ex{reinterpret_cast<T *>(smem_raw) + (size_t)slot * W::REGION};
+    const RowExchange<T, N> ex{reinterpret_cast<T *>(smem_raw) + (size_t)slot * W::REGION, slot};
     const int b = row / a.nz, k = row - b * a.nz;
     const size_t F = (size_t)a.nz * N, q = (size_t)k * N + t;
     const T *f = a.fsn + a.fbase + (size_t)b * a.fstride + q;
@@ -510,8 +512,7 @@ __global__ void __launch_bounds__(ROW_WPB *WARP) kacc_row_kernel(KAccArgs<T> a)
             mr.add(re[m]);
             mi.add(im[m]);
         }
-        mr.template reduce<L>();
-        mi.template reduce<L>();
+        row_maxima(mr, mi, ex);
         const RowScale<T> sr = row_scale<T>(mr), si = row_scale<T>(mi);
 #pragma unroll
         for (int m = 0; m < V; m++) {
@@ -531,7 +532,7 @@ __global__ void __launch_bounds__(ROW_WPB *WARP) kacc_row_kernel(KAccArgs<T> a)
 template <typename T, int N>
 static cudaError_t kacc_row_n(const KAccArgs<T> &a, cudaStream_t st)
 {
-    const int rows = a.nb * a.nz, slots = ROW_WPB * WFft<T, N>::ROWS;
+    const int rows = a.nb * a.nz, slots = WFft<T, N>::rows(ROW_WPB);
     const size_t smem = (size_t)slots * WFft<T, N>::REGION * sizeof(T);
     auto k = kacc_row_kernel<T, N>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

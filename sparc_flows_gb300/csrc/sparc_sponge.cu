@@ -20,19 +20,25 @@ namespace sparc {
 
 constexpr int S5_THREADS = 256, S5X_WARPS = 2;
 
-// ---- x pass: a unit of WFft lanes is one row and one pair of fields (pair 1: option 12)
+// ---- x pass: a unit of S5Fft::L threads is one row and one pair of fields (pair 1: option 12).  FP32 rows of 768 columns
+// keep to one warp and radix 8 here (four solves of 300 levels: 222 us a step against 232 with two warps); of 1024 the
+// registers are limited for eight blocks (259 us against 268).
 template <typename T, int N>
-__global__ void __launch_bounds__(S5X_WARPS *WARP) s5x_kernel(S5Step<T> a, S3Fft<T> f)
+using S5Fft = WFft<T, N, sizeof(T) == 8 && radix_four<T, N>()>;
+template <typename T, int N>
+constexpr int s5x_blocks() { return sizeof(T) == 4 && N == 1024 ? 8 : 0; }
+template <typename T, int N>
+__global__ void __launch_bounds__(S5X_WARPS *WARP, s5x_blocks<T, N>()) s5x_kernel(S5Step<T> a, S3Fft<T> f)
 {
-    using W = WFft<T, N>;
+    using W = S5Fft<T, N>;
     constexpr int V = W::V, L = W::L;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int t = (threadIdx.x & 31) % L, slot = threadIdx.x / L;
+    const int t = threadIdx.x % L, slot = threadIdx.x / L;
     const int rows = a.nz * a.nb, units = rows * (a.option == 12 ? 2 : 1);
-    const int first = blockIdx.x * (S5X_WARPS * W::ROWS) + slot;
+    const int first = blockIdx.x * (W::rows(S5X_WARPS)) + slot;
     const bool valid = first < units;
     const int unit = valid ? first : units - 1, pair = unit / rows, row = unit - pair * rows;
-    const RowExchange<T, N> ex{reinterpret_cast<T *>(smem_raw) + (size_t)slot * W::REGION};
+    const RowExchange<T, N, L> ex{reinterpret_cast<T *>(smem_raw) + (size_t)slot * W::REGION, slot};
     const long long F = a.F, o = (long long)row * N + t;
     T re[V], im[V];
     auto load = [&](int fld, T(&v)[V]) {
@@ -60,8 +66,7 @@ __global__ void __launch_bounds__(S5X_WARPS *WARP) s5x_kernel(S5Step<T> a, S3Fft
         mr.add(re[m]);
         mi.add(im[m]);
     }
-    mr.template reduce<L>();
-    mi.template reduce<L>();
+    row_maxima(mr, mi, ex);
     const RowScale<T> sr = row_scale<T>(mr), si = row_scale<T>(mi);
 #pragma unroll
     for (int m = 0; m < V; m++) {
@@ -274,8 +279,8 @@ static unsigned s5_grid(long long n)
 template <typename T, int N>
 static cudaError_t s5x_n(const S5Step<T> &a, const S3Fft<T> &f, cudaStream_t st)
 {
-    using W = WFft<T, N>;
-    const int units = a.nz * a.nb * (a.option == 12 ? 2 : 1), slots = S5X_WARPS * W::ROWS;
+    using W = S5Fft<T, N>;
+    const int units = a.nz * a.nb * (a.option == 12 ? 2 : 1), slots = W::rows(S5X_WARPS);
     const size_t smem = (size_t)slots * W::REGION * sizeof(T);
     auto k = s5x_kernel<T, N>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -54,10 +54,10 @@ __global__ void __launch_bounds__(TT_XWPB *WARP) tt_fft_x_kernel(double2 *data, 
     using W = WFft<double, N, false>;
     constexpr int V = W::V, L = W::L;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int t = (threadIdx.x & 31) % L, slot = threadIdx.x / L;
-    const long long first = (long long)blockIdx.x * (TT_XWPB * W::ROWS) + slot;
+    const int t = threadIdx.x % L, slot = threadIdx.x / L;
+    const long long first = (long long)blockIdx.x * (W::rows(TT_XWPB)) + slot;
     const bool valid = first < nrows;
-    const RowExchange<double, N> ex{reinterpret_cast<double *>(smem_raw) + (size_t)slot * W::REGION};
+    const RowExchange<double, N, L> ex{reinterpret_cast<double *>(smem_raw) + (size_t)slot * W::REGION, slot};
     double2 *d = data + (valid ? first : nrows - 1) * N + t;
     double re[V], im[V];
 #pragma unroll
@@ -134,14 +134,14 @@ __global__ void __launch_bounds__(COLS *WFft<double, M, false>::L)
     const double cs = inverse ? -1.0 : 1.0;  // conjugation of the input and output for the inverse
     for (int idx = threadIdx.x; idx < nt * COLS; idx += COLS * L) {
         const int k = idx / COLS, c = idx % COLS;
-        const RowExchange<double, M> ex{sm + (size_t)c * SW};
+        const RowExchange<double, M, L> ex{sm + (size_t)c * SW};
         double2 v = (x0 + c < nx) ? base[(size_t)k * nx + c] : make_double2(0.0, 0.0);
         v.y *= cs;
         const double2 w = chirp[k];
         ex.put<0>(k, v.x * w.x - v.y * w.y, v.x * w.y + v.y * w.x);
     }
     __syncthreads();
-    const RowExchange<double, M> ex{sm + (size_t)col * SW};
+    const RowExchange<double, M, L> ex{sm + (size_t)col * SW, col};
     double re[V], im[V];
 #pragma unroll
     for (int m = 0; m < V; m++) {
@@ -157,7 +157,7 @@ __global__ void __launch_bounds__(COLS *WFft<double, M, false>::L)
         im[m] = ar * b.y + ai * b.x;
     }
     wfft_stages<double, M, V, false, 0, 1, true, 0>(re, im, ex, twr, twi, t);
-    __syncwarp();  // the transform's last reads of the region are done
+    ex.sync();  // the transform's last reads of the region are done
     const double inv_m = 1.0 / (double)M;
 #pragma unroll
     for (int m = 0; m < V; m++) {  // X_k = w_k c_k / M, back into the column's region
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(COLS *WFft<double, M, false>::L)
     for (int idx = threadIdx.x; idx < nt * COLS; idx += COLS * L) {
         const int k = idx / COLS, c = idx % COLS;
         if (x0 + c >= nx) continue;
-        const RowExchange<double, M> ec{sm + (size_t)c * SW};
+        const RowExchange<double, M, L> ec{sm + (size_t)c * SW};
         double2 v;
         ec.get<0>(k, v.x, v.y);
         base[(size_t)k * nx + c] = v;
@@ -533,7 +533,7 @@ cudaError_t fft_x_n(sparc_tt_plan *p, double2 *f, int inverse, cudaStream_t st)
 {
     const long long nrows = (long long)p->nb * p->nt;
     using W = WFft<double, N, false>;
-    const int slots = TT_XWPB * W::ROWS;
+    const int slots = W::rows(TT_XWPB);
     const size_t smem = (size_t)slots * W::REGION * sizeof(double);
     auto k = inverse ? tt_fft_x_kernel<N, true> : tt_fft_x_kernel<N, false>;
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

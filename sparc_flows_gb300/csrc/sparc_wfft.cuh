@@ -8,12 +8,16 @@
 // place.  Radices and operation order are those of stockham_stage (sparc_common.cuh), so the results
 // are the same bits.
 //
-// V is a multiple of every radix of N, which gives every lane of a warp whole butterflies at every
+// V is a multiple of every radix of N, which gives every thread whole butterflies at every
 // stage: rows of 64 and 128 columns share a warp (four and two to a warp), where one row to a warp left 24
 // and 16 lanes of it idle.  That matters most in FP64, whose pipe takes 64 cycles per warp-wide
 // instruction and quadrant whether one lane works or all.  Radices 8, 8, ... with V = 8 for 64, 128, 256, 16
-// for 512, 24 for 192, 384, 768, 32 for 1024.  FP64 passes of 192 and 384 columns (FOUR) take radix 4 and V = 12,
+// for 512 and 1024, 24 for 192, 384.  FP64 passes of 192 and 384 columns (FOUR) take radix 4 and V = 12,
 // for twice the warps at the same operations (V = 24 leaves a 300-row pass 75 warps for 608 quadrants).
+// A row of 768 (FOUR, both types: radix 8 and 3 need V = 24) or 1024 columns is held by two warps: one warp would need
+// V = 24 or 32, which fills its registers (FP64 spilled up to 1 KB a thread; FP32 left 8 warps on an SM).  Step of 1024 x
+// 300, two warps against one: FP32 one solve 214 us against 280, six 531 against 752; FP64 one 946 against 1371, four
+// 3390 against 3414.  Of 768 x 300: FP32 six solves 373 against 450, FP64 one 818 against 1118 (GB300).
 #pragma once
 #include "sparc_common.cuh"
 
@@ -21,34 +25,44 @@ namespace sparc {
 
 template <typename T, int N, bool FOUR>
 struct WRadices {
-    static_assert(!FOUR || N == 192 || N == 384, "radix-4 form");
-    static constexpr int V = FOUR ? 12 : N % 3 == 0 ? 24 : N <= 256 ? 8 : N == 512 ? 16 : 32;
+    static_assert(!FOUR || N == 192 || N == 384 || N == 768, "radix-4 form");
+    static constexpr int V = FOUR ? 12 : N % 3 == 0 ? 24 : N <= 256 ? 8 : 16;
     static constexpr int count() { return FOUR ? (N == 192 ? 4 : 5) : Radices<N>::count(); }
-    static constexpr int at(int i) { return !FOUR ? Radices<N>::at(i) : i < 3 ? 4 : N == 384 && i == 3 ? 2 : 3; }
+    static constexpr int at(int i)
+    {
+        if (!FOUR) return Radices<N>::at(i);
+        return i < 3 || (N == 768 && i == 3) ? 4 : N == 384 && i == 3 ? 2 : 3;
+    }
 };
 
-// FP64 passes of a step use the radix-4 form where there is one.
+// Passes of a step use the radix-4 form in FP64 where there is one, at 768 columns in FP32 too (its error against
+// FP64 over 61 steps is that of the radix-8 form or below: records 2.28e-6 against 2.45e-6).
 template <typename T, int N>
-constexpr bool radix_four() { return sizeof(T) == 8 && (N == 192 || N == 384); }
+constexpr bool radix_four() { return (sizeof(T) == 8 && (N == 192 || N == 384)) || N == 768; }
 
 template <typename T, int N, bool FOUR = radix_four<T, N>()>
 struct WFft {
     static constexpr bool RADIX4 = FOUR;
     static constexpr int V = WRadices<T, N, FOUR>::V;
-    static constexpr int L = N / V;          // lanes of a row
-    static constexpr int ROWS = WARP / L;    // rows of a warp
+    static constexpr int L = N / V;          // threads of a row: lanes of one warp or (64) two warps
+    static constexpr int rows(int warps) { return warps * WARP / L; }  // rows of so many warps
     static constexpr int SPAN = N + N / 8;   // words of one exchange array (one word of padding per 8)
     static constexpr int REGION = 2 * SPAN + 8;  // real and imaginary parts of a row
 };
 
-// Exchange buffers.  Row: a row of L lanes of one warp; one padding word per 8 keeps the strided
-// writes of every stage on distinct banks.
-template <typename T, int N>
+// Exchange buffers.  Row: a row of L threads, of one warp or two (which meet at a barrier of the row's own, its
+// number in the block + 1); one padding word per 8 keeps the strided writes of every stage on distinct banks.
+template <typename T, int N, int L = WFft<T, N>::L>
 struct RowExchange {
     static constexpr bool TWO = false;  // a warp's barrier costs less than a second buffer
     static constexpr int SPAN = N + N / 8;
     T *s;
-    __device__ __forceinline__ void sync() const { __syncwarp(); }
+    int row = 0;  // of the block
+    __device__ __forceinline__ void sync() const
+    {
+        __syncwarp();
+        if constexpr (L > WARP) asm volatile("bar.sync %0, %1;" ::"r"(row + 1), "n"(L) : "memory");
+    }
     template <int BUF>
     __device__ __forceinline__ void put(int i, T re, T im) const
     {
@@ -206,6 +220,26 @@ struct RowMax<double> {  // m: the high words' maximum; any: a low word that is 
     }
     __device__ __forceinline__ double value() const { return __hiloint2double((int)m, m == 0u ? (int)any : 0); }
 };
+
+// The maxima of two rows that share a transform, over its threads; rows of two warps meet in the exchange's last words.
+template <typename T, int N, int L>
+__device__ __forceinline__ void row_maxima(RowMax<T> &re, RowMax<T> &im, const RowExchange<T, N, L> &ex)
+{
+    re.template reduce<(L < WARP ? L : WARP)>();
+    im.template reduce<(L < WARP ? L : WARP)>();
+    if constexpr (L > WARP) {
+        static_assert(L == 2 * WARP && 4 * sizeof(RowMax<T>) <= 8 * sizeof(T), "the words behind the exchange arrays");
+        RowMax<T> *w = reinterpret_cast<RowMax<T> *>(ex.s + 2 * RowExchange<T, N, L>::SPAN);
+        const int h = (threadIdx.x / WARP) % 2;
+        if (threadIdx.x % WARP == 0) {
+            w[2 * h] = re;
+            w[2 * h + 1] = im;
+        }
+        ex.sync();
+        re.merge(w[2 * (1 - h)]);
+        im.merge(w[2 * (1 - h) + 1]);
+    }
+}
 
 template <typename T>
 struct RowScale {
