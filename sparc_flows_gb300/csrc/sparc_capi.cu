@@ -1207,7 +1207,7 @@ int sparc_ddx(sparc_plan_t *p, const double *var, double *dvar, int nrows, doubl
 {
     if (!p || !var || !dvar || nrows < 0) return fail(SPARC_ERR_ARG, "sparc_ddx: bad argument");
     CK(launch_ddx<double>(var, dvar, nrows, p->cfg.nx, stretchx, p->fft64.twr, p->fft64.twi, p->fft64.kap,
-                          (cudaStream_t)stream, p->cfg.precision == 32));
+                          (cudaStream_t)stream, p->cfg.precision == 32 || p->cfg.nx == 192));  // at 192 the faster too
     return SPARC_OK;
 }
 

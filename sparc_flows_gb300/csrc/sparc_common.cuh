@@ -416,11 +416,11 @@ template <typename T>
 cudaError_t launch_col_stage(const StepArgs<T> &a, cudaStream_t st);
 template <typename T>
 cudaError_t launch_end_step(const StepArgs<T> &a, cudaStream_t st);
-// setup: radix 8 at every size, the transform that FP32 plans derive their backgrounds with (a last bit of an
+// radix8: radix 8 at every size, the transform that FP32 plans derive their backgrounds with (a last bit of an
 // FP64 background that differs can move an FP32 value, and with it the run)
 template <typename T>
 cudaError_t launch_ddx(const T *var, T *dvar, int nrows, int nx, T stretchx, const T *twr, const T *twi,
-                       const T *kap, cudaStream_t st, bool setup = false);
+                       const T *kap, cudaStream_t st, bool radix8 = false);
 template <typename T>
 cudaError_t launch_ddz(const ZTab<T> &tb, int nch, int L, const T *var, T *dvar, int n1, int nz,
                        const T *preset, const T *stretch, int filter, cudaStream_t st);

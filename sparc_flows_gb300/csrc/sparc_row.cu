@@ -380,6 +380,39 @@ __global__ void __launch_bounds__(ROW_WPB *WARP) ddx_kernel(const T *__restrict_
     }
 }
 
+// The same of few FP64 rows: a transform in shared memory, a pair of rows to a warp.  With radix 8 the register form
+// holds 24 values a thread at 192 and 384 columns, eight and sixteen lanes to a pair: too few warps for the FP64 pipe.
+template <int N>
+__global__ void __launch_bounds__(ROW_WPB *WARP) ddx_shared_kernel(const double *__restrict__ var, double *__restrict__ dvar,
+                                                                    int nrows, double stretchx, const double *twr,
+                                                                    const double *twi, const double *kap)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int warp = threadIdx.x / WARP, lane = threadIdx.x % WARP, r0 = 2 * (blockIdx.x * ROW_WPB + warp);
+    if (r0 >= nrows) return;
+    const bool two = r0 + 1 < nrows;
+    double *xr = reinterpret_cast<double *>(smem_raw) + (size_t)warp * 4 * N, *xi = xr + N, *yr = xi + N, *yi = yr + N;
+    const double *src = var + (size_t)r0 * N;
+    double mr = 0.0, mi = 0.0;
+    for (int x = lane; x < N; x += WARP) {
+        xr[x] = src[x];
+        xi[x] = two ? src[N + x] : 0.0;
+        mr = fmax(mr, fabs(xr[x]));
+        mi = fmax(mi, fabs(xi[x]));
+    }
+    double sr, si, isr, isi;
+    warp_row_scale(mr, sr, isr);
+    warp_row_scale(mi, si, isi);
+    __syncwarp();
+    double *re, *im, *dst = dvar + (size_t)r0 * N;
+    fft_deriv<double, N>(xr, xi, yr, yi, twr, twi, kap, stretchx, lane, re, im, sr, si);
+    __syncwarp();
+    for (int x = lane; x < N; x += WARP) {
+        dst[x] = re[x] * isr;
+        if (two) dst[N + x] = im[x] * isi;
+    }
+}
+
 #define SPARC_FFT_SIZES(X) X(64) X(128) X(192) X(256) X(384) X(512) X(768) X(1024)
 
 bool fft_size_supported(int n)
@@ -465,14 +498,34 @@ static cudaError_t ddx_n(const T *var, T *dvar, int nrows, T stretchx, const T *
     return cudaGetLastError();
 }
 
+template <int N>
+static cudaError_t ddx_shared_n(const double *var, double *dvar, int nrows, double stretchx, const double *twr,
+                                const double *twi, const double *kap, cudaStream_t st)
+{
+    const size_t smem = (size_t)ROW_WPB * 4 * N * sizeof(double);
+    auto k = ddx_shared_kernel<N>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<(nrows + 2 * ROW_WPB - 1) / (2 * ROW_WPB), ROW_WPB * WARP, smem, st>>>(var, dvar, nrows, stretchx, twr, twi, kap);
+    return cudaGetLastError();
+}
+
 template <typename T>
 cudaError_t launch_ddx(const T *var, T *dvar, int nrows, int nx, T stretchx, const T *twr, const T *twi,
-                       const T *kap, cudaStream_t st, bool setup)
+                       const T *kap, cudaStream_t st, bool radix8)
 {
     if (nrows <= 0) return cudaSuccess;
+    // FP64 at radix 8: three (192 columns) and one (384) waves of a pair of rows to each of four warps per SM.  192: 23 us
+    // up to 1200 rows and 50 at 3600 against 51 in registers, 66 against 56 at 4800; 384: 55 against 60, 93 against 60 at
+    // 1800 (GB300).  Both give the same bits.
+    if constexpr (sizeof(T) == 8) {
+        const int wave = 152 * ROW_WPB * 2;
+        if (radix8 && nx == 192 && nrows <= 3 * wave) return ddx_shared_n<192>(var, dvar, nrows, stretchx, twr, twi, kap, st);
+        if (radix8 && nx == 384 && nrows <= wave) return ddx_shared_n<384>(var, dvar, nrows, stretchx, twr, twi, kap, st);
+    }
 #define CASE(n_)                                                                                                     \
     if (nx == n_)                                                                                                    \
-        return radix_four<T, n_>() && !setup                                                                         \
+        return radix_four<T, n_>() && !radix8                                                                         \
                    ? ddx_n<T, n_, radix_four<T, n_>()>(var, dvar, nrows, stretchx, twr, twi, kap, st)                 \
                    : ddx_n<T, n_, false>(var, dvar, nrows, stretchx, twr, twi, kap, st);
     SPARC_FFT_SIZES(CASE)
