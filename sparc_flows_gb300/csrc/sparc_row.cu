@@ -137,13 +137,13 @@ __device__ __forceinline__ void row_mid_store_pml(const StepArgs<T> &a, const Ro
 
 // Resident blocks that the registers are limited for (0: no limit): four at 768 columns in FP32, eight rows on an SM (four solves of
 // 300 levels 299 us a step against 309 without the limit); at 1024 the limit costs more than it gives (308 against 294).
-template <typename T, int N>
-constexpr int row_blocks() { return sizeof(T) == 4 && N == 768 ? 4 : 0; }
+template <typename T, int N, bool TIGHT>
+constexpr int row_blocks() { return TIGHT ? 3 : sizeof(T) == 4 && N == 768 ? 4 : 0; }
 
 // The row pass with the register transforms of sparc_wfft.cuh: WFft<T, N>::L threads a row, thread t of a
 // row holding columns t + L m.
-template <typename T, int N, int MODE>
-__global__ void __launch_bounds__(ROW_WPB *WARP, row_blocks<T, N>()) row_stage_kernel(StepArgs<T> a, int region)
+template <typename T, int N, int MODE, bool TIGHT>
+__global__ void __launch_bounds__(ROW_WPB *WARP, (row_blocks<T, N, TIGHT>())) row_stage_kernel(StepArgs<T> a, int region)
 {
     using W = WFft<T, N>;
     constexpr int V = W::V, L = W::L;
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(ROW_WPB *WARP, row_blocks<T, N>()) row_stage_k
 
     RowMax<T> mr2, mi2;
     // FP32: every load of the row before its first store, where the registers hold what is to be stored
-    constexpr bool DEFER = sizeof(T) == 4 && V < 32;
+    constexpr bool DEFER = sizeof(T) == 4 && !TIGHT;
     constexpr int VD = DEFER ? V : 1;
     T svx[VD], dxo[VD];
     ex.sync();  // the transform's last reads of S are done before S holds the x-PML values
@@ -455,6 +455,23 @@ static void row_reg512_launch(const StepArgs<float> &a, cudaStream_t st)
     return row_reg512_n<MODE, 4>(a, st);
 }
 
+template <typename T, int N, bool TIGHT>
+static cudaError_t row_generic(const StepArgs<T> &a, cudaStream_t st)
+{
+    // four warps a block; two, so that the blocks reach every SM, where the rows are few
+    const int rows = a.nb * a.nz, wpb = rows <= 152 * WFft<T, N>::rows(ROW_WPB) ? 2 : ROW_WPB;
+    const int slots = WFft<T, N>::rows(wpb), grid = (rows + slots - 1) / slots;
+    const int region = max(WFft<T, N>::REGION, 3 * a.nhx);  // exchange arrays, or the row's x-PML values
+    const size_t smem = (size_t)slots * region * sizeof(T);
+    auto k = a.stage == 1   ? row_stage_kernel<T, N, 0, false>
+             : a.stage <= 5 ? row_stage_kernel<T, N, 1, TIGHT>
+                            : row_stage_kernel<T, N, 2, false>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<grid, wpb * WARP, smem, st>>>(a, region);
+    return cudaGetLastError();
+}
+
 template <typename T, int N>
 static cudaError_t row_stage_n(const StepArgs<T> &a, cudaStream_t st)
 {
@@ -464,16 +481,15 @@ static cudaError_t row_stage_n(const StepArgs<T> &a, cudaStream_t st)
         else row_reg512_launch<2>(a, st);
         return cudaGetLastError();
     }
-    // four warps a block; two, so that the blocks reach every SM, where the rows are few
-    const int rows = a.nb * a.nz, wpb = rows <= 152 * WFft<T, N>::rows(ROW_WPB) ? 2 : ROW_WPB;
-    const int slots = WFft<T, N>::rows(wpb), grid = (rows + slots - 1) / slots;
-    const int region = max(WFft<T, N>::REGION, 3 * a.nhx);  // exchange arrays, or the row's x-PML values
-    const size_t smem = (size_t)slots * region * sizeof(T);
-    auto k = a.stage == 1 ? row_stage_kernel<T, N, 0> : a.stage <= 5 ? row_stage_kernel<T, N, 1> : row_stage_kernel<T, N, 2>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    k<<<grid, wpb * WARP, smem, st>>>(a, region);
-    return cudaGetLastError();
+    // FP32 with 24 values a thread (192 and 384 columns): stages 2 to 5 hold every load of a row at once, two blocks an SM.  Rows that
+    // would make a second wave of those and one wave of three blocks take three, with 168 registers and their stores
+    // where the values arise (a solve keeps its bits): 12 solves of 384 x 300 353 us a step against 371, 24 of 192 x 300
+    // 335 against 387 (GB300)
+    if constexpr (sizeof(T) == 4 && (N == 192 || N == 384)) {
+        const int rows = a.nb * a.nz, block = WFft<T, N>::rows(ROW_WPB);
+        if (rows > 152 * 2 * block && rows <= 152 * 3 * block) return row_generic<T, N, true>(a, st);
+    }
+    return row_generic<T, N, false>(a, st);
 }
 
 template <typename T>
