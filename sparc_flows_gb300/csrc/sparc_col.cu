@@ -30,8 +30,9 @@ constexpr int max_nch() { return sizeof(T) == 8 && CW <= 8 ? 32 : 20; }
 template <typename T, int CW>
 constexpr int min_blocks() { return CW <= 8 ? (sizeof(T) == 4 ? 4 : 2) : 1; }
 
-template <typename T, int CW, int LMAX>
-__global__ void __launch_bounds__(CW *max_nch<T, CW>(), (min_blocks<T, CW>())) col_stage_kernel(StepArgs<T> a)
+// MINB: resident blocks that the registers are limited for.
+template <typename T, int CW, int LMAX, int MINB>
+__global__ void __launch_bounds__(CW *max_nch<T, CW>(), MINB) col_stage_kernel(StepArgs<T> a)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *B0 = reinterpret_cast<T *>(smem_raw);
@@ -563,15 +564,32 @@ cudaError_t launch_kacc(const KAccArgs<T> &a, cudaStream_t st)
 template cudaError_t launch_kacc<float>(const KAccArgs<float> &, cudaStream_t);
 template cudaError_t launch_kacc<double>(const KAccArgs<double> &, cudaStream_t);
 
-template <typename T, int CW, int LMAX = COL_LMAX>
+template <typename T, int CW, int LMAX = COL_LMAX, int MINB = min_blocks<T, CW>()>
 static cudaError_t launch_col_stage_cw(const StepArgs<T> &a, cudaStream_t st)
 {
     const size_t smem = ((size_t)2 * a.nz * CW + (size_t)8 * a.nch * CW) * sizeof(T);
-    auto k = col_stage_kernel<T, CW, LMAX>;
+    auto k = col_stage_kernel<T, CW, LMAX, MINB>;
     cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     dim3 grid(a.nx / CW, a.nb);
     k<<<grid, CW * a.nch, smem, st>>>(a);
     return cudaGetLastError();
+}
+
+// FP64 blocks of 8 columns with chunks of up to 10 rows.  A thread that keeps its rows in registers takes 128 of them (16
+// warps on an SM; up to 8 rows 104 and 19); with 80 some rows go through local memory, but 25 warps are resident.  That is the faster where it saves
+// a wave (one block is 4 to 8 warps): five solves of 512 x 300, 320 blocks in one wave of 456 instead of two of 304, 37.5 ms
+// for 16 steps against 41.3, of 512 x 217 25.7 against 29.9; the slower otherwise: eight, two waves of either, 55.2 against
+// 50.6 (GB300).
+template <typename T, int LMAX>
+static cudaError_t launch_col_stage_short(const StepArgs<T> &a, cudaStream_t st)
+{
+    const int warps = (8 * a.nch + WARP - 1) / WARP;
+    const long long blocks = (long long)(a.nx / 8) * a.nb;
+    auto waves = [&](int resident_warps) {
+        const long long wave = 152LL * (resident_warps / warps);
+        return (blocks + wave - 1) / wave;
+    };
+    return waves(25) < waves(LMAX <= 8 ? 19 : 16) ? launch_col_stage_cw<T, 8, LMAX, 3>(a, st) : launch_col_stage_cw<T, 8, LMAX, 2>(a, st);
 }
 
 template <typename T>
@@ -583,8 +601,11 @@ cudaError_t launch_col_stage(const StepArgs<T> &a, cudaStream_t st)
         // FP64 chunks of up to 12 rows: register arrays of that length, so that two 8-column blocks
         // are resident
         case 8:
-            if constexpr (sizeof(T) == 8)
+            if constexpr (sizeof(T) == 8) {
+                if (a.L <= 8) return launch_col_stage_short<T, 8>(a, st);
+                if (a.L <= 10) return launch_col_stage_short<T, 10>(a, st);
                 if (a.L <= 12) return launch_col_stage_cw<T, 8, 12>(a, st);
+            }
             return launch_col_stage_cw<T, 8>(a, st);
         case 4:
             if constexpr (sizeof(T) == 8)
