@@ -166,14 +166,13 @@ int sparc_check_state(sparc_plan_t *plan, double *norms, void *stream);
 /* Current step counter (synchronises the stream). */
 int sparc_get_time(sparc_plan_t *plan, int *time, void *stream);
 
-/* Diagnostics (no counterpart in the reference): the kernels this plan launches for its column
- * and end-of-step passes and whether each row pass starts on the SMs the column pass's last wave
- * leaves idle, as "column=<kernel> end=<kernel> stage_overlap=<0|1>" (NUL-terminated, at most len
- * bytes).  FP32 plans of 512 columns with the banded column pass have the overlap unless
- * SPARC_STAGE_OVERLAP=0 is set when the plan is created; it is taken where the column pass has a partial
- * last wave behind a full one (SPARC_STAGE_OVERLAP=1: everywhere).  Of a banded column kernel the first five
- * template arguments are named: the fifth is 1 on a grid with compiled sizes whose inputs are bulk-copied, 0 on
- * every other grid, bulk-copied or not. */
+/* Diagnostics (no counterpart in the reference): the kernels this plan launches for its column and
+ * end-of-step passes, as "column=<kernel> end=<kernel> stage_overlap=<0|1> overlap_taken=<0|1> staged=<0|1>"
+ * (NUL-terminated, at most len bytes).  stage_overlap: the plan has what it takes to start each row pass on the SMs the
+ * column pass's last wave leaves idle (FP32, 512 columns, the banded column pass, SPARC_STAGE_OVERLAP not 0 when the
+ * plan is created); overlap_taken: its steps do so (where the column pass has a partial last wave behind a full one, or
+ * SPARC_STAGE_OVERLAP is 1).  staged: the banded column pass has its inputs bulk-copied.  Of a banded column kernel the
+ * first five template arguments are named: the fifth is 1 where the grid's sizes are compiled in and staged. */
 int sparc_plan_describe(const sparc_plan_t *plan, char *buf, int len);
 
 /* Kernel construction from paired snapshots (kernels.f90:209-358): for record pair

@@ -1385,7 +1385,9 @@ int sparc_plan_describe(const sparc_plan_t *p, char *buf, int len)
               : S.end_stream ? "end_step_stream_kernel<double>" : "end_step_kernel<double>";
     }
     const bool overlap = p->cfg.precision == 32 && p->s32.a.tile_cnt != nullptr;
-    const std::string d = "column=" + col + " end=" + end + " stage_overlap=" + (overlap ? "1" : "0");
+    const bool staged = p->cfg.precision == 32 && p->s32.band_R && p->s32.have_maps32;
+    const std::string d = "column=" + col + " end=" + end + " stage_overlap=" + (overlap ? "1" : "0") + " overlap_taken=" +
+                          (overlap && p->s32.overlap ? "1" : "0") + " staged=" + (staged ? "1" : "0");
     std::snprintf(buf, (size_t)len, "%s", d.c_str());
     return SPARC_OK;
 }
