@@ -342,16 +342,27 @@ class ExactGradient:
         """Static device buffers of one reverse step: the state before the step, the adjoints,
         the gradient accumulators of each solve, the forcing row and the work of sparc_adjoint_step."""
         if getattr(self, "_s", None) is None:
-            ops, dev = self.ops, self.ws.dev
-            sa, sz, sw = ((ops.nb, 4, ops.nz, ops.nx), (ops.nb, 2, ops.nzpml, ops.nx), (ops.nb, 2, ops.nz, ops.nhx))
-            sg = (ops.nb, ops.nz, ops.nx)
-            z = lambda sh: torch.zeros(sh, dtype=F64, device=dev)  # noqa: E731
-            self._s = dict(a=z(sa), Pz=z(sz), Px=z(sw), la=z(sa), lZ=z(sz), lW=z(sw), gx=z(sg),
-                           gz=z(sg), gc=z(sg), f=z((ops.nb, ops.nx)))
-            self._work = torch.empty(int(self.ws.L.sparc_adjoint_step_bytes(self.ws.plan)), dtype=torch.uint8,
-                                     device=dev)
+            try:
+                s, work = self._step_buffers()
+            except torch.cuda.OutOfMemoryError:
+                if not self._keep_caches:
+                    raise
+                # the segment's stage caches leave no room for them: its states instead
+                self._keep_caches, self.segbuf = False, None
+                self.segbuf = torch.empty((self.seg, self.row), dtype=torch.uint8, device=self.ws.dev)
+                s, work = self._step_buffers()
             capi.check(self.ws.L.sparc_adjoint_prepare(self.ws.plan), "sparc_adjoint_prepare")
+            self._s, self._work = s, work
         return self._s
+
+    def _step_buffers(self):
+        ops, dev = self.ops, self.ws.dev
+        sa, sz, sw = ((ops.nb, 4, ops.nz, ops.nx), (ops.nb, 2, ops.nzpml, ops.nx), (ops.nb, 2, ops.nz, ops.nhx))
+        sg = (ops.nb, ops.nz, ops.nx)
+        z = lambda sh: torch.zeros(sh, dtype=F64, device=dev)  # noqa: E731
+        s = dict(a=z(sa), Pz=z(sz), Px=z(sw), la=z(sa), lZ=z(sz), lW=z(sw), gx=z(sg), gz=z(sg), gc=z(sg),
+                 f=z((ops.nb, ops.nx)))
+        return s, torch.empty(int(self.ws.L.sparc_adjoint_step_bytes(self.ws.plan)), dtype=torch.uint8, device=dev)
 
     def _reverse_step(self, cached: bool = False):
         """Recompute the stages of one step from the static state (cached: take them from the work's
