@@ -15,6 +15,7 @@ the Fortran compiler rounds them.
 from __future__ import annotations
 
 import ctypes
+import itertools
 import math
 import os
 
@@ -191,7 +192,7 @@ class TTAdjoint:
 
     def _rows(self, pord, x00s, modes, dt, windows, misfit=False) -> np.ndarray:
         """The measured receivers of a mode, (n, 7) int32 rows (b, i, timest, timefin, lef, rig, 0) by source and
-        column; windows {b: [(lef, rig), ...]} in that order, or None to pick."""
+        column; windows {b: any iterable of (lef, rig)} in that order, or None to pick."""
         mindist, maxdist, _ = modes[pord]
         out = []
         for b in range(self.nb):
@@ -204,10 +205,10 @@ class TTAdjoint:
                 # a search range outside the record: the reference reads out of bounds
                 rows = rows[np.maximum(ts, 1) <= np.minimum(tf, self.nt)]
             elif len(i):
-                given = windows.get(b, [])
+                given = list(itertools.islice(windows.get(b, []), len(i)))
                 if len(given) < len(i):
                     raise StopIteration("fewer windows than measured receivers")
-                rows[:, 4:6] = np.asarray(given[:len(i)])
+                rows[:, 4:6] = np.asarray(given)
             out.append(rows)
         return np.ascontiguousarray(np.concatenate(out) if out else np.zeros((0, 7), dtype=np.int32))
 
