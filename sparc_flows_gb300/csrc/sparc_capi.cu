@@ -783,9 +783,12 @@ int alloc_solver(sparc_plan *p)
     // stage overlap: the 512-column row pass starts on the SMs that the banded column pass's last
     // wave leaves idle, each row block waiting for its own solve's column tiles only
     // (SPARC_STAGE_OVERLAP=0 turns it off).  Taken where there is such a wave: a grid of one wave, or of whole
-    // waves, only pays for the counters and for row blocks that wait on SMs (one solve of 512 x 300: 227 us a step
-    // with it, 200 without; 10 solves 408 against 468, 32 solves 1052 against 1077, GB300).  SPARC_STAGE_OVERLAP=1
-    // takes it on every grid
+    // waves, only pays for the counters and for row blocks that wait on SMs.  us a step at 300 levels, with it and
+    // without: one solve 223 / 192, 9 solves (144 tiles) 381 / 307, 10 (160) 392 / 446, 14 (224) 490 / 518, 19 (two whole
+    // waves) 757 / 622, 24 809 / 818, 32 1012 / 1040.  It loses where the last wave is nearly full (18 solves, 136 of 152
+    // SMs, 657 / 609; 28, 144 of 152, 968 / 882) and, up to 217 levels, for 10 to 24 solves, where several tiles share an SM
+    // (150 levels 10 375 / 345; 217 levels 10 402 / 394, 14 461 / 495): a line there is not drawn yet (GB300).
+    // SPARC_STAGE_OVERLAP=1 takes it on every grid
     a.tile_cnt = nullptr;
     a.tiles_per_solve = 0;
     {

@@ -14,7 +14,6 @@
 namespace sparc {
 
 constexpr int WARP = 32;
-constexpr int MAX_NCH = 24;  // chunks per column (nz <= MAX_NCH * LMAX)
 constexpr int SPARC_DEV_ERR_TMA_TIMEOUT = 1;  // device error flag: a bounded mbarrier wait gave up
 constexpr int SPARC_DEV_ERR_TMA_ALIGN = 2;    // ... a TMA destination in shared memory was not 128-byte aligned
 constexpr int SPARC_DEV_ERR_STAGE_WAIT = 3;   // ... a row pass gave up waiting for its solve's column tiles

@@ -447,7 +447,7 @@ static void row_reg512_n(const StepArgs<float> &a, cudaStream_t st)
     k<<<grid, ROW_WPB * WARP, smem, st>>>(a);
 }
 
-// Few rows (a block on every other SM): registers for all loads of a row at once (two blocks per SM, 255
+// Few rows (at most one block on every SM): registers for all loads of a row at once (two blocks per SM, 255
 // registers) instead of four blocks: 11.9 us a launch for one solve of 512 x 300 against 12.9.
 template <int MODE>
 static void row_reg512_launch(const StepArgs<float> &a, cudaStream_t st)

@@ -6,7 +6,7 @@
 // shared memory, the first stage reads what was loaded from global memory, and the last leaves
 // element t + L m in register m again: the multiplication by i k and the inverse transform follow in
 // place.  Radices and operation order are those of stockham_stage (sparc_common.cuh), so the results
-// are the same bits.
+// are the same bits; the radix-4 form (FOUR, below) has its own.
 //
 // V is a multiple of every radix of N, which gives every thread whole butterflies at every
 // stage: rows of 64 and 128 columns share a warp (four and two to a warp), where one row to a warp left 24
@@ -161,7 +161,7 @@ __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, 
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 
 // Spectral derivative of a complex row held as re, im[m] = x[t + L m] (real and imaginary parts: two
-// real rows), in place; kap and scale as fft_deriv (sparc_common.cuh).
+// real rows), in place; kap (which carries 1 / N and a zero Nyquist bin) and scale as fft_deriv (sparc_common.cuh).
 template <typename T, int N, int V, bool FOUR, class EX>
 __device__ __forceinline__ void wfft_deriv(T (&re)[V], T (&im)[V], const EX &ex, const T *__restrict__ twr,
                                            const T *__restrict__ twi, const T *__restrict__ kap, T scale, int t)
