@@ -297,10 +297,6 @@ __global__ void __launch_bounds__(ROW_WPB *WARP, MINB) row_stage_reg512_kernel(S
 
     float mr2 = 0.f, mi2 = 0.f;
     float svx[16], dxo[16];
-    if (MODE != 2 && r.k == a.nz - 1) {  // without the x-PML term (physics2d.f90:954-955)
-#pragma unroll
-        for (int n2 = 0; n2 < 16; n2++) a.TOPDX[(size_t)r.b * 512 + lane + 32 * n2] = im[n2] * isi;
-    }
     __syncwarp();  // the transform's last reads of S are done before S holds the x-PML values
 #pragma unroll
     for (int n2 = 0; n2 < 16; n2++) {
@@ -319,7 +315,10 @@ __global__ void __launch_bounds__(ROW_WPB *WARP, MINB) row_stage_reg512_kernel(S
         for (int n2 = 0; n2 < 16; n2++) {
             const int x = lane + 32 * n2;
             if (MODE != 0) svp(a, a.slot_sm1, r.b, 0)[ro + x] = svx[n2];
-            if (MODE != 2) a.DX[(size_t)r.b * F + ro + x] = dxo[n2];
+            if (MODE != 2) {
+                a.DX[(size_t)r.b * F + ro + x] = dxo[n2];
+                if (r.k == a.nz - 1) a.TOPDX[(size_t)r.b * 512 + x] = dxo[n2];
+            }
         }
     }
     if (MODE == 2 || !a.flows) return;
