@@ -135,15 +135,10 @@ __device__ __forceinline__ void row_mid_store_pml(const StepArgs<T> &a, const Ro
     }
 }
 
-// Resident blocks that the registers are limited for (0: no limit): four at 768 columns in FP32, eight rows on an SM (four solves of
-// 300 levels 299 us a step against 309 without the limit); at 1024 the limit costs more than it gives (308 against 294).
-template <typename T, int N, bool TIGHT>
-constexpr int row_blocks() { return TIGHT ? 3 : sizeof(T) == 4 && N == 768 ? 4 : 0; }
-
 // The row pass with the register transforms of sparc_wfft.cuh: WFft<T, N>::L threads a row, thread t of a
 // row holding columns t + L m.
 template <typename T, int N, int MODE, bool TIGHT>
-__global__ void __launch_bounds__(ROW_WPB *WARP, (row_blocks<T, N, TIGHT>())) row_stage_kernel(StepArgs<T> a, int region)
+__global__ void __launch_bounds__(ROW_WPB *WARP, TIGHT ? 3 : 0) row_stage_kernel(StepArgs<T> a, int region)
 {
     using W = WFft<T, N>;
     constexpr int V = W::V, L = W::L;
@@ -481,11 +476,11 @@ static cudaError_t row_stage_n(const StepArgs<T> &a, cudaStream_t st)
         else row_reg512_launch<2>(a, st);
         return cudaGetLastError();
     }
-    // FP32 with 24 values a thread (192 and 384 columns): stages 2 to 5 hold every load of a row at once, two blocks an SM.  Rows that
-    // would make a second wave of those and one wave of three blocks take three, with 168 registers and their stores
-    // where the values arise (a solve keeps its bits): 12 solves of 384 x 300 353 us a step against 371, 24 of 192 x 300
-    // 335 against 387 (GB300)
-    if constexpr (sizeof(T) == 4 && (N == 192 || N == 384)) {
+    // FP32 with 24 values a thread (192, 384 and 768 columns): stages 2 to 5 hold every load of a row at once, two blocks
+    // an SM.  Rows that would make a second wave of those and one wave of three blocks take three, with 168 registers and
+    // their stores where the values arise (a solve keeps its bits): 12 solves of 384 x 300 353 us a step against 371, 24 of
+    // 192 x 300 335 against 387 (GB300)
+    if constexpr (sizeof(T) == 4 && N % 3 == 0) {
         const int rows = a.nb * a.nz, block = WFft<T, N>::rows(ROW_WPB);
         if (rows > 152 * 2 * block && rows <= 152 * 3 * block) return row_generic<T, N, true>(a, st);
     }

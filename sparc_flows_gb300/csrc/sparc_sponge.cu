@@ -20,17 +20,14 @@ namespace sparc {
 
 constexpr int S5_THREADS = 256, S5X_WARPS = 2;
 
-// ---- x pass: a unit of S5Fft::L threads is one row and one pair of fields (pair 1: option 12).  FP32 rows of 768 columns
-// keep to one warp and radix 8 here (four solves of 300 levels: 222 us a step against 232 with two warps); of 1024 the
-// registers are limited for eight blocks (259 us against 268).
-template <typename T, int N>
-using S5Fft = WFft<T, N, sizeof(T) == 8 && radix_four<T, N>()>;
+// ---- x pass: a unit of WFft::L threads is one row and one pair of fields (pair 1: option 12).  FP32 rows of 1024 columns:
+// registers for eight blocks an SM (four solves of 300 levels 259 us a step against 268 without the limit).
 template <typename T, int N>
 constexpr int s5x_blocks() { return sizeof(T) == 4 && N == 1024 ? 8 : 0; }
 template <typename T, int N>
 __global__ void __launch_bounds__(S5X_WARPS *WARP, s5x_blocks<T, N>()) s5x_kernel(S5Step<T> a, S3Fft<T> f)
 {
-    using W = S5Fft<T, N>;
+    using W = WFft<T, N>;
     constexpr int V = W::V, L = W::L;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int t = threadIdx.x % L, slot = threadIdx.x / L;
@@ -279,7 +276,7 @@ static unsigned s5_grid(long long n)
 template <typename T, int N>
 static cudaError_t s5x_n(const S5Step<T> &a, const S3Fft<T> &f, cudaStream_t st)
 {
-    using W = S5Fft<T, N>;
+    using W = WFft<T, N>;
     const int units = a.nz * a.nb * (a.option == 12 ? 2 : 1), slots = W::rows(S5X_WARPS);
     const size_t smem = (size_t)slots * W::REGION * sizeof(T);
     auto k = s5x_kernel<T, N>;

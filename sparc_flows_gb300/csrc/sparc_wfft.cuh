@@ -12,12 +12,12 @@
 // stage: rows of 64 and 128 columns share a warp (four and two to a warp), where one row to a warp left 24
 // and 16 lanes of it idle.  That matters most in FP64, whose pipe takes 64 cycles per warp-wide
 // instruction and quadrant whether one lane works or all.  Radices 8, 8, ... with V = 8 for 64, 128, 256, 16
-// for 512 and 1024, 24 for 192, 384.  FP64 passes of 192 and 384 columns (FOUR) take radix 4 and V = 12,
+// for 512 and 1024, 24 for 192, 384, 768.  FP64 passes of 192, 384 and 768 columns (FOUR) take radix 4 and V = 12,
 // for twice the warps at the same operations (V = 24 leaves a 300-row pass 75 warps for 608 quadrants).
-// A row of 768 (FOUR, both types: radix 8 and 3 need V = 24) or 1024 columns is held by two warps: one warp would need
-// V = 24 or 32, which fills its registers (FP64 spilled up to 1 KB a thread; FP32 left 8 warps on an SM).  Step of 1024 x
-// 300, two warps against one: FP32 one solve 214 us against 280, six 531 against 752; FP64 one 946 against 1371, four
-// 3390 against 3414.  Of 768 x 300: FP32 six solves 373 against 450, FP64 one 818 against 1118 (GB300).
+// A row of 1024 columns, and of 768 in FP64, is held by two warps: one warp would need V = 32 or 24, which fills its
+// registers (FP64 spilled up to 1 KB a thread; FP32 left 8 warps on an SM).  Step of 1024 x 300, two warps against
+// one: FP32 one solve 214 us against 280, six 545 against 797; FP64 one 946 against 1371, four 3390 against 3414.  Of
+// 768 x 300: FP64 one 818 against 1118 (GB300).  FP32 rows of 768 columns keep radix 8, and with it their bits.
 #pragma once
 #include "sparc_common.cuh"
 
@@ -35,10 +35,9 @@ struct WRadices {
     }
 };
 
-// Passes of a step use the radix-4 form in FP64 where there is one, at 768 columns in FP32 too (its error against
-// FP64 over 61 steps is that of the radix-8 form or below: records 2.28e-6 against 2.45e-6).
+// FP64 passes of a step use the radix-4 form where there is one.
 template <typename T, int N>
-constexpr bool radix_four() { return (sizeof(T) == 8 && (N == 192 || N == 384)) || N == 768; }
+constexpr bool radix_four() { return sizeof(T) == 8 && (N == 192 || N == 384 || N == 768); }
 
 template <typename T, int N, bool FOUR = radix_four<T, N>()>
 struct WFft {

@@ -1,4 +1,4 @@
-"""Rows of 768 and 1024 columns, whose transforms are shared by two warps: x-derivatives of few and many rows whose
+"""Rows of 768 (FP64) and 1024 columns, whose transforms are shared by two warps: x-derivatives of few and many rows whose
 largest value lies in either warp's part, the 2-D row pass and the kernel integral against the CPU oracle, FP32 against
 FP64."""
 import numpy as np

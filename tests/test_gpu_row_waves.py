@@ -1,4 +1,4 @@
-"""FP32 row pass of 192 and 384 columns at the batch sizes where its stages 2 to 5 run with fewer registers a thread: a
+"""FP32 row pass of 192, 384 and 768 columns at the batch sizes where its stages 2 to 5 run with fewer registers a thread: a
 solve of such a batch has the bits it has alone, and tracks FP64."""
 import numpy as np
 import pytest
@@ -9,9 +9,10 @@ from sparc_flows_gb300.config import RunConfig
 pytestmark = pytest.mark.gpu
 
 
-# rows (solves x levels) just inside both ends of (4864, 7296] at 192 and (2432, 3648] at 384, and outside
+# rows (solves x levels) just inside both ends of (4864, 7296] at 192, (2432, 3648] at 384 and (1216, 1824] at 768, and
+# outside
 @pytest.mark.parametrize("nx,nz,nb", [(192, 271, 18), (192, 256, 28), (192, 271, 17), (384, 271, 9), (384, 256, 14),
-                                      (384, 157, 24)])
+                                      (384, 157, 24), (768, 246, 5), (768, 300, 6)])
 def test_bits_of_a_solve(nx, nz, nb):
     from sparc_flows_gb300.solver import WaveSolver
     run = RunConfig(nx=nx, nz=nz, xlength_cm=nx * 0.78125e8, nsteps=31, flows=True, npmlbot=20)
