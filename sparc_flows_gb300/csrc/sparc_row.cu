@@ -229,6 +229,64 @@ __global__ void __launch_bounds__(ROW_WPB *WARP, TIGHT ? 3 : 0) row_stage_kernel
     }
 }
 
+// The row pass with the transforms in shared memory, one row to a warp: 109 registers where the register form with 24
+// values a thread takes 254, four blocks an SM instead of two (where it is taken: row_stage_n).  Same bits.
+template <int N, int MODE>
+__global__ void __launch_bounds__(ROW_WPB *WARP) row_stage_shared_kernel(StepArgs<float> a)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int warp = threadIdx.x / WARP, lane = threadIdx.x % WARP;
+    if (MODE == 0 && blockIdx.x == 0 && threadIdx.x == 0) *a.d_time += 1;  // new step begins
+    const int row = blockIdx.x * ROW_WPB + warp;
+    if (row >= a.nb * a.nz) return;
+    float *xr = reinterpret_cast<float *>(smem_raw) + (size_t)warp * 4 * N, *yr = xr + 2 * N;  // real, imaginary parts
+    const RowCtx<float> r(a, row, N);
+    float mr = 0.f, mi = 0.f;
+    for (int x = lane; x < N; x += WARP) {
+        float p, xis;
+        row_load<float, MODE>(a, r, x, p, xis);
+        xr[x] = p;
+        xr[N + x] = xis;
+        mr = fmaxf(mr, fabsf(p));
+        mi = fmaxf(mi, fabsf(xis));
+    }
+    float sr, si, isr, isi, *re, *im;
+    warp_row_scale(mr, sr, isr);
+    warp_row_scale(mi, si, isi);
+    __syncwarp();
+    fft_deriv<float, N>(xr, xr + N, yr, yr + N, a.twr, a.twi, a.kap, a.stretchx, lane, re, im, sr, si);
+    __syncwarp();
+    float *P = re == xr ? yr : xr;  // the x-PML values, then the next transform's other arrays
+    float mr2 = 0.f, mi2 = 0.f;
+    for (int x = lane; x < N; x += WARP) {
+        float svx, dxo, vxs, vzs;
+        const float dxx = im[x] * isi;
+        if (MODE != 2 && r.k == a.nz - 1) a.TOPDX[(size_t)r.b * N + x] = dxx;  // without the x-PML term
+        row_mid_load<float, MODE>(a, r, x, re[x] * isr, dxx, P, svx, dxo, vxs, vzs);
+        if (MODE != 0) svp(a, a.slot_sm1, r.b, 0)[r.ro + x] = svx;
+        if (MODE != 2) a.DX[(size_t)r.b * r.F + r.ro + x] = dxo;
+        re[x] = vxs;
+        im[x] = vzs;
+        mr2 = fmaxf(mr2, fabsf(vxs));
+        mi2 = fmaxf(mi2, fabsf(vzs));
+    }
+    __syncwarp();
+    row_mid_store_pml<float, MODE, WARP>(a, r, P, lane);
+    if (MODE == 2 || !a.flows) return;
+    warp_row_scale(mr2, sr, isr);
+    warp_row_scale(mi2, si, isi);
+    __syncwarp();  // the x-PML values are read before the transform takes their place
+    float *o2r, *o2i;
+    fft_deriv<float, N>(re, im, P, P + N, a.twr, a.twi, a.kap, a.stretchx, lane, o2r, o2i, sr, si);
+    __syncwarp();
+    for (int x = lane; x < N; x += WARP) {
+        const size_t q = (size_t)r.b * r.F + r.ro + x;
+        const float w = -2.f * a.fsign * __ldg(a.v0x + (size_t)r.b * a.bg2 + r.ro + x);
+        a.FXX[q] = w * (o2r[x] * isr);
+        a.FXZ[q] = w * (o2i[x] * isi);
+    }
+}
+
 // FP32 rows of 512 columns: the same row pass with the register-resident FFT (sparc_fft512.cuh);
 // register n2 of a lane holds column lane + 32 n2.  Each part loads everything it needs before it
 // stores anything, so no load waits behind a store of the row it may alias.
@@ -312,6 +370,8 @@ __global__ void __launch_bounds__(ROW_WPB *WARP, MINB) row_stage_reg512_kernel(S
             if (MODE != 0) svp(a, a.slot_sm1, r.b, 0)[ro + x] = svx[n2];
             if (MODE != 2) {
                 a.DX[(size_t)r.b * F + ro + x] = dxo[n2];
+                // with the x-PML term, where physics2d.f90:954-955 and the generic pass take it without: from rest the
+                // difference is below FP32's rounding, but any other rounding here moves the FP32 kernels by 1.5e-5
                 if (r.k == a.nz - 1) a.TOPDX[(size_t)r.b * 512 + x] = dxo[n2];
             }
         }
@@ -467,6 +527,19 @@ static cudaError_t row_generic(const StepArgs<T> &a, cudaStream_t st)
     return cudaGetLastError();
 }
 
+template <int N>
+static cudaError_t row_shared(const StepArgs<float> &a, cudaStream_t st)
+{
+    const size_t smem = (size_t)ROW_WPB * 4 * N * sizeof(float);
+    auto k = a.stage == 1   ? row_stage_shared_kernel<N, 0>
+             : a.stage <= 5 ? row_stage_shared_kernel<N, 1>
+                            : row_stage_shared_kernel<N, 2>;
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k<<<(a.nb * a.nz + ROW_WPB - 1) / ROW_WPB, ROW_WPB * WARP, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
 template <typename T, int N>
 static cudaError_t row_stage_n(const StepArgs<T> &a, cudaStream_t st)
 {
@@ -479,8 +552,13 @@ static cudaError_t row_stage_n(const StepArgs<T> &a, cudaStream_t st)
     // FP32 with 24 values a thread (192, 384 and 768 columns): stages 2 to 5 hold every load of a row at once, two blocks
     // an SM.  Rows that would make a second wave of those and one wave of three blocks take three, with 168 registers and
     // their stores where the values arise (a solve keeps its bits): 12 solves of 384 x 300 353 us a step against 371, 24 of
-    // 192 x 300 335 against 387 (GB300)
-    if constexpr (sizeof(T) == 4 && N % 3 == 0) {
+    // 192 x 300 335 against 387 (GB300).  At 768 columns that spills, and what would be the second wave
+    // goes to the transforms in shared memory, four blocks an SM: six solves of 768 x 300 403 us a step against 455
+    if constexpr (sizeof(T) == 4 && N == 768) {
+        const int rows = a.nb * a.nz;
+        if (rows > 152 * 2 * ROW_WPB && rows <= 152 * 4 * ROW_WPB && 3 * a.nhx <= 2 * N) return row_shared<N>(a, st);
+    }
+    if constexpr (sizeof(T) == 4 && (N == 192 || N == 384)) {
         const int rows = a.nb * a.nz, block = WFft<T, N>::rows(ROW_WPB);
         if (rows > 152 * 2 * block && rows <= 152 * 3 * block) return row_generic<T, N, true>(a, st);
     }

@@ -9,10 +9,10 @@ from sparc_flows_gb300.config import RunConfig
 pytestmark = pytest.mark.gpu
 
 
-# rows (solves x levels) just inside both ends of (4864, 7296] at 192, (2432, 3648] at 384 and (1216, 1824] at 768, and
+# rows (solves x levels) just inside both ends of (4864, 7296] at 192, (2432, 3648] at 384 and (1216, 2432] at 768, and
 # outside
 @pytest.mark.parametrize("nx,nz,nb", [(192, 271, 18), (192, 256, 28), (192, 271, 17), (384, 271, 9), (384, 256, 14),
-                                      (384, 157, 24), (768, 246, 5), (768, 300, 6)])
+                                      (384, 157, 24), (768, 246, 5), (768, 300, 8), (768, 174, 14)])
 def test_bits_of_a_solve(nx, nz, nb):
     from sparc_flows_gb300.solver import WaveSolver
     run = RunConfig(nx=nx, nz=nz, xlength_cm=nx * 0.78125e8, nsteps=31, flows=True, npmlbot=20)
